@@ -140,6 +140,11 @@ DevGrid make_grid(Allocs& A, const skg_grid& g, cudaStream_t s) {
     G.type = g.type;
     G.xmin = g.xmin; G.ymin = g.ymin; G.zmin = g.zmin; G.xmax = g.xmax; G.ymax = g.ymax; G.zmax = g.zmax;
     REQUIRE(g.xmax > g.xmin && g.ymax > g.ymin && g.zmax > g.zmin, "grid extent is empty");
+    const double blo[3] = {g.xmin, g.ymin, g.zmin}, bhi[3] = {g.xmax, g.ymax, g.zmax};
+    for (int a = 0; a < 3; a++) {
+        G.bmid[a] = (float)(0.5 * (blo[a] + bhi[a]));
+        G.bscale[a] = (float)(2.0 / (bhi[a] - blo[a]));
+    }
     double diag = grid_diag(g);
     G.eps = 1e-12 * diag;
     double amax = std::max({std::fabs(g.xmin), std::fabs(g.xmax), std::fabs(g.ymin), std::fabs(g.ymax),
@@ -371,6 +376,12 @@ struct skg_ctx {
     void* scan_scratch = nullptr; size_t scan_bytes = 0;
     std::string error;
 };
+
+// Bytes of a grid that the FP32 walks of one direction read: 32-byte leaf records, about 16 neighbour
+// entries of 32 bytes per Voronoi cell.
+static size_t walk_bytes(const DevGrid& g) {
+    return (size_t)g.ncells * (g.type == SKG_GRID_CARTESIAN ? 4 : g.type == SKG_GRID_VORONOI ? 512 : 32);
+}
 
 static int fail(skg_ctx* ctx, const Failure& f) {
     set_error(f.msg);
@@ -809,7 +820,7 @@ int skg_run_phase(skg_ctx* ctx, int phase, const int32_t* ells, int nell, uint64
         const bool big = total >= ((uint64_t)1 << 26) && ctx->grid.type != SKG_GRID_VORONOI;
         const size_t pool_max = (opts && opts->pool > 0) ? (size_t)opts->pool : ((size_t)1 << (big ? 23 : 21));
         const size_t npool = (size_t)std::min<uint64_t>(total, pool_max);
-        CK(ctx->waves.reserve(npool, ctx->hs.ngroups, ctx->grid.type));
+        CK(ctx->waves.reserve(npool, ctx->hs.ngroups, ctx->grid.type, walk_bytes(ctx->grid)));
         // one slot, one work item (pageable host sources: the copies are staged before return)
         BatchHeader H = {phase, 1, 1, 0, total};
         WorkItem W;
@@ -1285,7 +1296,9 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
         int ngroups = 0;
         for (skg_ctx* c : slots) ngroups = std::max(ngroups, c->hs.ngroups);
         if (total == 0) return SKG_OK;
-        CK(b->waves.reserve(npool, ngroups, gtype));
+        size_t wb = 0;
+        for (skg_ctx* c : slots) wb = std::max(wb, walk_bytes(c->grid));
+        CK(b->waves.reserve(npool, ngroups, gtype, wb));
         REQUIRE(!opts || (opts->refill >= 0 && opts->refill <= 32), "refill lanes must be in 0..32");
         RunParams P = b->T.params((opts && opts->max_scatt > 0) ? opts->max_scatt : 100000, opts ? opts->refill : 0);
         Staging& T = b->T;

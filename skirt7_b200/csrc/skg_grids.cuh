@@ -23,6 +23,7 @@ struct DevGrid {
     float  epsf;                // FP32 nudge (a few ulps of the domain size)
     int ncells;
     int max_steps;
+    float bmid[3], bscale[3];   // middle of the box and 1 / its half widths (bins of the walk order)
 
     // Cartesian planes
     int nx, ny, nz;

@@ -122,6 +122,7 @@ struct RunParams {
 // pass (one thread per record) advances every packet to its next traversals and writes them as
 // jobs, and a traversal pass walks all jobs of the wave.
 enum PacketState : int { PK_EMPTY = 0, PK_WAIT, PK_INTERACT, PK_TERM, PK_DONE };
+constexpr int JOB_BINS = 1 << 15;     // bins of the walk order, for path jobs and for peel-off jobs each
 constexpr int JOB_MAIN = 31;          // job type of the packet's own path; 0..15 = peel-off group
 
 struct __align__(16) Packet {
@@ -165,6 +166,12 @@ struct WaveParams {
     int* freelist;                    // records the event pass freed (count: jcount[5])
     int* intlist;                     // records it found at their interaction point (jcount[6])
     float4* ckpt;                     // per packet record: checkpoints of its path walk
+    // walk order of the wave's jobs (order_kernel); hist == nullptr: as appended
+    unsigned* hist;                   // [2][JOB_BINS] jobs per bin: path jobs, peel-off jobs (zero between waves)
+    unsigned* bin0;                   // [2][JOB_BINS] first place of each bin
+    uint2* jkey;                      // per job (its bin, its rank within it)
+    int* spath;                       // packets of the path jobs in walk order
+    int4* speel;                      // peel-off jobs in walk order: (packet, group, job index, 0)
     // the grid of a single-simulation launch: the traversal kernels' instantiation for one slot
     // reads it from their parameters (constant-bank operands, no load instructions per cell step)
     DevGrid g0;

@@ -58,9 +58,6 @@ namespace skg {
 #ifndef SKG_PEEL_MIN_BLOCKS
 #define SKG_PEEL_MIN_BLOCKS 4
 #endif
-#ifndef SKG_SPLIT_TRAV
-#define SKG_SPLIT_TRAV 1
-#endif
 // programmatic dependent launch of the peel-off-job kernel after the path-job kernel
 #ifndef SKG_PDL
 #define SKG_PDL 1
@@ -437,13 +434,44 @@ SKG_D int find_item(const WorkItem* items, int n, uint64_t p) {
 // ---------------------------------------------------------------------------------------------
 // event pass
 
+// Bins of the walk order.  A path job: the octant of its direction, then the Morton cell of its start
+// on a 16^3 division of the grid's box.  A peel-off job: its direction group (mod 8), then the Morton
+// cell, on a 64^2 division, of the point where its ray passes the middle plane of the box across the
+// direction's largest component.
+SKG_D int bin_coord(float u, int n) {
+    // u: -1..1 across the box
+    return min(n - 1, max(0, (int)((0.5f * u + 0.5f) * n)));
+}
+SKG_D unsigned spread3(unsigned v) { return (v & 1) | (v & 2) << 2 | (v & 4) << 4 | (v & 8) << 6; }
+SKG_D unsigned spread2(unsigned v) {
+    v = (v | v << 4) & 0x0F0Fu; v = (v | v << 2) & 0x3333u; return (v | v << 1) & 0x5555u;
+}
+SKG_D unsigned path_bin(const DevGrid& g, float x, float y, float z, float kx, float ky, float kz) {
+    const unsigned oct = (kx < 0.f ? 1u : 0u) | (ky < 0.f ? 2u : 0u) | (kz < 0.f ? 4u : 0u);
+    const int i = bin_coord((x - g.bmid[0]) * g.bscale[0], 16), j = bin_coord((y - g.bmid[1]) * g.bscale[1], 16),
+              k = bin_coord((z - g.bmid[2]) * g.bscale[2], 16);
+    return oct << 12 | spread3(i) | spread3(j) << 1 | spread3(k) << 2;
+}
+SKG_D unsigned peel_bin(const DevGrid& g, int grp, float x, float y, float z, float kx, float ky, float kz) {
+    // box coordinates (-1..1) of the position and the direction
+    float u = (x - g.bmid[0]) * g.bscale[0], v = (y - g.bmid[1]) * g.bscale[1], w = (z - g.bmid[2]) * g.bscale[2];
+    float du = kx * g.bscale[0], dv = ky * g.bscale[1], dw = kz * g.bscale[2];
+    // the axis of the largest component last
+    const float au = fabsf(du), av = fabsf(dv), aw = fabsf(dw);
+    if (au >= av && au >= aw) { float t = u; u = w; w = t; t = du; du = dw; dw = t; }
+    else if (av >= aw) { float t = v; v = w; w = t; t = dv; dv = dw; dw = t; }
+    const float f = w / dw;
+    const int i = bin_coord(u - f * du, 64), j = bin_coord(v - f * dv, 64);
+    return (unsigned)(grp & 7) << 12 | spread2(i) | spread2(j) << 1;
+}
+
 // The direction groups that get a peel-off traversal from (x, y, z), in group order
 // (MonteCarloSimulation.cpp:299-357): emission peel-offs carry weight 1, scattering peel-offs the
 // phase-function value, and a negative value ends the list (the reference aborts the peel-off).
 // With WRITE the jobs are stored from j0 on; returns their number.
 template<bool WRITE>
 SKG_D int peel_jobs(const DevScene& S, int ell, bool scat, int cell, double kx, double ky, double kz, double x,
-                    double y, double z, double L, int p, int j0, int2* jobs, double* jL) {
+                    double y, double z, double L, int p, int j0, const WaveParams* W, const DevGrid* grid) {
     int n = 0;
     for (int g = 0; g < S.ngroups; g++) {
         double w = 1.0;
@@ -452,7 +480,15 @@ SKG_D int peel_jobs(const DevScene& S, int ell, bool scat, int cell, double kx, 
             if (w < 0) break;
         }
         if (!group_needs_traversal(S, g, x, y, z)) continue;
-        if (WRITE) { jobs[j0 + n] = make_int2(p, g); jL[j0 + n] = L * w; }
+        if (WRITE) {
+            W->jobs[j0 + n] = make_int2(p, g);
+            W->jL[j0 + n] = L * w;
+            if (W->hist) {
+                const unsigned b = peel_bin(*grid, g, (float)x, (float)y, (float)z, (float)S.gkx[g], (float)S.gky[g],
+                                            (float)S.gkz[g]);
+                W->jkey[j0 + n] = make_uint2(b, atomicAdd(W->hist + JOB_BINS + b, 1u));
+            }
+        }
         n++;
     }
     return n;
@@ -565,11 +601,20 @@ SKG_D void append_jobs(const WaveParams& W, int p, Packet& K, int npeel, int nma
     if (npeel > 0) {
         const int j0 = W.npool + (int)(bp + inp - npeel);
         const DevScene& S = *W.R.scenes[W.R.items[K.item].slot];
-        peel_jobs<true>(S, K.ell, scat_peel, K.int_cell, kx0, ky0, kz0, K.x, K.y, K.z, K.L, p, j0, W.jobs, W.jL);
+        peel_jobs<true>(S, K.ell, scat_peel, K.int_cell, kx0, ky0, kz0, K.x, K.y, K.z, K.L, p, j0, &W,
+                        W.R.grids + W.R.items[K.item].slot);
         K.peel_j0 = j0;
     }
     K.peel_n = npeel;
-    if (nmain) W.jobs[bm + inm - 1] = make_int2(p, JOB_MAIN);
+    if (nmain) {
+        const unsigned j = bm + inm - 1;
+        W.jobs[j] = make_int2(p, JOB_MAIN);
+        if (W.hist) {
+            const unsigned b = path_bin(W.R.grids[W.R.items[K.item].slot], (float)K.x, (float)K.y, (float)K.z, (float)K.kx,
+                                        (float)K.ky, (float)K.kz);
+            W.jkey[j] = make_uint2(b, atomicAdd(W.hist + b, 1u));
+        }
+    }
 }
 
 template<typename R, bool STRIDE>
@@ -746,6 +791,57 @@ __global__ void __launch_bounds__(SKG_EVENT_THREADS) launch_kernel(const WavePar
 }
 
 // ---------------------------------------------------------------------------------------------
+// walk order: a counting sort of the wave's jobs by bin (each job has its rank within its bin from
+// the launch pass)
+
+// First place of each bin (block 0 path jobs, block 1 peel-off jobs); clears the counts.
+__global__ void __launch_bounds__(1024) bins_kernel(unsigned* hist, unsigned* bin0) {
+    __shared__ unsigned ws[32];
+    constexpr int PER = JOB_BINS / 1024;
+    uint4* h = reinterpret_cast<uint4*>(hist + blockIdx.x * JOB_BINS + threadIdx.x * PER);
+    uint4* o = reinterpret_cast<uint4*>(bin0 + blockIdx.x * JOB_BINS + threadIdx.x * PER);
+    uint4 c[PER / 4];
+    unsigned sum = 0;
+#pragma unroll
+    for (int i = 0; i < PER / 4; i++) { c[i] = h[i]; sum += c[i].x + c[i].y + c[i].z + c[i].w; }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned inc = sum;
+    for (int d = 1; d < 32; d <<= 1) { const unsigned t = __shfl_up_sync(0xffffffffu, inc, d); if (lane >= d) inc += t; }
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned v = ws[lane], w = v;
+        for (int d = 1; d < 32; d <<= 1) { const unsigned t = __shfl_up_sync(0xffffffffu, w, d); if (lane >= d) w += t; }
+        ws[lane] = w - v;
+    }
+    __syncthreads();
+    unsigned at = ws[warp] + inc - sum;
+#pragma unroll
+    for (int i = 0; i < PER / 4; i++) {
+        uint4 b;
+        b.x = at; at += c[i].x; b.y = at; at += c[i].y; b.z = at; at += c[i].z; b.w = at; at += c[i].w;
+        o[i] = b;
+        h[i] = make_uint4(0, 0, 0, 0);
+    }
+}
+
+// Writes the jobs in walk order.
+__global__ void __launch_bounds__(256) order_kernel(const WaveParams W) {
+    const unsigned nmain = W.jcount[0], npeel = W.jcount[1];
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nmain + npeel; i += gridDim.x * blockDim.x) {
+        if (i < nmain) {
+            const uint2 k = W.jkey[i];
+            W.spath[W.bin0[k.x] + k.y] = W.jobs[i].x;
+        } else {
+            const unsigned j = W.npool + (i - nmain);
+            const uint2 k = W.jkey[j];
+            const int2 jb = W.jobs[j];
+            W.speel[W.bin0[JOB_BINS + k.x] + k.y] = make_int4(jb.x, jb.y, (int)j, 0);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // traversal pass
 
 // Absorption in cell m of a path step: simulateescapeandabsorption (MonteCarloSimulation.cpp:441-462)
@@ -853,8 +949,8 @@ SKG_D bool resume_ckpt(const WaveParams& W, const DevGrid& g, int p, int nck, do
     return true;
 }
 
-// MODE: 0 every job of the wave; 1 the path jobs only; 2 the peel-off jobs only (a lean
-// instantiation: optical depth alone, no path state)
+// MODE: 1 the path jobs; 2 the peel-off jobs (a lean instantiation: optical depth alone, no path
+// state)
 // Resident blocks per SM of each instantiation.  The Voronoi path-job kernel runs at 3 blocks (80
 // registers, no spills: its neighbour scan keeps more state): 1219 against 1273 ms per 10^7-packet
 // phase; the tree and Cartesian ones are faster at 4 (189 against 194 ms, 94 against 100 ms).
@@ -888,8 +984,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
     // only from "unknown" to the cell, and either value is a valid hint for the peel-off walk.
     if (MODE == 1) asm volatile("griddepcontrol.launch_dependents;");
 #endif
-    const unsigned nmainj = W.jcount[0];
-    const unsigned njobs = MODE == 0 ? nmainj + W.jcount[1] : MODE == 1 ? nmainj : W.jcount[1];
+    const unsigned njobs = W.jcount[MODE == 1 ? 0 : 1];
     unsigned* const taken = W.jcount + (MODE == 2 ? 4 : 2);
     const int phase = H.phase;
     const int lane = threadIdx.x & 31;
@@ -951,10 +1046,18 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
             if (need) {
                 const unsigned jj = base + __popc(want & ((1u << lane) - 1));
                 if (jj >= njobs) break;
-                if (MODE == 0) j = jj < nmainj ? (int)jj : W.npool + (int)(jj - nmainj);
-                else if (MODE == 1) j = (int)jj;
-                else j = W.npool + (int)jj;
-                const int2 jb = W.jobs[j];
+                int2 jb;
+                if (MODE == 1) {
+                    j = (int)jj;
+                    jb = W.hist ? make_int2(W.spath[jj], JOB_MAIN) : W.jobs[j];
+                } else if (W.hist) {
+                    const int4 o = W.speel[jj];
+                    jb = make_int2(o.x, o.y);
+                    j = o.z;
+                } else {
+                    j = W.npool + (int)jj;
+                    jb = W.jobs[j];
+                }
                 p = jb.x;
                 const Packet& K = W.pk[p];
                 ell = K.ell;
@@ -1307,10 +1410,13 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
 #endif
         }
         launch_kernel<R><<<sms * per, SKG_EVENT_THREADS, 0, s>>>(W);
+        if (W.hist) {
+            bins_kernel<<<2, 1024, 0, s>>>(W.hist, W.bin0);
+            order_kernel<<<std::min(sms * 8, (W.npool + 255) / 256), 256, 0, s>>>(W);
+        }
     }
 #endif
     if (mid) cudaEventRecord(mid, s);
-#if SKG_SPLIT_TRAV
     // the path jobs, then the peel-off jobs in their lean kernel
     trav_kernel<R, Stepper, 1, ONE><<<trav_blocks > 0 ? trav_blocks : resident_blocks<R, Stepper, 1, ONE>(smem), 256, smem, s>>>(W);
 #if SKG_PDL
@@ -1328,9 +1434,6 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
     if (e != cudaSuccess) return e;
 #else
     trav_kernel<R, Stepper, 2, ONE><<<resident_blocks<R, Stepper, 2, ONE>(smem), 256, smem, s>>>(W);
-#endif
-#else
-    trav_kernel<R, Stepper, 0, ONE><<<trav_blocks > 0 ? trav_blocks : resident_blocks<R, Stepper, 0, ONE>(smem), 256, smem, s>>>(W);
 #endif
     return cudaGetLastError();
 }
@@ -1377,7 +1480,9 @@ WaveRunner::~WaveRunner() {
     for (cudaEvent_t e : ev_) cudaEventDestroy(e);
     for (cudaEvent_t e : tail_ev_) if (e) cudaEventDestroy(e);
     // (a runner that never reserved frees nothing: no device-wide synchronisation)
-    for (void* p : {(void*)pk_, (void*)free_, (void*)ckpt_, (void*)ctr_}) if (p) cudaFree(p);
+    for (void* p : {(void*)pk_, (void*)free_, (void*)ckpt_, (void*)ctr_, (void*)bins_, (void*)jkey_, (void*)spath_,
+                    (void*)speel_})
+        if (p) cudaFree(p);
     for (int b = 0; b < 2; b++)
         for (void* p : {(void*)jobs_[b], (void*)jtau_[b], (void*)jL_[b]}) if (p) cudaFree(p);
     if (h_ctr_) cudaFreeHost(h_ctr_);
@@ -1391,8 +1496,19 @@ static bool ckpt_grid(int grid_type) {
     return Resumable<TreeLatticeStepper<float>>::value;
 }
 
-cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type) {
+// Jobs in spatial order: the lanes of a warp walk through the same region, so more of the grid's
+// records come from L1 and L2, for the cost of the counting sort.  Worth it when the wave has enough
+// jobs to be dense and the records are more than what stays close anyway: phases of 2*10^7 packets on
+// a 3*10^6-leaf octree (96 MB of records) 306 against 293 ms, of 2*10^6 on 10^6 Voronoi cells (512 MB)
+// 262 against 254 ms; below these bounds the sort costs more than it gives (2.4*10^5 packets on a small octree
+// 4.1 against 4.7 ms; Cartesian densities are a few MB: a batch of 24 fit variants 53.5 against 56.2 ms).
+static bool order_pays(int grid_type, size_t pool, size_t walk_bytes) {
+    return grid_type != SKG_GRID_CARTESIAN && pool >= ((size_t)3 << 19) && walk_bytes >= ((size_t)8 << 20);
+}
+
+cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes) {
     cudaError_t e;
+    order_on_ = order_pays(grid_type, pool, walk_bytes);
     if (!ctr_) {
         if ((e = cudaMalloc(&ctr_, NCTR * sizeof(unsigned))) != cudaSuccess) return e;
         if ((e = cudaMallocHost((void**)&h_ctr_, NCTR * sizeof(unsigned))) != cudaSuccess) return e;
@@ -1409,8 +1525,13 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type) {
         if ((e = cudaMalloc(&ckpt_, pool * SKG_CKPT_N * 2 * sizeof(float4))) != cudaSuccess) return e;
         cap_ckpt_ = pool;
     }
+    if (order_on_ && !bins_) {
+        if ((e = cudaMalloc(&bins_, 4 * JOB_BINS * sizeof(unsigned))) != cudaSuccess) return e;
+        if ((e = cudaMemset(bins_, 0, 4 * JOB_BINS * sizeof(unsigned))) != cudaSuccess) return e;
+    }
     const size_t jobs = pool * (size_t)(ngroups + 1);
     if (jobs > cap_jobs_) {
+
         for (int b = 0; b < 2; b++) {
             cudaFree(jobs_[b]); cudaFree(jtau_[b]); cudaFree(jL_[b]);
             jobs_[b] = nullptr; jtau_[b] = nullptr; jL_[b] = nullptr;
@@ -1422,6 +1543,14 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type) {
             if ((e = cudaMalloc(&jL_[b], jobs * sizeof(double))) != cudaSuccess) return e;
         }
         cap_jobs_ = jobs;
+    }
+    if (order_on_ && jobs > cap_order_) {
+        cudaFree(jkey_); cudaFree(speel_); cudaFree(spath_);
+        jkey_ = nullptr; speel_ = nullptr; spath_ = nullptr; cap_order_ = 0;
+        if ((e = cudaMalloc(&jkey_, jobs * sizeof(uint2))) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&speel_, jobs * sizeof(int4))) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&spath_, jobs * sizeof(int))) != cudaSuccess) return e;
+        cap_order_ = jobs;
     }
     return cudaSuccess;
 }
@@ -1438,6 +1567,8 @@ cudaError_t WaveRunner::enqueue(int n) {
         W.last_busy = ctr_ + 16;
         W.freelist = free_; W.intlist = free_ + npool_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
         W.g0 = g0_;
+        W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
+        W.jkey = jkey_; W.spath = spath_; W.speel = speel_;
         if ((e = cudaMemsetAsync(ctr_ + 8 * b, 0, 8 * sizeof(unsigned), stream_)) != cudaSuccess) return e;
         if (timed_) {
             while (ev_.size() < 3 * (size_t)(w + 1)) {
@@ -1488,6 +1619,7 @@ cudaError_t WaveRunner::enqueue_tail() {
     W.pjobs = jobs_[b]; W.pjtau = jtau_[b]; W.pjL = jL_[b];
     W.last_busy = ctr_ + 16;
     W.freelist = nullptr; W.intlist = nullptr; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+    W.hist = nullptr; W.bin0 = nullptr; W.jkey = nullptr; W.spath = nullptr; W.speel = nullptr;
     cudaError_t e;
     if (timed_) {
         for (int i = 0; i < 2; i++)

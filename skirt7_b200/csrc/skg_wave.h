@@ -23,8 +23,9 @@ public:
 
     // Sizes the pool and job buffers (allocates; call outside stream capture).  pool packets,
     // ngroups peel-off groups at most per packet; grid_type decides whether path walks keep
-    // checkpoints (grids whose FP32 walk resumes).
-    cudaError_t reserve(size_t pool, int ngroups, int grid_type);
+    // checkpoints (grids whose FP32 walk resumes); walk_bytes, what the FP32 walks read of the (largest)
+    // grid, with the pool whether the jobs are walked in spatial order.
+    cudaError_t reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes);
     // Enqueues the reset of the pool and the first waves of a phase on stream s.  P holds the
     // staged tables; nslots the slots whose DevGrid the traversal pass keeps in shared memory;
     // tree_walk the FP32 tree walk (TreeWalk) of tree grids; one_grid (host copy), when given with
@@ -63,6 +64,12 @@ private:
     double* jtau_[2] = {nullptr, nullptr};
     double* jL_[2] = {nullptr, nullptr};
     size_t cap_jobs_ = 0;
+    unsigned* bins_ = nullptr;        // [2][JOB_BINS] counts, [2][JOB_BINS] first places (walk order)
+    uint2* jkey_ = nullptr;
+    int* spath_ = nullptr;
+    int4* speel_ = nullptr;
+    size_t cap_order_ = 0;
+    bool order_on_ = false;           // the running phase walks its jobs in spatial order
     static constexpr int NCTR = 17;
     unsigned* ctr_ = nullptr;         // [8b .. 8b+7]: counters of job buffer b; [16]: last busy wave
     unsigned* h_ctr_ = nullptr;       // pinned copy read by finish()
