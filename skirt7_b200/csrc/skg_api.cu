@@ -516,6 +516,12 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
             if (sc->ncomp == 1 && (ctx->grid.lrec || ctx->grid.prec)) CK(launch_embed_density(ctx->grid, rf, s));
         }
 
+        // octant records of the FP32 walk (256 bytes per cell; without them it takes the lattice records)
+        if (ctx->grid.lattice && ctx->grid.search != SKG_SEARCH_BOOKKEEPING && nc <= (1 << 27)) {
+            uint4* rec = A.alloc<uint4>(16 * (size_t)nc);
+            if (rec) { CK(launch_octant_records(ctx->grid, rec, s)); ctx->grid.orec = rec; }
+        }
+
         // stellar system (StellarSystem.cpp:35-52)
         H.nstellar = sc->nstellar;
         std::vector<double> starL(sc->nstellar * nl), Lv(nl, 0.0), Xvv((size_t)nl * (sc->nstellar + 1), 0.0);
@@ -1257,6 +1263,7 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
             const int bk = tree_walk_of(w.ctx->grid);
             if (gbk < 0) gbk = bk;
             if (gtype == SKG_GRID_CARTESIAN) gbk = std::min(gbk, bk);   // the plane tables serve every grid
+            else if (tree(gtype) && std::min(bk, gbk) == TW_LATTICE) gbk = TW_LATTICE;   // octant and lattice records: the latter
             else if (tree(gtype)) REQUIRE(bk == gbk, "a batch holds trees of one walk kind (Bookkeeping search, rope or lattice records)");
             if (phase != SKG_PHASE_STELLAR) REQUIRE(w.ctx->emit_cdf != nullptr, "dust phases need dust emission enabled");
             int slot = -1;

@@ -58,6 +58,9 @@ struct DevGrid {
     // lattice form (trees split at midpoints): 32-byte leaf records in cell order, walls at
     // fmaf(integer, lunit, lorg); irec as above (layout: RopeTree in skg_tree.h)
     const uint4*  prec;
+    // per direction octant (bit a set: k_a < 0) the leaves' exit walls, density and ropes
+    // (launch_octant_records): 32-byte records, [octant][cell]; null when not built
+    const uint4*  orec;
     int lattice;
     float lorg[3], lunit[3];
 
@@ -81,11 +84,11 @@ struct DevGrid {
 // The FP32 walk a grid takes.  Trees: the node walk (Bookkeeping search), the 64-byte rope records
 // or their lattice form; Cartesian grids: the plane tables, or computed walls when every axis is
 // evenly spaced.
-enum TreeWalk : int { TW_ROPE = 0, TW_NODES = 1, TW_LATTICE = 2 };
+enum TreeWalk : int { TW_ROPE = 0, TW_NODES = 1, TW_LATTICE = 2, TW_OCTANT = 3 };
 enum CartWalk : int { CW_TABLE = 0, CW_UNIFORM = 1 };
 inline int tree_walk_of(const DevGrid& g) {
     if (g.type == SKG_GRID_CARTESIAN) return g.cart_uniform ? CW_UNIFORM : CW_TABLE;
-    return g.search == SKG_SEARCH_BOOKKEEPING ? TW_NODES : g.lattice ? TW_LATTICE : TW_ROPE;
+    return g.search == SKG_SEARCH_BOOKKEEPING ? TW_NODES : !g.lattice ? TW_ROPE : g.orec ? TW_OCTANT : TW_LATTICE;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -981,6 +984,107 @@ struct TreeLatticeStepper<float> {
             }
             if (next < 0) done = true;
             else { leaf = next; d += eps; }
+            if (d > 0.f) { ds = d; return true; }
+        }
+        return false;
+    }
+};
+
+// The lattice walk on the octant records: the walls ahead, the density and the ropes of the exit
+// walls of the walk's direction octant come ready from one 32-byte record, where the lattice record
+// has to be decoded every step (three codes to walls, the rope to a reference).  The walls are the
+// floats the lattice walk computes and every comparison and sum is the same, so the segments are
+// bit-identical to TreeLatticeStepper<float>.
+template<typename R> struct TreeOctantStepper : TreeNodeWalk<R> {};
+
+template<>
+struct TreeOctantStepper<float> {
+    float x, y, z, kx, ky, kz;
+    float ux, uy, uz;           // 1/k per axis (0 where |k| <= 1e-15)
+    float bx, by, bz;           // 0, or FLT_MAX on an axis that is never crossed
+    float wx, wy, wz;           // the current leaf's walls ahead
+    float wrho;                 // its density
+    int gx_, gy_, gz_;          // its ropes: a record of this octant's table, -1 outside, <= -2 an internal record
+    int idx, obase;             // its record and the first record of the octant's table
+    Pend<float> pd;
+    bool done;
+    int steps, fallbacks;
+    SKG_D int nscanned() const { return steps; }   // one rope followed per step
+    int cell0;
+    float rho;                  // density of the last segment's cell
+
+    SKG_D void load(const DevGrid& g) {
+        const uint4* p = g.orec + 2 * (size_t)(unsigned)idx;
+        uint32_t a0, a1, a2, a3, a4, a5, a6, a7;
+        asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3), "=r"(a4), "=r"(a5), "=r"(a6), "=r"(a7) : "l"(p));
+        wx = __uint_as_float(a0); wy = __uint_as_float(a1); wz = __uint_as_float(a2); wrho = __uint_as_float(a3);
+        gx_ = (int)a4; gy_ = (int)a5; gz_ = (int)a6;
+    }
+    // does cell c hold the point? (its lattice record)
+    SKG_D static bool holds(const DevGrid& g, int c, float px, float py, float pz) {
+        const uint4 a = __ldg(g.prec + 2 * (size_t)c);
+        return TreeLatticeStepper<float>::within(TreeLatticeStepper<float>::code_x(a), px, g.lorg[0], g.lunit[0]) &&
+               TreeLatticeStepper<float>::within(TreeLatticeStepper<float>::code_y(a), py, g.lorg[1], g.lunit[1]) &&
+               TreeLatticeStepper<float>::within(TreeLatticeStepper<float>::code_z(a), pz, g.lorg[2], g.lunit[2]);
+    }
+    static constexpr bool resumable = false;
+
+    SKG_D void init(const DevGrid& g, float rx, float ry, float rz, float dx, float dy, float dz, int hint = -1) {
+        kx = dx; ky = dy; kz = dz; pd.clear(); done = false; steps = 0; fallbacks = 0;
+        cell0 = -1; rho = -1.f;
+        ux = (fabsf(kx) > 1e-15f) ? 1.f / kx : 0.f; bx = ux != 0.f ? 0.f : FLT_MAX;
+        uy = (fabsf(ky) > 1e-15f) ? 1.f / ky : 0.f; by = uy != 0.f ? 0.f : FLT_MAX;
+        uz = (fabsf(kz) > 1e-15f) ? 1.f / kz : 0.f; bz = uz != 0.f ? 0.f : FLT_MAX;
+        obase = ((kx < 0.f ? 1 : 0) + (ky < 0.f ? 2 : 0) + (kz < 0.f ? 4 : 0)) * g.ncells;
+        int c;
+        if (hint >= 0 && holds(g, hint, rx, ry, rz)) {
+            c = hint; cell0 = hint;
+        } else {
+            c = move_inside<float>(g, g.epsf, rx, ry, rz, kx, ky, kz, pd) ? TreeStepper<float>::locate(g, rx, ry, rz) : -1;
+            if (c < 0) { pd.n = 0; done = true; return; }
+            if (pd.n == 0) cell0 = c;
+        }
+        idx = obase + c;
+        load(g);
+        x = rx; y = ry; z = rz;
+    }
+
+    SKG_D bool next(const DevGrid& g, int& m, float& ds) {
+        if (pd.pop(ds)) { m = -1; rho = 0.f; return true; }
+        return walk(g, m, ds);
+    }
+    SKG_D bool walk(const DevGrid& g, int& m, float& ds) {
+        while (!done) {
+            if (++steps > g.max_steps) { done = true; return false; }
+            // FLT_MAX on an axis that is never crossed: (w - p) * 0 + FLT_MAX
+            const float dsx = fmaf(wx - x, ux, bx), dsy = fmaf(wy - y, uy, by), dsz = fmaf(wz - z, uz, bz);
+            const bool px = dsx <= dsy && dsx <= dsz, py = !px && dsy <= dsz, pz = !px && !py;
+            float d = px ? dsx : py ? dsy : dsz;
+            const int rp = px ? gx_ : py ? gy_ : gz_;
+            const float lim = d + g.epsf;
+            m = idx - obase;
+            rho = wrho;
+            x += lim * kx; y += lim * ky; z += lim * kz;
+            const bool on_face = (px || dsx >= lim) && (py || dsy >= lim) && (pz || dsz >= lim);
+            if (rp >= 0 && on_face) {              // the leaf behind the exit wall holds the point
+                idx = rp; d = lim;
+                load(g);
+            } else {
+                int next = rp >= 0 ? rp - obase : rp == -1 ? -1 : TreeStepper<float>::descend(g, rp, x, y, z);
+                if (rp != -1 && (next < 0 || (!on_face && !holds(g, next, x, y, z)))) {
+                    next = TreeStepper<float>::locate(g, x, y, z); fallbacks++;
+                }
+                if (next == m) {                   // stuck (TreeDustGrid.cpp:476-493)
+                    x = nextafterf(x, (kx < 0.f) ? -FLT_MAX : FLT_MAX);
+                    y = nextafterf(y, (ky < 0.f) ? -FLT_MAX : FLT_MAX);
+                    z = nextafterf(z, (kz < 0.f) ? -FLT_MAX : FLT_MAX);
+                    next = TreeStepper<float>::locate(g, x, y, z);
+                    if (next == m) next = -1;
+                }
+                if (next < 0) done = true;
+                else { idx = obase + next; d = lim; load(g); }
+            }
             if (d > 0.f) { ds = d; return true; }
         }
         return false;

@@ -38,6 +38,7 @@ cudaError_t launch_emission_sources(const DevScene* dS, int nlambda, int ncells,
                                     cudaStream_t s);
 size_t emission_scan_scratch_bytes(int ncells);
 cudaError_t launch_sum(const double* x, int64_t n, double* out, cudaStream_t s);
+cudaError_t launch_octant_records(const DevGrid& g, void* out, cudaStream_t s);   // out: 16 uint4 per cell
 cudaError_t launch_embed_density(const DevGrid& g, const float* rhof, cudaStream_t s);
 
 // skg_host.cpp

@@ -212,6 +212,35 @@ cudaError_t launch_embed_density(const DevGrid& g, const float* rhof, cudaStream
     return cudaGetLastError();
 }
 
+// The octant records of a lattice tree from its leaf records (density embedded): for octant o of the
+// direction (bit a set: k_a < 0) and cell m, record o * ncells + m holds the walls ahead on x, y, z,
+// the density, and the ropes of those walls (a record of the same octant, -1 outside, <= -2 an
+// internal record).
+__global__ void octant_records_kernel(const DevGrid g, uint4* out) {
+    using L = TreeLatticeStepper<float>;
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= g.ncells) return;
+    L st;
+    st.load(g, m);
+    const uint32_t c[3] = {L::code_x(st.a), L::code_y(st.a), L::code_z(st.a)};
+    for (int o = 0; o < 8; o++) {
+        uint32_t w[3], r[3];
+        for (int a = 0; a < 3; a++) {
+            const bool up = !(o >> a & 1);
+            w[a] = __float_as_uint(L::wall(c[a], up, g.lorg[a], g.lunit[a]));
+            const int rp = st.rope(2 * a + (up ? 1 : 0));
+            r[a] = (uint32_t)(rp >= 0 ? rp + o * g.ncells : rp);
+        }
+        uint4* p = out + 2 * ((size_t)o * g.ncells + m);
+        p[0] = make_uint4(w[0], w[1], w[2], st.a.x);
+        p[1] = make_uint4(r[0], r[1], r[2], 0);
+    }
+}
+cudaError_t launch_octant_records(const DevGrid& g, void* out, cudaStream_t s) {
+    octant_records_kernel<<<(g.ncells + 127) / 128, 128, 0, s>>>(g, (uint4*)out);
+    return cudaGetLastError();
+}
+
 // Sum of a vector (absorbed-luminosity totals for the self-absorption convergence test).
 __global__ void sum_kernel(const double* __restrict__ x, int64_t n, double* out) {
     __shared__ double sh[256];

@@ -55,6 +55,12 @@ namespace skg {
 #ifndef SKG_VOR_PATH_MIN_BLOCKS
 #define SKG_VOR_PATH_MIN_BLOCKS 3
 #endif
+#ifndef SKG_OCT_PATH_BLOCKS
+#define SKG_OCT_PATH_BLOCKS 4
+#endif
+#ifndef SKG_OCT_PEEL_BLOCKS
+#define SKG_OCT_PEEL_BLOCKS 4
+#endif
 #ifndef SKG_PEEL_MIN_BLOCKS
 #define SKG_PEEL_MIN_BLOCKS 4
 #endif
@@ -957,6 +963,8 @@ SKG_D bool resume_ckpt(const WaveParams& W, const DevGrid& g, int p, int nck, do
 template<int MODE, template<typename> class Stepper> struct TravBlocks { static constexpr int value = SKG_TRAV_MIN_BLOCKS; };
 template<template<typename> class Stepper> struct TravBlocks<1, Stepper> { static constexpr int value = SKG_PATH_MIN_BLOCKS; };
 template<> struct TravBlocks<1, VoronoiStepper> { static constexpr int value = SKG_VOR_PATH_MIN_BLOCKS; };
+template<> struct TravBlocks<1, TreeOctantStepper> { static constexpr int value = SKG_OCT_PATH_BLOCKS; };
+template<> struct TravBlocks<2, TreeOctantStepper> { static constexpr int value = SKG_OCT_PEEL_BLOCKS; };
 template<template<typename> class Stepper> struct TravBlocks<2, Stepper> { static constexpr int value = SKG_PEEL_MIN_BLOCKS; };
 
 template<typename R, template<typename> class Stepper, int MODE, bool ONE>
@@ -1467,6 +1475,7 @@ PassFns pick(int grid_type, int tree_walk, int precision, bool one) {
     case SKG_GRID_BINTREE:
         if (f64) return fns<double, TreeStepper>();
         if (tree_walk == TW_NODES) return fns<float, TreeNodeWalk>();
+        if (tree_walk == TW_OCTANT) return fns32<TreeOctantStepper>(one);
         if (tree_walk == TW_LATTICE) return fns32<TreeLatticeStepper>(one);
         return fns32<TreeStepper>(one);
     default:
