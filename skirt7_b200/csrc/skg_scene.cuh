@@ -129,7 +129,8 @@ struct __align__(16) Packet {
     double x, y, z;                   // position (rounded to the traversal precision)
     double kx, ky, kz;                // direction
     double L, Lth;                    // luminosity and its termination threshold
-    double s_int;                     // distance to the interaction point (result of the path job)
+    double s_int;                     // distance to the interaction point (before its re-walk: the
+                                      // interaction optical depth)
     uint64_t id;                      // packet number within its work item (RNG counter words)
     int item;                         // work item
     int ell;
@@ -140,9 +141,21 @@ struct __align__(16) Packet {
     int state;                        // PacketState
     int flags;                        // bit 0 stellar origin, bit 1 the pending peel-offs follow a scattering
     int peel_j0, peel_n;              // this packet's peel-off jobs of the last wave
-    int pad[2];
+    int nck;                          // checkpoints of the path walk
+    int pad;
 };
 static_assert(sizeof(Packet) == 128, "packet record is two 64-byte lines");
+
+// Counters of a wave's jobs and lists.
+enum JobCount : int {
+    J_PATH = 0,                       // path jobs
+    J_PEEL,                           // peel-off jobs
+    J_BUSY,                           // packets with jobs
+    J_FREE, J_INT,                    // records on the free list, on the interaction list
+    J_REWALK,                         // packets on the re-walk list
+    J_TAKEN_PATH, J_TAKEN_TAU, J_TAKEN_REWALK,   // jobs taken by each walk
+    J_N = 16
+};
 
 struct WaveParams {
     RunParams R;
@@ -154,17 +167,17 @@ struct WaveParams {
     int2* jobs;                       // (packet, type)
     double* jtau;                     // peel-off optical depth
     double* jL;                       // peel-off luminosity
-    unsigned* jcount;                 // [0] path jobs, [1] peel-off jobs, [2] jobs taken by the
-                                      // traversal pass (its path kernel when split), [3] packets
-                                      // with jobs, [4] peel-off jobs taken by a split pass,
-                                      // [5] records on the free list, [6] on the interaction list
+    unsigned* jcount;                 // counters of this wave (JobCount)
     // the previous wave's jobs (peel-off detection)
     const int2* pjobs;
     const double* pjtau;
     const double* pjL;
     unsigned* last_busy;              // highest wave index that had jobs
-    int* freelist;                    // records the event pass freed (count: jcount[5])
-    int* intlist;                     // records it found at their interaction point (jcount[6])
+    int* freelist;                    // records the event pass freed (J_FREE)
+    int* intlist;                     // records it found at their interaction point (J_INT)
+    int* rlist;                       // packets that interact on their path (J_REWALK; the free list's
+                                      // memory, which the launch pass has consumed)
+    int path_tau;                     // the path jobs need the optical depth alone (walked with the peel-offs)
     float4* ckpt;                     // per packet record: checkpoints of its path walk
     // walk order of the wave's jobs (order_kernel); hist == nullptr: as appended
     unsigned* hist;                   // [2][JOB_BINS] jobs per bin: path jobs, peel-off jobs (zero between waves)

@@ -45,24 +45,12 @@ namespace skg {
 #ifndef SKG_TRAV_MIN_BLOCKS
 #define SKG_TRAV_MIN_BLOCKS 4
 #endif
-// The traversal pass as two kernels: the path jobs, then the peel-off jobs in an instantiation
-// that holds the optical depth alone (no spills at 64 registers).  Octree disk, 10^7 packets:
-// 202.5 ms against 214.2 ms for one kernel over both (Voronoi disk: 1357 against 1421 ms); the
-// peel-off kernel at 5 or 6 blocks per SM (48 or 40 registers, spilling) is slower (219, 240 ms).
-#ifndef SKG_PATH_MIN_BLOCKS
-#define SKG_PATH_MIN_BLOCKS 4
-#endif
+// The walks of a wave run in kernels of their own (TravMode below): each holds the registers of its
+// own state alone, and the path's long end (path_end_kernel) holds none of them.  Octree disk, 2*10^7
+// packets: traversal pass 179.6 ms against 209.8 with the end of the path and the re-walk inside the
+// path-job kernel (220 bytes of spills at 64 registers); fit-variant batch 46.2 against 53.5 ms.
 #ifndef SKG_VOR_PATH_MIN_BLOCKS
 #define SKG_VOR_PATH_MIN_BLOCKS 3
-#endif
-#ifndef SKG_OCT_PATH_BLOCKS
-#define SKG_OCT_PATH_BLOCKS 4
-#endif
-#ifndef SKG_OCT_PEEL_BLOCKS
-#define SKG_OCT_PEEL_BLOCKS 4
-#endif
-#ifndef SKG_PEEL_MIN_BLOCKS
-#define SKG_PEEL_MIN_BLOCKS 4
 #endif
 // programmatic dependent launch of the peel-off-job kernel after the path-job kernel
 #ifndef SKG_PDL
@@ -92,16 +80,6 @@ namespace skg {
 // octree disk: traversal pass 275 ms against 336 ms at 1 per 10^7 packets)
 #ifndef SKG_REFILL_LANES
 #define SKG_REFILL_LANES 8
-#endif
-// lanes whose path walk ended run the end of the path (escape fraction, termination test, the
-// interaction sampling: long, divergent FP64 code) once this many lanes of the warp wait for it,
-// or no lane is walking.  Per 10^7 packets, traversal pass at 1 / 4 / 8 / 16: octree disk 193 /
-// 176 / 170 / 174 ms; at 1 / 8: Cartesian 95 / 71 ms, k-d tree 224 / 201 ms, Voronoi 1212 / 1186 ms.
-#ifndef SKG_AFTER_LANES
-#define SKG_AFTER_LANES 8
-#endif
-#ifndef SKG_REFILL_PEEL
-#define SKG_REFILL_PEEL SKG_REFILL_LANES
 #endif
 // checkpoints of a path's walk (FP32 steppers that can resume): every SKG_CKPT_STRIDE cell steps,
 // up to SKG_CKPT_N per packet record, the walk stores its state with the optical depth and path
@@ -594,14 +572,14 @@ SKG_D void append_jobs(const WaveParams& W, int p, Packet& K, int npeel, int nma
     const int totm = __shfl_sync(FULL, inm, 31), totp = __shfl_sync(FULL, inp, 31);
     unsigned bm = 0, bp = 0;
     if (lane == 31) {
-        if (totm > 0) bm = atomicAdd(W.jcount, (unsigned)totm);
-        if (totp > 0) bp = atomicAdd(W.jcount + 1, (unsigned)totp);
+        if (totm > 0) bm = atomicAdd(W.jcount + J_PATH, (unsigned)totm);
+        if (totp > 0) bp = atomicAdd(W.jcount + J_PEEL, (unsigned)totp);
     }
     bm = __shfl_sync(FULL, bm, 31);
     bp = __shfl_sync(FULL, bp, 31);
     const unsigned busy = __ballot_sync(FULL, npeel + nmain > 0);
     if (lane == 0 && busy) {
-        atomicAdd(W.jcount + 3, (unsigned)__popc(busy));
+        atomicAdd(W.jcount + J_BUSY, (unsigned)__popc(busy));
         atomicMax(W.last_busy, (unsigned)W.wave);
     }
     if (npeel > 0) {
@@ -684,7 +662,7 @@ __global__ void __launch_bounds__(SKG_EVENT_THREADS, SKG_EVENT_MIN_BLOCKS * 256 
         if (im) {
             const int leader = __ffs(im) - 1;
             unsigned base = 0;
-            if (lane == leader) base = atomicAdd(W.jcount + 6, (unsigned)__popc(im));
+            if (lane == leader) base = atomicAdd(W.jcount + J_INT, (unsigned)__popc(im));
             base = __shfl_sync(FULL, base, leader);
             if (inter) W.intlist[base + __popc(im & ((1u << lane) - 1))] = p;
         }
@@ -703,7 +681,7 @@ __global__ void __launch_bounds__(SKG_EVENT_THREADS, SKG_EVENT_MIN_BLOCKS * 256 
         if (fm) {
             const int leader = __ffs(fm) - 1;
             unsigned base = 0;
-            if (lane == leader) base = atomicAdd(W.jcount + 5, (unsigned)__popc(fm));
+            if (lane == leader) base = atomicAdd(W.jcount + J_FREE, (unsigned)__popc(fm));
             base = __shfl_sync(FULL, base, leader);
             if (freed) W.freelist[base + __popc(fm & ((1u << lane) - 1))] = p;
         }
@@ -755,7 +733,7 @@ __global__ void __launch_bounds__(SKG_EVENT_THREADS) launch_kernel(const WavePar
     const int phase = H.phase;
     const bool peel_on = phase != SKG_PHASE_DUST_SELFABS;
     const int lane = threadIdx.x & 31;
-    const unsigned nint = W.jcount[6];
+    const unsigned nint = W.jcount[J_INT];
     for (unsigned b0 = blockIdx.x * blockDim.x; b0 < nint; b0 += gridDim.x * blockDim.x) {
         const unsigned i = b0 + threadIdx.x;
         const bool mine = i < nint;
@@ -776,7 +754,7 @@ __global__ void __launch_bounds__(SKG_EVENT_THREADS) launch_kernel(const WavePar
             W.pk[p] = K;
         }
     }
-    const unsigned nfree = W.jcount[5];
+    const unsigned nfree = W.jcount[J_FREE];
     for (unsigned b0 = blockIdx.x * blockDim.x; b0 < nfree; b0 += gridDim.x * blockDim.x) {
         const unsigned i = b0 + threadIdx.x;
         const bool mine = i < nfree;
@@ -833,7 +811,7 @@ __global__ void __launch_bounds__(1024) bins_kernel(unsigned* hist, unsigned* bi
 
 // Writes the jobs in walk order.
 __global__ void __launch_bounds__(256) order_kernel(const WaveParams W) {
-    const unsigned nmain = W.jcount[0], npeel = W.jcount[1];
+    const unsigned nmain = W.jcount[J_PATH], npeel = W.jcount[J_PEEL];
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nmain + npeel; i += gridDim.x * blockDim.x) {
         if (i < nmain) {
             const uint2 k = W.jkey[i];
@@ -955,17 +933,18 @@ SKG_D bool resume_ckpt(const WaveParams& W, const DevGrid& g, int p, int nck, do
     return true;
 }
 
-// MODE: 1 the path jobs; 2 the peel-off jobs (a lean instantiation: optical depth alone, no path
-// state)
-// Resident blocks per SM of each instantiation.  The Voronoi path-job kernel runs at 3 blocks (80
-// registers, no spills: its neighbour scan keeps more state): 1219 against 1273 ms per 10^7-packet
-// phase; the tree and Cartesian ones are faster at 4 (189 against 194 ms, 94 against 100 ms).
+// The walks of a wave, each in an instantiation that holds its own state alone:
+//   TRAV_PATH    the path jobs of phases that keep absorption or of several dust components (and, on
+//                steppers that resume, of every phase: they write checkpoints)
+//   TRAV_TAU     jobs that need the optical depth alone: the peel-offs, and the path jobs otherwise
+//   TRAV_REWALK  the paths that interact, to the interaction optical depth
+enum TravMode : int { TRAV_PATH = 1, TRAV_TAU = 2, TRAV_REWALK = 3 };
+// Resident blocks per SM of each instantiation.
 template<int MODE, template<typename> class Stepper> struct TravBlocks { static constexpr int value = SKG_TRAV_MIN_BLOCKS; };
-template<template<typename> class Stepper> struct TravBlocks<1, Stepper> { static constexpr int value = SKG_PATH_MIN_BLOCKS; };
-template<> struct TravBlocks<1, VoronoiStepper> { static constexpr int value = SKG_VOR_PATH_MIN_BLOCKS; };
-template<> struct TravBlocks<1, TreeOctantStepper> { static constexpr int value = SKG_OCT_PATH_BLOCKS; };
-template<> struct TravBlocks<2, TreeOctantStepper> { static constexpr int value = SKG_OCT_PEEL_BLOCKS; };
-template<template<typename> class Stepper> struct TravBlocks<2, Stepper> { static constexpr int value = SKG_PEEL_MIN_BLOCKS; };
+template<> struct TravBlocks<TRAV_PATH, VoronoiStepper> { static constexpr int value = SKG_VOR_PATH_MIN_BLOCKS; };
+
+template<typename R, template<typename> class Stepper>
+struct HasCkpt { static constexpr bool value = SKG_CKPT && Resumable<Stepper<R>>::value; };
 
 template<typename R, template<typename> class Stepper, int MODE, bool ONE>
 __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_kernel(const WaveParams W) {
@@ -987,30 +966,29 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
 #if SKG_PDL
     // the path-job kernel lets the peel-off-job kernel of the same wave be scheduled now: its blocks
     // become resident as this kernel's blocks run out of jobs and exit, so the two overlap in the
-    // tail of this one.  The peel-off kernel reads only what the event pass wrote (complete before
+    // tail of this one.  The peel-off kernel reads only what the launch pass wrote (complete before
     // this kernel started); the one word both may touch, a packet's start cell, is written here
     // only from "unknown" to the cell, and either value is a valid hint for the peel-off walk.
-    if (MODE == 1) asm volatile("griddepcontrol.launch_dependents;");
+    if (MODE == TRAV_PATH) asm volatile("griddepcontrol.launch_dependents;");
 #endif
-    const unsigned njobs = W.jcount[MODE == 1 ? 0 : 1];
-    unsigned* const taken = W.jcount + (MODE == 2 ? 4 : 2);
+    const unsigned npath = (MODE == TRAV_PATH || (MODE == TRAV_TAU && W.path_tau)) ? W.jcount[J_PATH] : 0;
+    const unsigned njobs = MODE == TRAV_PATH ? npath : MODE == TRAV_TAU ? npath + W.jcount[J_PEEL] : W.jcount[J_REWALK];
+    unsigned* const taken = W.jcount + (MODE == TRAV_PATH ? J_TAKEN_PATH : MODE == TRAV_TAU ? J_TAKEN_TAU : J_TAKEN_REWALK);
     const int phase = H.phase;
     const int lane = threadIdx.x & 31;
-    const int refill_lanes = P.refill > 0 ? P.refill : (MODE == 2 ? SKG_REFILL_PEEL : SKG_REFILL_LANES);
+    const int refill_lanes = P.refill > 0 ? P.refill : SKG_REFILL_LANES;
+    constexpr bool CKPT = HasCkpt<R, Stepper>::value;
 
-    int j = -1;                       // the lane's job (-1: none)
+    int j = -1;                       // where the lane's job leaves its result (-1: no job)
     int p = 0, slot = 0, ell = 0;
-    int kind = 0;                     // 0 peel-off, 1 path, 2 re-walk to the interaction point
     double tau = 0;                   // optical depth walked
-    // values of one job kind share two registers -- path: v1 = L e^-tau (the luminosity that
-    // reaches the current cell, kept as a running product: one expm1 per absorbing cell step),
-    // v2 = L_sca (several dust components); re-walk: v1 = path length walked, v2 = the
-    // interaction optical depth
+    // TRAV_PATH: v1 = L e^-tau (the luminosity that reaches the current cell, kept as a running
+    // product: one expm1 per absorbing cell step), v2 = L_sca (several dust components);
+    // TRAV_REWALK: v1 = path length walked, v2 = the interaction optical depth
     double v1 = 0, v2 = 0;
     float kext1 = -1.f;               // kappa_ext at the job's wavelength (one dust component), else -1
     unsigned c_steps = 0;
     Stepper<R> st;
-    constexpr bool CKPT = SKG_CKPT && MODE != 2 && Resumable<Stepper<R>>::value;
     int nck = 0;                      // checkpoints of the path walk
 
     while (true) {
@@ -1018,35 +996,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
         const unsigned live = __activemask();
         const bool need = j < 0;
         const unsigned want = __ballot_sync(live, need);
-        // lanes whose path walk ended (kind 3) run the end of the path together
-        const unsigned pend = (MODE == 2) ? 0u : __ballot_sync(live, kind == 3);
-        const bool idle = (live & ~want & ~pend) == 0;      // no lane of the warp is walking
-        if (pend && (__popc(pend) >= SKG_AFTER_LANES || idle)) {
-            if (kind == 3) {
-                const DevGrid& g = grid_of(slot);
-                const DevScene& S = *s_scene[slot];
-                double L = W.pk[p].L, tau_int = 0;      // the packet's luminosity at the path start
-                const int rc = after_path(W, S, p, phase, ell, tau, v2, L, tau_int);
-                if (rc == 1) {
-                    kind = 2; v2 = tau_int;
-                    bool resumed = false;
-                    if constexpr (CKPT) resumed = W.ckpt && resume_ckpt(W, g, p, nck, tau_int, st, tau, v1);
-                    if (!resumed) {
-                        const Packet& K = W.pk[p];
-                        st.init(g, (R)K.x, (R)K.y, (R)K.z, (R)K.kx, (R)K.ky, (R)K.kz, K.pos_cell);
-                        tau = 0; v1 = 0;
-                        R d0;
-                        while (st.pd.pop(d0)) v1 += (double)d0;
-                    }
-                } else {
-                    if (rc < 0) atomicAdd(&s_cnt[C_ERR], 1ull);
-                    j = -1;
-                    kind = 0;
-                }
-            }
-            continue;
-        }
-        if (want && (__popc(want) >= refill_lanes || (live & ~want & ~pend) == 0)) {
+        if (want && (__popc(want) >= refill_lanes || want == live)) {
             const int leader = __ffs(want) - 1;
             unsigned base = 0;
             if (lane == leader) base = atomicAdd(taken, (unsigned)__popc(want));
@@ -1054,103 +1004,106 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
             if (need) {
                 const unsigned jj = base + __popc(want & ((1u << lane) - 1));
                 if (jj >= njobs) break;
-                int2 jb;
-                if (MODE == 1) {
+                int grp = JOB_MAIN;
+                if (MODE == TRAV_REWALK) {
                     j = (int)jj;
-                    jb = W.hist ? make_int2(W.spath[jj], JOB_MAIN) : W.jobs[j];
+                    p = W.rlist[jj];
+                } else if (MODE == TRAV_PATH || jj < npath) {
+                    j = (int)jj;
+                    p = W.hist ? W.spath[jj] : W.jobs[jj].x;
                 } else if (W.hist) {
-                    const int4 o = W.speel[jj];
-                    jb = make_int2(o.x, o.y);
-                    j = o.z;
+                    const int4 o = W.speel[jj - npath];
+                    p = o.x; grp = o.y; j = o.z;
                 } else {
-                    j = W.npool + (int)jj;
-                    jb = W.jobs[j];
+                    j = W.npool + (int)(jj - npath);
+                    const int2 jb = W.jobs[j];
+                    p = jb.x; grp = jb.y;
                 }
-                p = jb.x;
                 const Packet& K = W.pk[p];
                 ell = K.ell;
                 slot = P.items[K.item].slot;
                 const DevScene& S = *s_scene[slot];
+                const DevGrid& g = grid_of(slot);
                 const int hint = K.pos_cell;
                 kext1 = (S.ncomp == 1) ? (float)S.kext[ell] : -1.f;
-                R kx, ky, kz;
-                if (MODE != 2 && jb.y == JOB_MAIN) { kx = (R)K.kx; ky = (R)K.ky; kz = (R)K.kz; kind = 1; v1 = K.L; v2 = 0; nck = 0; }
-                else { kx = (R)S.gkx[jb.y]; ky = (R)S.gky[jb.y]; kz = (R)S.gkz[jb.y]; kind = 0; }
-                st.init(grid_of(slot), (R)K.x, (R)K.y, (R)K.z, kx, ky, kz, hint);
-                if (kind == 1 && hint == -2) W.pk[p].pos_cell = st.cell0;
                 tau = 0;
                 // entry segments outside the grid (m = -1) carry no optical depth: only the
                 // re-walk, which measures length, takes them
+                if (MODE == TRAV_REWALK) {
+                    v1 = 0; v2 = K.s_int;
+                    bool resumed = false;
+                    if constexpr (CKPT) resumed = W.ckpt && resume_ckpt(W, g, p, K.nck, v2, st, tau, v1);
+                    if (!resumed) {
+                        st.init(g, (R)K.x, (R)K.y, (R)K.z, (R)K.kx, (R)K.ky, (R)K.kz, hint);
+                        R d0;
+                        while (st.pd.pop(d0)) v1 += (double)d0;
+                    }
+                } else {
+                    R kx, ky, kz;
+                    if (MODE == TRAV_PATH || grp == JOB_MAIN) { kx = (R)K.kx; ky = (R)K.ky; kz = (R)K.kz; }
+                    else { kx = (R)S.gkx[grp]; ky = (R)S.gky[grp]; kz = (R)S.gkz[grp]; }
+                    st.init(g, (R)K.x, (R)K.y, (R)K.z, kx, ky, kz, hint);
+                    if ((MODE == TRAV_PATH || grp == JOB_MAIN) && hint == -2) W.pk[p].pos_cell = st.cell0;
+                    if (MODE == TRAV_PATH) { v1 = K.L; v2 = 0; nck = 0; }
+                }
             }
         }
 
-        if (j < 0 || kind == 3) continue;   // waiting for enough lanes to refill / end paths together
+        if (j < 0) continue;            // waiting for enough lanes to refill
 
         const DevGrid& g = grid_of(slot);
         const DevScene& S = *s_scene[slot];
-        // one cell step of the job (m, ds, its optical depth); true when it ended the job (a re-walk
-        // that reached the interaction optical depth)
-        auto take_step = [&](int m, R ds, double dtau) -> bool {
-            c_steps++;
-            if (kind == 0) {
-                tau += dtau;
-            } else if (kind == 1) {
-                if (absorb_step<R>(S, phase, m, ell, dtau, v1, v2)) atomicAdd(&s_cnt[C_ABS], 1ull);
-                tau += dtau;
-                if constexpr (CKPT) {
-                    if (W.ckpt && nck < SKG_CKPT_N && st.steps >= (nck + 1) * SKG_CKPT_STRIDE && !st.done) {
-                        save_ckpt(W, p, nck, st, tau);
-                        nck++;
-                    }
-                }
-            } else {
-                const double tn = tau + dtau, sn = v1 + (double)ds;
-                if (tn > v2) {
-                    Packet& K = W.pk[p];
-                    K.s_int = v1 + ((v2 - tau) / (tn - tau)) * (sn - v1);
-                    K.int_cell = m;
-                    K.state = PK_INTERACT;
-                    atomicAdd(&s_cnt[C_TRAV], 1ull);
-                    atomicAdd(&s_cnt[C_NBR], (unsigned long long)st.nscanned());
-                    atomicAdd(&s_cnt[C_FB], (unsigned long long)st.fallbacks);
-                    j = -1;
-                    return true;
-                }
-                tau = tn; v1 = sn;
-            }
-            return false;
-        };
-        // the traversal reached the edge of the grid
-        auto at_edge = [&]() {
-            atomicAdd(&s_cnt[C_TRAV], 1ull);
-            atomicAdd(&s_cnt[C_NBR], (unsigned long long)st.nscanned());
-            atomicAdd(&s_cnt[C_FB], (unsigned long long)st.fallbacks);
-            if (st.steps > g.max_steps) { atomicOr(P.err, ERR_STEP_BUDGET); atomicAdd(&s_cnt[C_ERR], 1ull); }
-            if (kind == 0) {
-                W.jtau[j] = tau;
-                j = -1;
-            } else if (kind == 1) {
-                kind = 3;                       // the end of the path runs with other lanes' (above)
-            } else {
-                // DustGridPath::pathlength: an optical depth beyond the last segment gives the full length
-                Packet& K = W.pk[p];
-                K.s_int = v1; K.int_cell = -1; K.state = PK_INTERACT;
-                j = -1;
-            }
-        };
-
-        // cell steps: up to SKG_INNER_STEPS of them before the warp looks at refills again.  (Walking
+        // cell steps: several of them before the warp looks at refills again.  (Walking
         // four steps ahead and loading their densities together, for the walks whose records do
         // not carry the density, was slower: Cartesian traversal pass 83 against 64 ms, Voronoi
         // peel-off walks 298 against 258 ms; the walk is issue-bound, not waiting on those loads.)
 #pragma unroll 1
-        for (int is = 0; is < (MODE == 2 ? SKG_INNER_STEPS : SKG_INNER_PATH); is++) {
+        for (int is = 0; is < (MODE == TRAV_PATH ? SKG_INNER_PATH : SKG_INNER_STEPS); is++) {
             int m; R ds;
             if (st.walk(g, m, ds)) {
-                // one dust component: the FP32 tree walk carries the cell density in its leaf record
-                if (take_step(m, ds, step_dtau<R>(S, st, kext1, m, ell, ds))) break;
+                c_steps++;
+                const double dtau = step_dtau<R>(S, st, kext1, m, ell, ds);
+                if (MODE == TRAV_TAU) {
+                    tau += dtau;
+                } else if (MODE == TRAV_PATH) {
+                    if (absorb_step<R>(S, phase, m, ell, dtau, v1, v2)) atomicAdd(&s_cnt[C_ABS], 1ull);
+                    tau += dtau;
+                    if constexpr (CKPT) {
+                        if (W.ckpt && nck < SKG_CKPT_N && st.steps >= (nck + 1) * SKG_CKPT_STRIDE && !st.done) {
+                            save_ckpt(W, p, nck, st, tau);
+                            nck++;
+                        }
+                    }
+                } else {
+                    const double tn = tau + dtau, sn = v1 + (double)ds;
+                    if (tn > v2) {
+                        Packet& K = W.pk[p];
+                        K.s_int = v1 + ((v2 - tau) / (tn - tau)) * (sn - v1);
+                        K.int_cell = m;
+                        K.state = PK_INTERACT;
+                        atomicAdd(&s_cnt[C_TRAV], 1ull);
+                        atomicAdd(&s_cnt[C_NBR], (unsigned long long)st.nscanned());
+                        atomicAdd(&s_cnt[C_FB], (unsigned long long)st.fallbacks);
+                        j = -1;
+                        break;
+                    }
+                    tau = tn; v1 = sn;
+                }
             } else {
-                at_edge();
+                // the traversal reached the edge of the grid
+                atomicAdd(&s_cnt[C_TRAV], 1ull);
+                atomicAdd(&s_cnt[C_NBR], (unsigned long long)st.nscanned());
+                atomicAdd(&s_cnt[C_FB], (unsigned long long)st.fallbacks);
+                if (st.steps > g.max_steps) { atomicOr(P.err, ERR_STEP_BUDGET); atomicAdd(&s_cnt[C_ERR], 1ull); }
+                if (MODE == TRAV_REWALK) {
+                    // DustGridPath::pathlength: an optical depth beyond the last segment gives the full length
+                    Packet& K = W.pk[p];
+                    K.s_int = v1; K.int_cell = -1; K.state = PK_INTERACT;
+                } else {
+                    W.jtau[j] = tau;
+                    if (MODE == TRAV_PATH) { W.jL[j] = v2; if (CKPT) W.pk[p].nck = nck; }
+                }
+                j = -1;
                 break;
             }
         }
@@ -1161,9 +1114,41 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
     if (threadIdx.x < C_N && s_cnt[threadIdx.x]) atomicAdd(P.counters + threadIdx.x, s_cnt[threadIdx.x]);
 #if SKG_PDL
     // the peel-off kernel completes only after the path-job kernel it overlapped (and its writes
-    // are visible), so the next wave's event pass, ordered after this kernel, sees both
-    if (MODE == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // are visible), so what follows it in the stream sees both
+    if (MODE == TRAV_TAU) asm volatile("griddepcontrol.wait;" ::: "memory");
 #endif
+}
+
+// The ends of the wave's paths, one thread per path job in walk order: escape fraction, termination
+// test and interaction optical depth (after_path); the packets that interact go on the re-walk list.
+// In a kernel of its own every lane of a warp does this long FP64 work at once, and the walks need
+// no registers for it.
+__global__ void __launch_bounds__(128) path_end_kernel(const WaveParams W) {
+    const RunParams& P = W.R;
+    const unsigned n = W.jcount[J_PATH];
+    const int lane = threadIdx.x & 31;
+    const int phase = P.hdr->phase;
+    for (unsigned b0 = blockIdx.x * blockDim.x; b0 < n; b0 += gridDim.x * blockDim.x) {
+        const unsigned i = b0 + threadIdx.x;
+        bool again = false;
+        int p = 0;
+        if (i < n) {
+            p = W.hist ? W.spath[i] : W.jobs[i].x;
+            Packet& K = W.pk[p];
+            const DevScene& S = *P.scenes[P.items[K.item].slot];
+            double L = K.L, tau_int = 0;
+            const int rc = after_path(W, S, p, phase, K.ell, W.jtau[i], W.path_tau ? 0.0 : W.jL[i], L, tau_int);
+            if (rc < 0) atomicAdd(P.counters + C_ERR, 1ull);
+            if (rc == 1) { K.s_int = tau_int; again = true; }
+        }
+        const unsigned am = __ballot_sync(0xffffffffu, again);
+        if (am) {
+            unsigned base = 0;
+            if (lane == 0) base = atomicAdd(W.jcount + J_REWALK, (unsigned)__popc(am));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (again) W.rlist[base + __popc(am & ((1u << lane) - 1))] = p;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1369,6 +1354,16 @@ __global__ void __launch_bounds__(128) tail_kernel(const WaveParams W) {
 
 namespace {
 
+int dev_sms() {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return sms;
+}
+
 // Resident blocks of a traversal instantiation (persistent grid = this many blocks per SM x SMs).
 template<typename R, template<typename> class Stepper, int MODE, bool ONE>
 int resident_blocks(size_t smem) {
@@ -1425,24 +1420,26 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
     }
 #endif
     if (mid) cudaEventRecord(mid, s);
-    // the path jobs, then the peel-off jobs in their lean kernel
-    trav_kernel<R, Stepper, 1, ONE><<<trav_blocks > 0 ? trav_blocks : resident_blocks<R, Stepper, 1, ONE>(smem), 256, smem, s>>>(W);
-#if SKG_PDL
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(resident_blocks<R, Stepper, 2, ONE>(smem));
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, trav_kernel<R, Stepper, 2, ONE>, W);
-    if (e != cudaSuccess) return e;
-#else
-    trav_kernel<R, Stepper, 2, ONE><<<resident_blocks<R, Stepper, 2, ONE>(smem), 256, smem, s>>>(W);
-#endif
+    auto blocks = [&](int resident) { return trav_blocks > 0 ? trav_blocks : resident; };
+    if (W.path_tau) {
+        trav_kernel<R, Stepper, TRAV_TAU, ONE><<<blocks(resident_blocks<R, Stepper, TRAV_TAU, ONE>(smem)), 256, smem, s>>>(W);
+    } else {
+        trav_kernel<R, Stepper, TRAV_PATH, ONE><<<blocks(resident_blocks<R, Stepper, TRAV_PATH, ONE>(smem)), 256, smem, s>>>(W);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(resident_blocks<R, Stepper, TRAV_TAU, ONE>(smem));
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = SKG_PDL;
+        cudaError_t e = cudaLaunchKernelEx(&cfg, trav_kernel<R, Stepper, TRAV_TAU, ONE>, W);
+        if (e != cudaSuccess) return e;
+    }
+    path_end_kernel<<<std::min(need * SKG_EVENT_THREADS / 128 + 1, dev_sms() * 16), 128, 0, s>>>(W);
+    trav_kernel<R, Stepper, TRAV_REWALK, ONE><<<resident_blocks<R, Stepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
     return cudaGetLastError();
 }
 
@@ -1571,14 +1568,14 @@ cudaError_t WaveRunner::enqueue(int n) {
         const int w = waves_ + i, b = w & 1;
         WaveParams W;
         W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = w;
-        W.jobs = jobs_[b]; W.jtau = jtau_[b]; W.jL = jL_[b]; W.jcount = ctr_ + 8 * b;
+        W.jobs = jobs_[b]; W.jtau = jtau_[b]; W.jL = jL_[b]; W.jcount = ctr_ + J_N * b;
         W.pjobs = jobs_[b ^ 1]; W.pjtau = jtau_[b ^ 1]; W.pjL = jL_[b ^ 1];
-        W.last_busy = ctr_ + 16;
-        W.freelist = free_; W.intlist = free_ + npool_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+        W.last_busy = ctr_ + 2 * J_N;
+        W.freelist = free_; W.intlist = free_ + npool_; W.rlist = free_; W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
         W.g0 = g0_;
         W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
         W.jkey = jkey_; W.spath = spath_; W.speel = speel_;
-        if ((e = cudaMemsetAsync(ctr_ + 8 * b, 0, 8 * sizeof(unsigned), stream_)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(ctr_ + J_N * b, 0, J_N * sizeof(unsigned), stream_)) != cudaSuccess) return e;
         if (timed_) {
             while (ev_.size() < 3 * (size_t)(w + 1)) {
                 cudaEvent_t x;
@@ -1600,7 +1597,7 @@ cudaError_t WaveRunner::enqueue(int n) {
 }
 
 cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, int precision, int nslots,
-                              size_t npool, int trav_blocks, cudaStream_t s, const DevGrid* one_grid) {
+                              size_t npool, int trav_blocks, bool absorbs, cudaStream_t s, const DevGrid* one_grid) {
     if (npool == 0 || npool > cap_pool_) return cudaErrorInvalidValue;
     P_ = P; grid_type_ = grid_type; tree_walk_ = tree_walk; precision_ = precision; nslots_ = nslots;
     one_ = one_grid != nullptr && nslots == 1;
@@ -1608,6 +1605,7 @@ cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, 
     trav_blocks_ = trav_blocks; stream_ = s; npool_ = (int)npool; waves_ = 0; tail_ran_ = false;
     const char* td = std::getenv("SKG_TAIL_DIV");
     tail_div_ = td ? std::atoi(td) : tail_div;
+    path_tau_ = !absorbs && !(precision == SKG_PREC_FP32 && ckpt_grid(grid_type));
     const char* ck = std::getenv("SKG_CKPT");
     ckpt_on_ = !(ck && std::atoi(ck) == 0) && ckpt_ && cap_ckpt_ >= (size_t)npool;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1624,10 +1622,10 @@ cudaError_t WaveRunner::enqueue_tail() {
     const int b = (waves_ - 1) & 1;               // the last wave's jobs hold the pending peel-offs
     WaveParams W;
     W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = waves_;
-    W.jobs = nullptr; W.jtau = nullptr; W.jL = nullptr; W.jcount = ctr_ + 8 * (b ^ 1);
+    W.jobs = nullptr; W.jtau = nullptr; W.jL = nullptr; W.jcount = ctr_ + J_N * (b ^ 1);
     W.pjobs = jobs_[b]; W.pjtau = jtau_[b]; W.pjL = jL_[b];
-    W.last_busy = ctr_ + 16;
-    W.freelist = nullptr; W.intlist = nullptr; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+    W.last_busy = ctr_ + 2 * J_N;
+    W.freelist = nullptr; W.intlist = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
     W.hist = nullptr; W.bin0 = nullptr; W.jkey = nullptr; W.spath = nullptr; W.speel = nullptr;
     cudaError_t e;
     if (timed_) {
@@ -1657,10 +1655,10 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
             }
             std::this_thread::sleep_for(std::chrono::microseconds(50));
         }
-        const unsigned busy = h_ctr_[8 * ((waves_ - 1) & 1) + 3];
+        const unsigned busy = h_ctr_[J_N * ((waves_ - 1) & 1) + J_BUSY];
         if (busy == 0) {
             pending_ = false;
-            estimate = (int)h_ctr_[16] + 3;        // the last busy wave, the detection wave, one spare
+            estimate = (int)h_ctr_[2 * J_N] + 3;        // the last busy wave, the detection wave, one spare
             break;
         }
         if (tail_div_ > 0 && (size_t)busy * (size_t)tail_div_ <= (size_t)npool_) {

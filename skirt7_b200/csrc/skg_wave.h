@@ -27,11 +27,12 @@ public:
     // grid, with the pool whether the jobs are walked in spatial order.
     cudaError_t reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes);
     // Enqueues the reset of the pool and the first waves of a phase on stream s.  P holds the
-    // staged tables; nslots the slots whose DevGrid the traversal pass keeps in shared memory;
+    // staged tables; absorbs: some simulation tallies absorption in this phase or has several dust
+    // components (its path walks then carry luminosities); nslots the slots whose DevGrid the traversal pass keeps in shared memory;
     // tree_walk the FP32 tree walk (TreeWalk) of tree grids; one_grid (host copy), when given with
     // nslots = 1, the grid the FP32 traversal kernels take as a kernel parameter instead.
     cudaError_t begin(const RunParams& P, int grid_type, int tree_walk, int precision, int nslots,
-                      size_t npool, int trav_blocks, cudaStream_t s, const DevGrid* one_grid = nullptr);
+                      size_t npool, int trav_blocks, bool absorbs, cudaStream_t s, const DevGrid* one_grid = nullptr);
     // Waits for the enqueued waves and enqueues more until no packet is left; then records
     // `end` (if given) on the phase's stream.  timeout_ms < 0 waits without limit.
     cudaError_t finish(int timeout_ms, cudaEvent_t end, bool* timed_out);
@@ -70,8 +71,9 @@ private:
     int4* speel_ = nullptr;
     size_t cap_order_ = 0;
     bool order_on_ = false;           // the running phase walks its jobs in spatial order
-    static constexpr int NCTR = 17;
-    unsigned* ctr_ = nullptr;         // [8b .. 8b+7]: counters of job buffer b; [16]: last busy wave
+    bool path_tau_ = false;
+    static constexpr int NCTR = 2 * J_N + 1;
+    unsigned* ctr_ = nullptr;         // [J_N b + JobCount]: counters of job buffer b; [2 J_N]: last busy wave
     unsigned* h_ctr_ = nullptr;       // pinned copy read by finish()
     cudaEvent_t copied_ = nullptr;
 
