@@ -122,7 +122,14 @@ struct RunParams {
 // pass (one thread per record) advances every packet to its next traversals and writes them as
 // jobs, and a traversal pass walks all jobs of the wave.
 enum PacketState : int { PK_EMPTY = 0, PK_WAIT, PK_INTERACT, PK_TERM, PK_DONE };
-constexpr int JOB_BINS = 1 << 15;     // bins of the walk order, for path jobs and for peel-off jobs each
+#ifndef SKG_BIN_XY
+#define SKG_BIN_XY 6
+#endif
+#ifndef SKG_BIN_Z
+#define SKG_BIN_Z 5
+#endif
+constexpr int BIN_BITS_XY = SKG_BIN_XY, BIN_BITS_Z = SKG_BIN_Z;   // division of the box for the walk order
+constexpr int JOB_BINS = 1 << (3 + 2 * BIN_BITS_XY + BIN_BITS_Z);  // bins, for path jobs and for peel-off jobs each
 constexpr int JOB_MAIN = 31;          // job type of the packet's own path; 0..15 = peel-off group
 
 struct __align__(16) Packet {

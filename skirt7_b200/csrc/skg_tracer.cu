@@ -418,35 +418,29 @@ SKG_D int find_item(const WorkItem* items, int n, uint64_t p) {
 // ---------------------------------------------------------------------------------------------
 // event pass
 
-// Bins of the walk order.  A path job: the octant of its direction, then the Morton cell of its start
-// on a 16^3 division of the grid's box.  A peel-off job: its direction group (mod 8), then the Morton
-// cell, on a 64^2 division, of the point where its ray passes the middle plane of the box across the
-// direction's largest component.
-SKG_D int bin_coord(float u, int n) {
-    // u: -1..1 across the box
-    return min(n - 1, max(0, (int)((0.5f * u + 0.5f) * n)));
+// Bins of the walk order: the octant of a path job's direction or the group (mod 8) of a peel-off
+// job, then the Morton cell of its start on a division of the grid's box.
+SKG_D unsigned bin_coord(float u, int bits) {       // u: -1..1 across the box
+    const int n = 1 << bits;
+    return (unsigned)min(n - 1, max(0, (int)((0.5f * u + 0.5f) * n)));
 }
-SKG_D unsigned spread3(unsigned v) { return (v & 1) | (v & 2) << 2 | (v & 4) << 4 | (v & 8) << 6; }
-SKG_D unsigned spread2(unsigned v) {
-    v = (v | v << 4) & 0x0F0Fu; v = (v | v << 2) & 0x3333u; return (v | v << 1) & 0x5555u;
+SKG_D unsigned spread3(unsigned v) {                // up to 10 bits, two zeros between
+    v = (v | v << 16) & 0x030000FFu; v = (v | v << 8) & 0x0300F00Fu;
+    v = (v | v << 4) & 0x030C30C3u; return (v | v << 2) & 0x09249249u;
+}
+SKG_D unsigned box_bin(float u, float v, float w) {
+    const unsigned i = bin_coord(u, BIN_BITS_XY), j = bin_coord(v, BIN_BITS_XY), k = bin_coord(w, BIN_BITS_Z);
+    constexpr int D = BIN_BITS_XY - BIN_BITS_Z;     // the finer bits of x and y last
+    return (spread3(i >> D) | spread3(j >> D) << 1 | spread3(k) << 2) << (2 * D) | (i & ((1 << D) - 1)) << D | (j & ((1 << D) - 1));
 }
 SKG_D unsigned path_bin(const DevGrid& g, float x, float y, float z, float kx, float ky, float kz) {
     const unsigned oct = (kx < 0.f ? 1u : 0u) | (ky < 0.f ? 2u : 0u) | (kz < 0.f ? 4u : 0u);
-    const int i = bin_coord((x - g.bmid[0]) * g.bscale[0], 16), j = bin_coord((y - g.bmid[1]) * g.bscale[1], 16),
-              k = bin_coord((z - g.bmid[2]) * g.bscale[2], 16);
-    return oct << 12 | spread3(i) | spread3(j) << 1 | spread3(k) << 2;
+    return oct << (2 * BIN_BITS_XY + BIN_BITS_Z) |
+           box_bin((x - g.bmid[0]) * g.bscale[0], (y - g.bmid[1]) * g.bscale[1], (z - g.bmid[2]) * g.bscale[2]);
 }
-SKG_D unsigned peel_bin(const DevGrid& g, int grp, float x, float y, float z, float kx, float ky, float kz) {
-    // box coordinates (-1..1) of the position and the direction
-    float u = (x - g.bmid[0]) * g.bscale[0], v = (y - g.bmid[1]) * g.bscale[1], w = (z - g.bmid[2]) * g.bscale[2];
-    float du = kx * g.bscale[0], dv = ky * g.bscale[1], dw = kz * g.bscale[2];
-    // the axis of the largest component last
-    const float au = fabsf(du), av = fabsf(dv), aw = fabsf(dw);
-    if (au >= av && au >= aw) { float t = u; u = w; w = t; t = du; du = dw; dw = t; }
-    else if (av >= aw) { float t = v; v = w; w = t; t = dv; dv = dw; dw = t; }
-    const float f = w / dw;
-    const int i = bin_coord(u - f * du, 64), j = bin_coord(v - f * dv, 64);
-    return (unsigned)(grp & 7) << 12 | spread2(i) | spread2(j) << 1;
+SKG_D unsigned peel_bin(const DevGrid& g, int grp, float x, float y, float z) {
+    return (unsigned)(grp & 7) << (2 * BIN_BITS_XY + BIN_BITS_Z) |
+           box_bin((x - g.bmid[0]) * g.bscale[0], (y - g.bmid[1]) * g.bscale[1], (z - g.bmid[2]) * g.bscale[2]);
 }
 
 // The direction groups that get a peel-off traversal from (x, y, z), in group order
@@ -468,8 +462,7 @@ SKG_D int peel_jobs(const DevScene& S, int ell, bool scat, int cell, double kx, 
             W->jobs[j0 + n] = make_int2(p, g);
             W->jL[j0 + n] = L * w;
             if (W->hist) {
-                const unsigned b = peel_bin(*grid, g, (float)x, (float)y, (float)z, (float)S.gkx[g], (float)S.gky[g],
-                                            (float)S.gkz[g]);
+                const unsigned b = peel_bin(*grid, g, (float)x, (float)y, (float)z);
                 W->jkey[j0 + n] = make_uint2(b, atomicAdd(W->hist + JOB_BINS + b, 1u));
             }
         }
@@ -778,30 +771,54 @@ __global__ void __launch_bounds__(SKG_EVENT_THREADS) launch_kernel(const WavePar
 // walk order: a counting sort of the wave's jobs by bin (each job has its rank within its bin from
 // the launch pass)
 
-// First place of each bin (block 0 path jobs, block 1 peel-off jobs); clears the counts.
-__global__ void __launch_bounds__(1024) bins_kernel(unsigned* hist, unsigned* bin0) {
+// First place of each bin: the counts of the bins before it among path jobs or among peel-off jobs.
+// Blocks of 1024 threads, 8 bins a thread; bin_sums_kernel sums each block's bins first.
+constexpr int BIN_BLOCK = 8192;
+SKG_D unsigned warp_sum(unsigned v) {
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    return v;
+}
+__global__ void __launch_bounds__(1024) bin_sums_kernel(const unsigned* __restrict__ hist, unsigned* sums) {
     __shared__ unsigned ws[32];
-    constexpr int PER = JOB_BINS / 1024;
-    uint4* h = reinterpret_cast<uint4*>(hist + blockIdx.x * JOB_BINS + threadIdx.x * PER);
-    uint4* o = reinterpret_cast<uint4*>(bin0 + blockIdx.x * JOB_BINS + threadIdx.x * PER);
-    uint4 c[PER / 4];
+    const uint4* h = reinterpret_cast<const uint4*>(hist + (size_t)blockIdx.x * BIN_BLOCK);
+    const uint4 a = h[threadIdx.x], b = h[threadIdx.x + 1024];
+    const unsigned v = warp_sum(a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const unsigned t = warp_sum(ws[threadIdx.x]);
+        if (threadIdx.x == 0) sums[blockIdx.x] = t;
+    }
+}
+// Clears the counts as well.
+__global__ void __launch_bounds__(1024) bins_kernel(unsigned* hist, unsigned* bin0, const unsigned* __restrict__ sums) {
+    __shared__ unsigned ws[32], before;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint4* h = reinterpret_cast<uint4*>(hist + (size_t)blockIdx.x * BIN_BLOCK) + 2 * threadIdx.x;
+    uint4* o = reinterpret_cast<uint4*>(bin0 + (size_t)blockIdx.x * BIN_BLOCK) + 2 * threadIdx.x;
+    uint4 c[2];
     unsigned sum = 0;
 #pragma unroll
-    for (int i = 0; i < PER / 4; i++) { c[i] = h[i]; sum += c[i].x + c[i].y + c[i].z + c[i].w; }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = 0; i < 2; i++) { c[i] = h[i]; sum += c[i].x + c[i].y + c[i].z + c[i].w; }
     unsigned inc = sum;
     for (int d = 1; d < 32; d <<= 1) { const unsigned t = __shfl_up_sync(0xffffffffu, inc, d); if (lane >= d) inc += t; }
     if (lane == 31) ws[warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        unsigned v = ws[lane], w = v;
-        for (int d = 1; d < 32; d <<= 1) { const unsigned t = __shfl_up_sync(0xffffffffu, w, d); if (lane >= d) w += t; }
-        ws[lane] = w - v;
+        constexpr int HALF = JOB_BINS / BIN_BLOCK;
+        unsigned v = 0;
+        for (int b = blockIdx.x / HALF * HALF + lane; b < (int)blockIdx.x; b += 32) v += sums[b];
+        v = warp_sum(v);
+        const unsigned t = ws[lane];
+        unsigned w = t;
+        for (int d = 1; d < 32; d <<= 1) { const unsigned q = __shfl_up_sync(0xffffffffu, w, d); if (lane >= d) w += q; }
+        ws[lane] = w - t;
+        if (lane == 0) before = v;
     }
     __syncthreads();
-    unsigned at = ws[warp] + inc - sum;
+    unsigned at = before + ws[warp] + inc - sum;
 #pragma unroll
-    for (int i = 0; i < PER / 4; i++) {
+    for (int i = 0; i < 2; i++) {
         uint4 b;
         b.x = at; at += c[i].x; b.y = at; at += c[i].y; b.z = at; at += c[i].z; b.w = at; at += c[i].w;
         o[i] = b;
@@ -1414,7 +1431,8 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
         }
         launch_kernel<R><<<sms * per, SKG_EVENT_THREADS, 0, s>>>(W);
         if (W.hist) {
-            bins_kernel<<<2, 1024, 0, s>>>(W.hist, W.bin0);
+            bin_sums_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0 + 2 * JOB_BINS);
+            bins_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0, W.bin0 + 2 * JOB_BINS);
             order_kernel<<<std::min(sms * 8, (W.npool + 255) / 256), 256, 0, s>>>(W);
         }
     }
@@ -1532,7 +1550,7 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t 
         cap_ckpt_ = pool;
     }
     if (order_on_ && !bins_) {
-        if ((e = cudaMalloc(&bins_, 4 * JOB_BINS * sizeof(unsigned))) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&bins_, (4 * (size_t)JOB_BINS + 1024) * sizeof(unsigned))) != cudaSuccess) return e;
         if ((e = cudaMemset(bins_, 0, 4 * JOB_BINS * sizeof(unsigned))) != cudaSuccess) return e;
     }
     const size_t jobs = pool * (size_t)(ngroups + 1);
