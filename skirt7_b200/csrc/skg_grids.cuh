@@ -1037,17 +1037,32 @@ struct TreeOctantStepper<float> {
         uy = (fabsf(ky) > 1e-15f) ? 1.f / ky : 0.f; by = uy != 0.f ? 0.f : FLT_MAX;
         uz = (fabsf(kz) > 1e-15f) ? 1.f / kz : 0.f; bz = uz != 0.f ? 0.f : FLT_MAX;
         obase = ((kx < 0.f ? 1 : 0) + (ky < 0.f ? 2 : 0) + (kz < 0.f ? 4 : 0)) * g.ncells;
-        int c;
-        if (hint >= 0 && holds(g, hint, rx, ry, rz)) {
-            c = hint; cell0 = hint;
-        } else {
-            c = move_inside<float>(g, g.epsf, rx, ry, rz, kx, ky, kz, pd) ? TreeStepper<float>::locate(g, rx, ry, rz) : -1;
-            if (c < 0) { pd.n = 0; done = true; return; }
-            if (pd.n == 0) cell0 = c;
+        x = rx; y = ry; z = rz;
+        if (hint >= 0) {
+            // the lattice record of the cell tells whether it holds the start and has all that the
+            // octant record has: one load
+            TreeLatticeStepper<float> l;
+            l.load(g, hint);
+            if (l.inside(g, rx, ry, rz)) {
+                using L = TreeLatticeStepper<float>;
+                wx = L::wall(L::code_x(l.a), kx >= 0.f, g.lorg[0], g.lunit[0]);
+                wy = L::wall(L::code_y(l.a), ky >= 0.f, g.lorg[1], g.lunit[1]);
+                wz = L::wall(L::code_z(l.a), kz >= 0.f, g.lorg[2], g.lunit[2]);
+                wrho = __uint_as_float(l.a.x);
+                l.kx = kx; l.ky = ky; l.kz = kz;
+                gx_ = l.exit_rope(0); gy_ = l.exit_rope(1); gz_ = l.exit_rope(2);
+                if (gx_ >= 0) gx_ += obase;
+                if (gy_ >= 0) gy_ += obase;
+                if (gz_ >= 0) gz_ += obase;
+                idx = obase + hint; cell0 = hint;
+                return;
+            }
         }
+        const int c = move_inside<float>(g, g.epsf, x, y, z, kx, ky, kz, pd) ? TreeStepper<float>::locate(g, x, y, z) : -1;
+        if (c < 0) { pd.n = 0; done = true; return; }
+        if (pd.n == 0) cell0 = c;
         idx = obase + c;
         load(g);
-        x = rx; y = ry; z = rz;
     }
 
     SKG_D bool next(const DevGrid& g, int& m, float& ds) {
@@ -1283,6 +1298,25 @@ SKG_D bool VoronoiStepper<float>::walk(const DevGrid& g, int& m, float& ds) {
         return true;
     }
     return false;
+}
+
+// The cell of a start position strictly inside the box, as the FP32 walks' own search finds it
+// (-2: left to the walk).
+SKG_D int start_cell(const DevGrid& g, float x, float y, float z) {
+    if (!(x > (float)g.xmin && x < (float)g.xmax && y > (float)g.ymin && y < (float)g.ymax && z > (float)g.zmin &&
+          z < (float)g.zmax)) return -2;
+    if (g.type == SKG_GRID_CARTESIAN) {
+        const int i = locate_clip_dev<float, gx<float>>(g, g.nx + 1, x), j = locate_clip_dev<float, gy<float>>(g, g.ny + 1, y),
+                  k = locate_clip_dev<float, gz<float>>(g, g.nz + 1, z);
+        return k + g.nz * j + g.nz * g.ny * i;
+    }
+    if (g.type == SKG_GRID_VORONOI) {
+        const int m = voronoi_cell_index<float>(g, x, y, z);
+        return m >= 0 ? m : -2;
+    }
+    if (!g.lattice || g.search == SKG_SEARCH_BOOKKEEPING) return -2;
+    const int m = TreeStepper<float>::locate(g, x, y, z);
+    return m >= 0 ? m : -2;
 }
 
 }  // namespace skg

@@ -132,26 +132,35 @@ constexpr int BIN_BITS_XY = SKG_BIN_XY, BIN_BITS_Z = SKG_BIN_Z;   // division of
 constexpr int JOB_BINS = 1 << (3 + 2 * BIN_BITS_XY + BIN_BITS_Z);  // bins, for path jobs and for peel-off jobs each
 constexpr int JOB_MAIN = 31;          // job type of the packet's own path; 0..15 = peel-off group
 
-struct __align__(16) Packet {
+struct __align__(64) Packet {
+    // what every walk reads: one 64-byte line
     double x, y, z;                   // position (rounded to the traversal precision)
     double kx, ky, kz;                // direction
-    double L, Lth;                    // luminosity and its termination threshold
-    double s_int;                     // distance to the interaction point (before its re-walk: the
-                                      // interaction optical depth)
-    uint64_t id;                      // packet number within its work item (RNG counter words)
     int item;                         // work item
     int ell;
-    int nscatt;
     int pos_cell;                     // cell of the position: -2 unknown, -1 outside the grid
+    int state;                        // PacketState
+    double L, Lth;                    // luminosity and its termination threshold
+    double s_int;                     // distance to the interaction point
+    uint64_t id;                      // packet number within its work item (RNG counter words)
+    int nscatt;
     int int_cell;                     // cell of the interaction point (-1 unknown)
     unsigned rngc;                    // next Philox block of the packet's stream
-    int state;                        // PacketState
     int flags;                        // bit 0 stellar origin, bit 1 the pending peel-offs follow a scattering
     int peel_j0, peel_n;              // this packet's peel-off jobs of the last wave
     int nck;                          // checkpoints of the path walk
     int pad;
 };
 static_assert(sizeof(Packet) == 128, "packet record is two 64-byte lines");
+
+// What a walk needs of its job (staged in shared memory by the warp that took it).
+template<typename R> struct __align__(16) WalkJob {
+    R x, y, z, kx, ky, kz;            // start and direction
+    float kext1;                      // kappa_ext at its wavelength (one dust component), else -1
+    int hint;                         // cell of the start, if known
+    int out;                          // where its optical depth goes
+    int p, slot, ell;                 // packet, simulation, wavelength
+};
 
 // Counters of a wave's jobs and lists.
 enum JobCount : int {
@@ -182,16 +191,16 @@ struct WaveParams {
     unsigned* last_busy;              // highest wave index that had jobs
     int* freelist;                    // records the event pass freed (J_FREE)
     int* intlist;                     // records it found at their interaction point (J_INT)
-    int* rlist;                       // packets that interact on their path (J_REWALK; the free list's
-                                      // memory, which the launch pass has consumed)
+    int2* rlist;                      // the paths that interact: (packet, place in walk order) (J_REWALK;
+                                      // the memory of the lists above, which the launch pass has consumed)
     int path_tau;                     // the path jobs need the optical depth alone (walked with the peel-offs)
     float4* ckpt;                     // per packet record: checkpoints of its path walk
     // walk order of the wave's jobs (order_kernel); hist == nullptr: as appended
     unsigned* hist;                   // [2][JOB_BINS] jobs per bin: path jobs, peel-off jobs (zero between waves)
     unsigned* bin0;                   // [2][JOB_BINS] first place of each bin
     uint2* jkey;                      // per job (its bin, its rank within it)
-    int* spath;                       // packets of the path jobs in walk order
-    int4* speel;                      // peel-off jobs in walk order: (packet, group, job index, 0)
+    int* spath;                       // packets of the path jobs
+    int4* speel;                      // peel-off jobs: (packet, group, job index, 0)
     // the grid of a single-simulation launch: the traversal kernels' instantiation for one slot
     // reads it from their parameters (constant-bank operands, no load instructions per cell step)
     DevGrid g0;

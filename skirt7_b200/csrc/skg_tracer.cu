@@ -74,10 +74,10 @@ namespace skg {
 #ifndef SKG_EVENT_THREADS
 #define SKG_EVENT_THREADS 64
 #endif
-// a lane whose job ended takes the next one when this many lanes of its warp (or all of its live
-// lanes) wait for one: the job start (job, packet record, start leaf: dependent loads) is then paid
-// once for several lanes instead of stalling the warp for each (8 measured fastest of 1-32 on the
-// octree disk: traversal pass 275 ms against 336 ms at 1 per 10^7 packets)
+// a lane whose job ended takes the next one when this many lanes of its warp (or all of them) wait for
+// one.  With the job records staged by the warp a start costs little: 4, 8 and 12 lanes take the octree
+// disk's traversal pass 166.7, 162.3 and 161.5 ms (2*10^7 packets), the fit-variant batch 43.8, 43.3
+// and 43.8 ms
 #ifndef SKG_REFILL_LANES
 #define SKG_REFILL_LANES 8
 #endif
@@ -102,16 +102,11 @@ namespace skg {
 #ifndef SKG_EVENT_STRIDE_POOL
 #define SKG_EVENT_STRIDE_POOL (1 << 21)
 #endif
-// cell steps a lane takes per pass of the traversal loop (the warp's refill and end-of-path votes
-// run once per pass): peel-off-job kernel, path-job kernel.  Traversal pass of a 10^7-packet
-// phase (octree disk / Cartesian disk): 1 and 1: 161 / 69.1 ms; 2 and 1: 156 / 68.6; 2 and 2: 153 /
-// 68.1; 2 and 3: 152.4 / 67.0; 2 and 4: 151.3 / 66.4; 3 or 4 steps in the peel-off kernel spilled
-// then: 165 / 68.3.  With the per-axis rope the peel-off kernel no longer spills at 3 or 4, and at
-// 2·10^6 packets per wavelength 3 and 4 take the octree disk 1360 ms against 1367 at 2 and 4 (4 and
-// 4: 1365, 2 and 6: 1404); 3 and 4 against 2 and 4 elsewhere: Cartesian disk 61.2 / 61.7, k-d tree
-// disk 1730 / 1734, Voronoi disk 252.8 / 253.4 ms, a batch of 24 fit variants 566 / 571 ms
+// cell steps a lane takes per pass of the traversal loop (the warp's refill vote runs once per
+// pass): optical-depth and re-walk kernels, path kernel.  Octree disk, 2*10^7 packets, traversal pass
+// at 3 and 5: 162.3 and 156.8 ms; Cartesian disk 7.30 and 7.19, k-d tree disk 23.4 and 22.7 ms
 #ifndef SKG_INNER_STEPS
-#define SKG_INNER_STEPS 3
+#define SKG_INNER_STEPS 5
 #endif
 #ifndef SKG_INNER_PATH
 #define SKG_INNER_PATH 4
@@ -756,6 +751,9 @@ __global__ void __launch_bounds__(SKG_EVENT_THREADS) launch_kernel(const WavePar
         int state = PK_DONE, npeel = 0, nmain = 0;
         if (mine) { K = W.pk[p]; state = K.state; }
         take_packets<R>(P, H, phase, peel_on, lane, mine, K, state, npeel, nmain, s_cnt);
+        // the start cell once per packet, all lanes together (otherwise each of its walks looks for it)
+        if (sizeof(R) == 4 && mine && nmain + npeel > 0)
+            K.pos_cell = start_cell(P.grids[P.items[K.item].slot], (float)K.x, (float)K.y, (float)K.z);
         append_jobs(W, p, K, npeel, nmain, false, 0, 0, 0, lane);
         if (mine) {
             K.flags &= ~2;
@@ -828,17 +826,13 @@ __global__ void __launch_bounds__(1024) bins_kernel(unsigned* hist, unsigned* bi
 
 // Writes the jobs in walk order.
 __global__ void __launch_bounds__(256) order_kernel(const WaveParams W) {
-    const unsigned nmain = W.jcount[J_PATH], npeel = W.jcount[J_PEEL];
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nmain + npeel; i += gridDim.x * blockDim.x) {
-        if (i < nmain) {
-            const uint2 k = W.jkey[i];
-            W.spath[W.bin0[k.x] + k.y] = W.jobs[i].x;
-        } else {
-            const unsigned j = W.npool + (i - nmain);
-            const uint2 k = W.jkey[j];
-            const int2 jb = W.jobs[j];
-            W.speel[W.bin0[JOB_BINS + k.x] + k.y] = make_int4(jb.x, jb.y, (int)j, 0);
-        }
+    const unsigned npath = W.jcount[J_PATH], n = npath + W.jcount[J_PEEL];
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned j = i < npath ? i : W.npool + (i - npath);
+        const uint2 k = W.jkey[j];
+        const int2 jb = W.jobs[j];
+        if (i < npath) W.spath[W.bin0[k.x] + k.y] = jb.x;
+        else W.speel[W.bin0[JOB_BINS + k.x] + k.y] = make_int4(jb.x, jb.y, (int)j, 0);
     }
 }
 
@@ -988,13 +982,27 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
     // only from "unknown" to the cell, and either value is a valid hint for the peel-off walk.
     if (MODE == TRAV_PATH) asm volatile("griddepcontrol.launch_dependents;");
 #endif
-    const unsigned npath = (MODE == TRAV_PATH || (MODE == TRAV_TAU && W.path_tau)) ? W.jcount[J_PATH] : 0;
-    const unsigned njobs = MODE == TRAV_PATH ? npath : MODE == TRAV_TAU ? npath + W.jcount[J_PEEL] : W.jcount[J_REWALK];
+    // the walk's jobs in the wave's list
+    const unsigned npath = W.jcount[J_PATH];
+    const unsigned job0 = (MODE == TRAV_TAU && !W.path_tau) ? npath : 0;   // (re-walks: listed by the path ends)
+    const unsigned njobs = MODE == TRAV_PATH ? npath : MODE == TRAV_TAU ? npath - job0 + W.jcount[J_PEEL] : W.jcount[J_REWALK];
     unsigned* const taken = W.jcount + (MODE == TRAV_PATH ? J_TAKEN_PATH : MODE == TRAV_TAU ? J_TAKEN_TAU : J_TAKEN_REWALK);
     const int phase = H.phase;
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int refill_lanes = P.refill > 0 ? P.refill : SKG_REFILL_LANES;
     constexpr bool CKPT = HasCkpt<R, Stepper>::value;
+    // A warp takes jobs in chunks of up to 32 and stages their records in shared memory, all lanes
+    // loading at once: the chain of dependent loads of a job start (job, packet, tables) is paid once
+    // per chunk instead of once per refill, and the lanes walk neighbours in walk order.  A wave with
+    // fewer jobs than lanes spreads them over the warps.  Fit-variant batch 39.5 against 46.2 ms,
+    // octree disk (2*10^7 packets) traversal pass 162.3 against 171.2 ms.
+    __shared__ WalkJob<R> s_job[256];
+    WalkJob<R>* const mine = s_job + (threadIdx.x & ~31);
+    const unsigned nwarps = gridDim.x * 8;
+    const int chunk = (int)min(32u, max(1u, (njobs + nwarps - 1) / nwarps));
+    int have = 0, used = 0;           // jobs of the chunk, and those handed to lanes
+    bool more = true;                 // the list has jobs left
 
     int j = -1;                       // where the lane's job leaves its result (-1: no job)
     int p = 0, slot = 0, ell = 0;
@@ -1003,66 +1011,82 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
     // product: one expm1 per absorbing cell step), v2 = L_sca (several dust components);
     // TRAV_REWALK: v1 = path length walked, v2 = the interaction optical depth
     double v1 = 0, v2 = 0;
-    float kext1 = -1.f;               // kappa_ext at the job's wavelength (one dust component), else -1
-    unsigned c_steps = 0;
+    float kext1 = -1.f;
+    unsigned c_steps = 0, c_trav = 0, c_fb = 0, c_abs = 0;
+    unsigned long long c_nbr = 0;
     Stepper<R> st;
     int nck = 0;                      // checkpoints of the path walk
 
     while (true) {
-        // lanes without a job take the next ones: one atomic per warp
-        const unsigned live = __activemask();
-        const bool need = j < 0;
-        const unsigned want = __ballot_sync(live, need);
-        if (want && (__popc(want) >= refill_lanes || want == live)) {
-            const int leader = __ffs(want) - 1;
-            unsigned base = 0;
-            if (lane == leader) base = atomicAdd(taken, (unsigned)__popc(want));
-            base = __shfl_sync(live, base, leader);
-            if (need) {
-                const unsigned jj = base + __popc(want & ((1u << lane) - 1));
-                if (jj >= njobs) break;
-                int grp = JOB_MAIN;
-                if (MODE == TRAV_REWALK) {
-                    j = (int)jj;
-                    p = W.rlist[jj];
-                } else if (MODE == TRAV_PATH || jj < npath) {
-                    j = (int)jj;
-                    p = W.hist ? W.spath[jj] : W.jobs[jj].x;
-                } else if (W.hist) {
-                    const int4 o = W.speel[jj - npath];
-                    p = o.x; grp = o.y; j = o.z;
-                } else {
-                    j = W.npool + (int)(jj - npath);
-                    const int2 jb = W.jobs[j];
-                    p = jb.x; grp = jb.y;
-                }
-                const Packet& K = W.pk[p];
-                ell = K.ell;
-                slot = P.items[K.item].slot;
-                const DevScene& S = *s_scene[slot];
-                const DevGrid& g = grid_of(slot);
-                const int hint = K.pos_cell;
-                kext1 = (S.ncomp == 1) ? (float)S.kext[ell] : -1.f;
-                tau = 0;
-                // entry segments outside the grid (m = -1) carry no optical depth: only the
-                // re-walk, which measures length, takes them
-                if (MODE == TRAV_REWALK) {
-                    v1 = 0; v2 = K.s_int;
-                    bool resumed = false;
-                    if constexpr (CKPT) resumed = W.ckpt && resume_ckpt(W, g, p, K.nck, v2, st, tau, v1);
-                    if (!resumed) {
-                        st.init(g, (R)K.x, (R)K.y, (R)K.z, (R)K.kx, (R)K.ky, (R)K.kz, hint);
-                        R d0;
-                        while (st.pd.pop(d0)) v1 += (double)d0;
+        const unsigned want = __ballot_sync(FULL, j < 0);
+        if (want && (__popc(want) >= refill_lanes || want == FULL)) {
+            if (used == have && more) {
+                unsigned base = 0;
+                if (lane == 0) base = atomicAdd(taken, (unsigned)chunk);
+                base = __shfl_sync(FULL, base, 0);
+                have = base < njobs ? (int)min((unsigned)chunk, njobs - base) : 0;
+                used = 0;
+                more = have > 0;
+                if (lane < have) {
+                    WalkJob<R> w;
+                    const unsigned i = job0 + base + lane;
+                    int grp = JOB_MAIN;
+                    if (MODE == TRAV_REWALK) {
+                        const int2 r = W.rlist[i];
+                        w.p = r.x; w.out = r.y;
+                    } else if (MODE == TRAV_PATH || i < npath) {
+                        w.p = W.hist ? W.spath[i] : W.jobs[i].x;
+                        w.out = (int)i;
+                    } else if (W.hist) {
+                        const int4 o = W.speel[i - npath];
+                        w.p = o.x; grp = o.y; w.out = o.z;
+                    } else {
+                        w.out = W.npool + (int)(i - npath);
+                        const int2 jb = W.jobs[w.out];
+                        w.p = jb.x; grp = jb.y;
                     }
-                } else {
-                    R kx, ky, kz;
-                    if (MODE == TRAV_PATH || grp == JOB_MAIN) { kx = (R)K.kx; ky = (R)K.ky; kz = (R)K.kz; }
-                    else { kx = (R)S.gkx[grp]; ky = (R)S.gky[grp]; kz = (R)S.gkz[grp]; }
-                    st.init(g, (R)K.x, (R)K.y, (R)K.z, kx, ky, kz, hint);
-                    if ((MODE == TRAV_PATH || grp == JOB_MAIN) && hint == -2) W.pk[p].pos_cell = st.cell0;
-                    if (MODE == TRAV_PATH) { v1 = K.L; v2 = 0; nck = 0; }
+                    const Packet& K = W.pk[w.p];
+                    w.ell = K.ell; w.hint = K.pos_cell;
+                    w.slot = ONE ? 0 : P.items[K.item].slot;
+                    const DevScene& S = *s_scene[w.slot];
+                    w.kext1 = (S.ncomp == 1) ? (float)S.kext[w.ell] : -1.f;
+                    w.x = (R)K.x; w.y = (R)K.y; w.z = (R)K.z;
+                    if (MODE != TRAV_TAU || grp == JOB_MAIN) { w.kx = (R)K.kx; w.ky = (R)K.ky; w.kz = (R)K.kz; }
+                    else { w.kx = (R)S.gkx[grp]; w.ky = (R)S.gky[grp]; w.kz = (R)S.gkz[grp]; }
+                    mine[lane] = w;
                 }
+                __syncwarp();
+            }
+            if (used == have) {
+                if (want == FULL) break;
+            } else {
+                const int r = used + __popc(want & ((1u << lane) - 1));
+                if (j < 0 && r < have) {
+                    const WalkJob<R> w = mine[r];
+                    j = w.out; p = w.p; slot = w.slot; ell = w.ell; kext1 = w.kext1;
+                    tau = 0;
+                    const DevGrid& g = grid_of(slot);
+                    // entry segments outside the grid (m = -1) carry no optical depth: only the
+                    // re-walk, which measures length, takes them
+                    if (MODE == TRAV_REWALK) {
+                        v1 = 0; v2 = W.jtau[j];
+                        bool resumed = false;
+                        if constexpr (CKPT) resumed = W.ckpt && resume_ckpt(W, g, p, W.pk[p].nck, v2, st, tau, v1);
+                        if (!resumed) {
+                            st.init(g, w.x, w.y, w.z, w.kx, w.ky, w.kz, w.hint);
+                            R d0;
+                            while (st.pd.pop(d0)) v1 += (double)d0;
+                        }
+                    } else {
+                        st.init(g, w.x, w.y, w.z, w.kx, w.ky, w.kz, w.hint);
+                        if (MODE == TRAV_PATH || (job0 == 0 && j < (int)npath)) {
+                            if (w.hint == -2) W.pk[p].pos_cell = st.cell0;
+                        }
+                        if (MODE == TRAV_PATH) { v1 = W.pk[p].L; v2 = 0; nck = 0; }
+                    }
+                }
+                used = min(have, used + __popc(want));
+                __syncwarp();
             }
         }
 
@@ -1083,7 +1107,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                 if (MODE == TRAV_TAU) {
                     tau += dtau;
                 } else if (MODE == TRAV_PATH) {
-                    if (absorb_step<R>(S, phase, m, ell, dtau, v1, v2)) atomicAdd(&s_cnt[C_ABS], 1ull);
+                    c_abs += absorb_step<R>(S, phase, m, ell, dtau, v1, v2);
                     tau += dtau;
                     if constexpr (CKPT) {
                         if (W.ckpt && nck < SKG_CKPT_N && st.steps >= (nck + 1) * SKG_CKPT_STRIDE && !st.done) {
@@ -1098,9 +1122,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                         K.s_int = v1 + ((v2 - tau) / (tn - tau)) * (sn - v1);
                         K.int_cell = m;
                         K.state = PK_INTERACT;
-                        atomicAdd(&s_cnt[C_TRAV], 1ull);
-                        atomicAdd(&s_cnt[C_NBR], (unsigned long long)st.nscanned());
-                        atomicAdd(&s_cnt[C_FB], (unsigned long long)st.fallbacks);
+                        c_trav++; c_nbr += st.nscanned(); c_fb += st.fallbacks;
                         j = -1;
                         break;
                     }
@@ -1108,9 +1130,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                 }
             } else {
                 // the traversal reached the edge of the grid
-                atomicAdd(&s_cnt[C_TRAV], 1ull);
-                atomicAdd(&s_cnt[C_NBR], (unsigned long long)st.nscanned());
-                atomicAdd(&s_cnt[C_FB], (unsigned long long)st.fallbacks);
+                c_trav++; c_nbr += st.nscanned(); c_fb += st.fallbacks;
                 if (st.steps > g.max_steps) { atomicOr(P.err, ERR_STEP_BUDGET); atomicAdd(&s_cnt[C_ERR], 1ull); }
                 if (MODE == TRAV_REWALK) {
                     // DustGridPath::pathlength: an optical depth beyond the last segment gives the full length
@@ -1126,7 +1146,12 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
         }
     }
 
+    // the counters, once per lane
     atomicAdd(&s_cnt[C_STEPS], (unsigned long long)c_steps);
+    atomicAdd(&s_cnt[C_TRAV], (unsigned long long)c_trav);
+    atomicAdd(&s_cnt[C_NBR], c_nbr);
+    atomicAdd(&s_cnt[C_FB], (unsigned long long)c_fb);
+    if (MODE == TRAV_PATH) atomicAdd(&s_cnt[C_ABS], (unsigned long long)c_abs);
     __syncthreads();
     if (threadIdx.x < C_N && s_cnt[threadIdx.x]) atomicAdd(P.counters + threadIdx.x, s_cnt[threadIdx.x]);
 #if SKG_PDL
@@ -1151,19 +1176,19 @@ __global__ void __launch_bounds__(128) path_end_kernel(const WaveParams W) {
         int p = 0;
         if (i < n) {
             p = W.hist ? W.spath[i] : W.jobs[i].x;
-            Packet& K = W.pk[p];
+            const Packet& K = W.pk[p];
             const DevScene& S = *P.scenes[P.items[K.item].slot];
             double L = K.L, tau_int = 0;
             const int rc = after_path(W, S, p, phase, K.ell, W.jtau[i], W.path_tau ? 0.0 : W.jL[i], L, tau_int);
             if (rc < 0) atomicAdd(P.counters + C_ERR, 1ull);
-            if (rc == 1) { K.s_int = tau_int; again = true; }
+            if (rc == 1) { W.jtau[i] = tau_int; again = true; }
         }
         const unsigned am = __ballot_sync(0xffffffffu, again);
         if (am) {
             unsigned base = 0;
             if (lane == 0) base = atomicAdd(W.jcount + J_REWALK, (unsigned)__popc(am));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (again) W.rlist[base + __popc(am & ((1u << lane) - 1))] = p;
+            if (again) W.rlist[base + __popc(am & ((1u << lane) - 1))] = make_int2(p, (int)i);
         }
     }
 }
@@ -1589,7 +1614,7 @@ cudaError_t WaveRunner::enqueue(int n) {
         W.jobs = jobs_[b]; W.jtau = jtau_[b]; W.jL = jL_[b]; W.jcount = ctr_ + J_N * b;
         W.pjobs = jobs_[b ^ 1]; W.pjtau = jtau_[b ^ 1]; W.pjL = jL_[b ^ 1];
         W.last_busy = ctr_ + 2 * J_N;
-        W.freelist = free_; W.intlist = free_ + npool_; W.rlist = free_; W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+        W.freelist = free_; W.intlist = free_ + npool_; W.rlist = reinterpret_cast<int2*>(free_); W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
         W.g0 = g0_;
         W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
         W.jkey = jkey_; W.spath = spath_; W.speel = speel_;
