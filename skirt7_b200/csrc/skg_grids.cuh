@@ -417,62 +417,76 @@ struct CartStepper<float> : CartStepperRef<float> {
 // FP32 walk of a Cartesian grid whose planes are evenly spaced on every axis: the DDA of
 // CartStepper<float> with the ray parameter of plane q on axis a computed as t = c0_a + q dt_a
 // (c0 = (first plane - origin) / k, dt = spacing / k, fixed for a walk; one FMA) instead of loading
-// the plane and selecting its table, the origin and the reciprocal by axis.  The sign of dt is the
-// direction's, so the step needs no direction component either.
+// the plane.  The walk is bound by instructions, so a step carries the next plane of each axis as a
+// float and the cell number itself, steps one axis under predicates instead of selecting every
+// per-axis value by axis, and compares with the ray parameter of the exit instead of the plane
+// index: same segments, a batch of 24 fit variants 35.3 against 39.5 ms.
 template<typename R> struct CartUniStepper : CartStepperRef<R> {};
 template<>
-struct CartUniStepper<float> : CartStepperRef<float> {
+struct CartUniStepper<float> {
     float tx, ty, tz;           // ray parameter of the next x, y and z wall
     float tc;                   // ray parameter of the current point
+    float tend;                 // ray parameter where the ray leaves the grid
     float cx, cy, cz;           // ray parameter of plane 0 per axis
     float dtx, dty, dtz;        // per plane (0 for an axis with |k| <= 1e-15: never crossed)
+    float qx, qy, qz;           // next plane per axis (exact in FP32)
+    int mx, my, mz;             // cell number per step along each axis
+    int cell;
+    Pend<float> pd;
+    bool done;
+    int steps;
+    int cell0;
+    static constexpr int fallbacks = 0;
+    static constexpr float rho = -1.f;
+    SKG_D int nscanned() const { return 0; }
 
-    SKG_D static void axis(float org, float h, float o, float k, int c, float& c0, float& dt, float& tn) {
+    SKG_D static void axis(float org, float h, float o, float k, int c, int n, float& c0, float& dt, float& q, float& tn,
+                           float& end) {
         if (fabsf(k) > 1e-15f) {
             const float u = 1.f / k;
             c0 = (org - o) * u; dt = h * u;
-            tn = fmaf((float)(k < 0.f ? c : c + 1), dt, c0);
+            q = (float)(k < 0.f ? c : c + 1);
+            tn = fmaf(q, dt, c0);
+            end = fminf(end, fmaf(k < 0.f ? 0.f : (float)n, dt, c0));
         } else {
-            c0 = 0.f; dt = 0.f; tn = FLT_MAX;
+            c0 = 0.f; dt = 0.f; q = 0.f; tn = FLT_MAX;
         }
     }
     SKG_D void init(const DevGrid& g, float rx, float ry, float rz, float dx, float dy, float dz, int hint = -1) {
-        CartStepperRef<float>::init(g, rx, ry, rz, dx, dy, dz, hint);
+        CartStepperRef<float> e;
+        e.init(g, rx, ry, rz, dx, dy, dz, hint);
+        pd = e.pd; done = e.done; steps = 0; cell0 = e.cell0;
         tc = 0.f;
         if (done) return;
-        if (isnan(kx) || isnan(ky) || isnan(kz)) { done = true; return; }   // the reference walk stops
-        axis(g.corg[0], g.cstep[0], x, kx, i, cx, dtx, tx);
-        axis(g.corg[1], g.cstep[1], y, ky, j, cy, dty, ty);
-        axis(g.corg[2], g.cstep[2], z, kz, k, cz, dtz, tz);
+        if (isnan(dx) || isnan(dy) || isnan(dz)) { done = true; return; }   // the reference walk stops
+        tend = FLT_MAX;
+        axis(g.corg[0], g.cstep[0], e.x, dx, e.i, g.nx, cx, dtx, qx, tx, tend);
+        axis(g.corg[1], g.cstep[1], e.y, dy, e.j, g.ny, cy, dty, qy, ty, tend);
+        axis(g.corg[2], g.cstep[2], e.z, dz, e.k, g.nz, cz, dtz, qz, tz, tend);
+        if (!(fabsf(tx) <= FLT_MAX && fabsf(ty) <= FLT_MAX && fabsf(tz) <= FLT_MAX)) done = true;
+        mz = dz < 0.f ? -1 : 1;
+        my = dy < 0.f ? -g.nz : g.nz;
+        mx = (dx < 0.f ? -g.nz : g.nz) * g.ny;
+        cell = e.k + g.nz * (e.j + g.ny * e.i);
     }
     static constexpr bool resumable = false;
     SKG_D bool next(const DevGrid& g, int& m, float& ds) {
         if (pd.pop(ds)) { m = -1; return true; }
         return walk(g, m, ds);
     }
-    // one cell step: the crossed axis (the reference's tie order) and every per-axis value a select
+    // One cell step: the nearest wall (the reference's tie order x, y, z) and, predicated, its axis's
+    // next plane, wall and cell.  The ray leaves the grid with the first wall at tend: crossings that
+    // share that parameter have no length, and the reference drops them.
     SKG_D bool walk(const DevGrid& g, int& m, float& ds) {
         while (!done) {
             if (++steps > g.max_steps) { done = true; return false; }
-            m = k + g.nz * j + g.nz * g.ny * i;
-            const int a = (tx <= ty && tx <= tz) ? 0 : (ty <= tz ? 1 : 2);
-            const float t = a == 0 ? tx : (a == 1 ? ty : tz);
-            if (t != t) { done = true; return false; }   // NaN direction
-            const float dt = a == 0 ? dtx : (a == 1 ? dty : dtz);
-            const bool neg = dt < 0.f;
-            const int n = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
-            const int q = (a == 0 ? i : (a == 1 ? j : k)) + (neg ? -1 : 1);
-            if (a == 0) i = q;
-            if (a == 1) j = q;
-            if (a == 2) k = q;
-            if (q >= n || q < 0) done = true;
-            else {
-                const float c0 = a == 0 ? cx : (a == 1 ? cy : cz);
-                const float tn = fmaf((float)(neg ? q : q + 1), dt, c0);
-                if (a == 0) tx = tn;
-                if (a == 1) ty = tn;
-                if (a == 2) tz = tn;
-            }
+            m = cell;
+            const float t = fminf(fminf(tx, ty), tz);
+            const bool ax = tx <= t, ay = !ax && ty <= t;
+            if (ax) { qx += copysignf(1.f, dtx); tx = fmaf(qx, dtx, cx); cell += mx; }
+            else if (ay) { qy += copysignf(1.f, dty); ty = fmaf(qy, dty, cy); cell += my; }
+            else { qz += copysignf(1.f, dtz); tz = fmaf(qz, dtz, cz); cell += mz; }
+            done = t >= tend;
             const float d = t - tc;
             tc = t;
             if (d > 0.f) { ds = d; return true; }   // DustGridPath::addSegment drops ds <= 0
