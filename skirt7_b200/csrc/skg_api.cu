@@ -856,7 +856,7 @@ int skg_run_phase(skg_ctx* ctx, int phase, const int32_t* ells, int nell, uint64
         int precision = opts ? opts->precision : SKG_PREC_FP32;
         int blocks = opts ? opts->blocks : 0;
         CK(cudaEventRecord(ctx->ev0, s));
-        CK(ctx->waves.begin(P, ctx->grid.type, tree_walk_of(ctx->grid), precision, 1, npool, blocks,
+        CK(ctx->waves.begin(P, ctx->grid.type, tree_walk_of(ctx->grid), precision, 1, npool, total <= npool, blocks,
                             carries_luminosity(ctx->hs, phase), s, &g));
         CK(cudaEventRecord(ctx->ev1, s));
         return SKG_OK;
@@ -1161,7 +1161,7 @@ struct skg_batch {
     cudaGraphExec_t graph = nullptr;
     int g_type = -1, g_bk = -1, g_prec = -1, g_blocks = -1;
     size_t g_npool = 0;
-    bool g_absorbs = false;
+    bool g_absorbs = false, g_fits = false;
     int g_waves = 0;                       // waves captured in the graph
     bool g_stale = false;                  // a replay needed more waves than captured
     cudaStream_t g_stream = nullptr;
@@ -1330,11 +1330,11 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
             CK(cudaMemsetAsync(T.err, 0, sizeof(unsigned), q));
             // every slot's DevGrid is copied into shared memory: size for the batch's capacity
             CK(b->waves.begin(P, gtype < 0 ? SKG_GRID_CARTESIAN : gtype, gbk < 0 ? TW_ROPE : gbk, precision, T.max_slots, npool,
-                              blocks, absorbs, q));
+                              total <= npool, blocks, absorbs, q));
         };
         CK(cudaEventRecord(b->ev0, s));
         if (flags & SKG_BATCH_GRAPH) {
-            bool same = b->graph && !b->g_stale && b->g_absorbs == absorbs && b->g_type == gtype && b->g_bk == gbk && b->g_prec == precision &&
+            bool same = b->graph && !b->g_stale && b->g_absorbs == absorbs && b->g_fits == (total <= npool) && b->g_type == gtype && b->g_bk == gbk && b->g_prec == precision &&
                         b->g_blocks == blocks && b->g_npool == npool;
             if (!same) {
                 if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
@@ -1347,7 +1347,7 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
                 cudaGraphDestroy(gr);
                 CK(e);
                 b->g_type = gtype; b->g_bk = gbk; b->g_prec = precision; b->g_blocks = blocks; b->g_npool = npool;
-                b->g_absorbs = absorbs;
+                b->g_absorbs = absorbs; b->g_fits = total <= npool;
                 b->g_waves = b->waves.waves(); b->g_stale = false;
             }
             CK(cudaGraphLaunch(b->graph, s));

@@ -193,6 +193,7 @@ struct WaveParams {
     int* intlist;                     // records it found at their interaction point (J_INT)
     int2* rlist;                      // the paths that interact: (packet, place in walk order) (J_REWALK;
                                       // the memory of the lists above, which the launch pass has consumed)
+    int tail_lanes;                   // tail pass: packets to a warp
     int path_tau;                     // the path jobs need the optical depth alone (walked with the peel-offs)
     float4* ckpt;                     // per packet record: checkpoints of its path walk
     // walk order of the wave's jobs (order_kernel); hist == nullptr: as appended
@@ -200,7 +201,7 @@ struct WaveParams {
     unsigned* bin0;                   // [2][JOB_BINS] first place of each bin
     uint2* jkey;                      // per job (its bin, its rank within it)
     int* spath;                       // packets of the path jobs
-    int4* speel;                      // peel-off jobs: (packet, group, job index, 0)
+    uint2* speel;                     // peel-off jobs: (packet << 4 | group, job index)
     // the grid of a single-simulation launch: the traversal kernels' instantiation for one slot
     // reads it from their parameters (constant-bank operands, no load instructions per cell step)
     DevGrid g0;

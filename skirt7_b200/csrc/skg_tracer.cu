@@ -118,6 +118,19 @@ namespace skg {
 #define SKG_CKPT_STRIDE 16
 #endif
 
+// phases of at most this many packets (Cartesian, other grids) run in the tail pass alone: with a few
+// lanes of every warp busy a wave lasts as long as its longest walk, about 100 us each on a small Cartesian grid, and a
+// phase takes some twenty of them.  Waves against the tail pass alone, ms per phase: 40x40x20 Cartesian
+// grid 10^4 packets 2.10 / 0.90, 4*10^4 2.37 / 1.92, 8*10^4 2.66 / 2.55; 100x100x50 4*10^4 3.37 / 3.28, 8*10^4 3.60 /
+// 4.50; octree with four observers 4*10^3 1.70 / 1.00, 10^4 1.80 / 1.73, 2*10^4 1.87 / 2.75; 10^6 Voronoi
+// cells 10^4 28.8 / 28.2, 2*10^4 34.2 / 42.5
+#ifndef SKG_TAIL_ONLY_CART
+#define SKG_TAIL_ONLY_CART (1 << 15)
+#endif
+#ifndef SKG_TAIL_ONLY
+#define SKG_TAIL_ONLY (1 << 13)
+#endif
+
 enum Cnt : int { C_PACKETS = 0, C_STEPS, C_TRAV, C_SCATT, C_PEEL, C_ABS, C_PIX, C_NBR, C_FB, C_ERR, C_N };
 
 template<typename R> SKG_D double rho_load(const DevScene& S, size_t i);
@@ -832,7 +845,7 @@ __global__ void __launch_bounds__(256) order_kernel(const WaveParams W) {
         const uint2 k = W.jkey[j];
         const int2 jb = W.jobs[j];
         if (i < npath) W.spath[W.bin0[k.x] + k.y] = jb.x;
-        else W.speel[W.bin0[JOB_BINS + k.x] + k.y] = make_int4(jb.x, jb.y, (int)j, 0);
+        else W.speel[W.bin0[JOB_BINS + k.x] + k.y] = make_uint2((unsigned)jb.x << 4 | (unsigned)jb.y, j);
     }
 }
 
@@ -1038,8 +1051,8 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                         w.p = W.hist ? W.spath[i] : W.jobs[i].x;
                         w.out = (int)i;
                     } else if (W.hist) {
-                        const int4 o = W.speel[i - npath];
-                        w.p = o.x; grp = o.y; w.out = o.z;
+                        const uint2 o = W.speel[i - npath];
+                        w.p = (int)(o.x >> 4); grp = (int)(o.x & 15); w.out = (int)o.y;
                     } else {
                         w.out = W.npool + (int)(i - npath);
                         const int2 jb = W.jobs[w.out];
@@ -1309,8 +1322,11 @@ SKG_D void tail_path(const WaveParams& W, const DevGrid& g, const DevScene& S, i
 template<typename R, template<typename> class Stepper>
 __global__ void __launch_bounds__(128) tail_kernel(const WaveParams W) {
     const RunParams& P = W.R;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= W.npool) return;
+    // tail_lanes packets to a warp: few packets run side by side in few lanes, which then seldom
+    // wait for one another's branches
+    const int lane = threadIdx.x & 31;
+    const int p = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * W.tail_lanes + lane;
+    if (lane >= W.tail_lanes || p >= W.npool) return;
     Packet& K = W.pk[p];
     int state = K.state;
     if (state == PK_DONE) return;
@@ -1488,7 +1504,8 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
 
 template<typename R, template<typename> class Stepper>
 cudaError_t enqueue_tail(const WaveParams& W, cudaStream_t s) {
-    tail_kernel<R, Stepper><<<(W.npool + 127) / 128, 128, 0, s>>>(W);
+    const int warps = (W.npool + W.tail_lanes - 1) / W.tail_lanes;
+    tail_kernel<R, Stepper><<<(warps + 3) / 4, 128, 0, s>>>(W);
     return cudaGetLastError();
 }
 
@@ -1529,8 +1546,7 @@ WaveRunner::~WaveRunner() {
     for (cudaEvent_t e : ev_) cudaEventDestroy(e);
     for (cudaEvent_t e : tail_ev_) if (e) cudaEventDestroy(e);
     // (a runner that never reserved frees nothing: no device-wide synchronisation)
-    for (void* p : {(void*)pk_, (void*)free_, (void*)ckpt_, (void*)ctr_, (void*)bins_, (void*)jkey_, (void*)spath_,
-                    (void*)speel_})
+    for (void* p : {(void*)pk_, (void*)free_, (void*)ckpt_, (void*)ctr_, (void*)bins_, (void*)order_})
         if (p) cudaFree(p);
     for (int b = 0; b < 2; b++)
         for (void* p : {(void*)jobs_[b], (void*)jtau_[b], (void*)jL_[b]}) if (p) cudaFree(p);
@@ -1552,7 +1568,7 @@ static bool ckpt_grid(int grid_type) {
 // 262 against 254 ms; below these bounds the sort costs more than it gives (2.4*10^5 packets on a small octree
 // 4.1 against 4.7 ms; Cartesian densities are a few MB: a batch of 24 fit variants 53.5 against 56.2 ms).
 static bool order_pays(int grid_type, size_t pool, size_t walk_bytes) {
-    return grid_type != SKG_GRID_CARTESIAN && pool >= ((size_t)3 << 19) && walk_bytes >= ((size_t)8 << 20);
+    return grid_type != SKG_GRID_CARTESIAN && pool >= ((size_t)3 << 19) && pool < ((size_t)1 << 28) && walk_bytes >= ((size_t)8 << 20);
 }
 
 cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes) {
@@ -1594,11 +1610,9 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t 
         cap_jobs_ = jobs;
     }
     if (order_on_ && jobs > cap_order_) {
-        cudaFree(jkey_); cudaFree(speel_); cudaFree(spath_);
-        jkey_ = nullptr; speel_ = nullptr; spath_ = nullptr; cap_order_ = 0;
-        if ((e = cudaMalloc(&jkey_, jobs * sizeof(uint2))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&speel_, jobs * sizeof(int4))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&spath_, jobs * sizeof(int))) != cudaSuccess) return e;
+        // (peel-off jobs, then the path jobs)
+        cudaFree(order_); order_ = nullptr; cap_order_ = 0;
+        if ((e = cudaMalloc(&order_, jobs * sizeof(uint2))) != cudaSuccess) return e;
         cap_order_ = jobs;
     }
     return cudaSuccess;
@@ -1617,7 +1631,9 @@ cudaError_t WaveRunner::enqueue(int n) {
         W.freelist = free_; W.intlist = free_ + npool_; W.rlist = reinterpret_cast<int2*>(free_); W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
         W.g0 = g0_;
         W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
-        W.jkey = jkey_; W.spath = spath_; W.speel = speel_;
+        // (a job's key lies where its optical depth will)
+        W.jkey = reinterpret_cast<uint2*>(jtau_[b]); W.speel = order_;
+        W.spath = reinterpret_cast<int*>(order_ + (cap_order_ - npool_));
         if ((e = cudaMemsetAsync(ctr_ + J_N * b, 0, J_N * sizeof(unsigned), stream_)) != cudaSuccess) return e;
         if (timed_) {
             while (ev_.size() < 3 * (size_t)(w + 1)) {
@@ -1632,6 +1648,11 @@ cudaError_t WaveRunner::enqueue(int n) {
     }
     waves_ += n;
     if ((e = cudaMemcpyAsync(h_ctr_, ctr_, NCTR * sizeof(unsigned), cudaMemcpyDeviceToHost, stream_)) != cudaSuccess) return e;
+    return record_copied();
+}
+
+cudaError_t WaveRunner::record_copied() {
+    cudaError_t e;
     // inside stream capture the record must become a graph node that the host can wait on
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if ((e = cudaStreamIsCapturing(stream_, &cs)) != cudaSuccess) return e;
@@ -1640,7 +1661,8 @@ cudaError_t WaveRunner::enqueue(int n) {
 }
 
 cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, int precision, int nslots,
-                              size_t npool, int trav_blocks, bool absorbs, cudaStream_t s, const DevGrid* one_grid) {
+                              size_t npool, bool fits, int trav_blocks, bool absorbs, cudaStream_t s,
+                              const DevGrid* one_grid) {
     if (npool == 0 || npool > cap_pool_) return cudaErrorInvalidValue;
     P_ = P; grid_type_ = grid_type; tree_walk_ = tree_walk; precision_ = precision; nslots_ = nslots;
     one_ = one_grid != nullptr && nslots == 1;
@@ -1658,16 +1680,20 @@ cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, 
     if ((e = cudaMemsetAsync(pk_, 0, npool * sizeof(Packet), s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(ctr_, 0, NCTR * sizeof(unsigned), s)) != cudaSuccess) return e;
     pending_ = true;
-    return enqueue(estimate);
+    tail_only_ = tail_div_ > 0 && fits && npool <= (size_t)(grid_type == SKG_GRID_CARTESIAN ? SKG_TAIL_ONLY_CART : SKG_TAIL_ONLY);
+    if (!tail_only_) return enqueue(estimate);
+    if ((e = enqueue_tail()) != cudaSuccess) return e;
+    return record_copied();
 }
 
 cudaError_t WaveRunner::enqueue_tail() {
-    const int b = (waves_ - 1) & 1;               // the last wave's jobs hold the pending peel-offs
+    const int b = (waves_ + 1) & 1;               // the last wave's jobs hold the pending peel-offs
     WaveParams W;
     W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = waves_;
     W.jobs = nullptr; W.jtau = nullptr; W.jL = nullptr; W.jcount = ctr_ + J_N * (b ^ 1);
     W.pjobs = jobs_[b]; W.pjtau = jtau_[b]; W.pjL = jL_[b];
     W.last_busy = ctr_ + 2 * J_N;
+    W.tail_lanes = waves_ ? 32 : std::min(32, std::max(1, npool_ / (dev_sms() * 16)));
     W.freelist = nullptr; W.intlist = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
     W.hist = nullptr; W.bin0 = nullptr; W.jkey = nullptr; W.spath = nullptr; W.speel = nullptr;
     cudaError_t e;
@@ -1698,6 +1724,7 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
             }
             std::this_thread::sleep_for(std::chrono::microseconds(50));
         }
+        if (tail_only_) { pending_ = false; break; }
         const unsigned busy = h_ctr_[J_N * ((waves_ - 1) & 1) + J_BUSY];
         if (busy == 0) {
             pending_ = false;

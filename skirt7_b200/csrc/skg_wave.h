@@ -27,17 +27,18 @@ public:
     // grid, with the pool whether the jobs are walked in spatial order.
     cudaError_t reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes);
     // Enqueues the reset of the pool and the first waves of a phase on stream s.  P holds the
-    // staged tables; absorbs: some simulation tallies absorption in this phase or has several dust
+    // staged tables; fits: the phase has no more packets than the pool; absorbs: some simulation tallies absorption in this phase or has several dust
     // components (its path walks then carry luminosities); nslots the slots whose DevGrid the traversal pass keeps in shared memory;
     // tree_walk the FP32 tree walk (TreeWalk) of tree grids; one_grid (host copy), when given with
     // nslots = 1, the grid the FP32 traversal kernels take as a kernel parameter instead.
     cudaError_t begin(const RunParams& P, int grid_type, int tree_walk, int precision, int nslots,
-                      size_t npool, int trav_blocks, bool absorbs, cudaStream_t s, const DevGrid* one_grid = nullptr);
+                      size_t npool, bool fits, int trav_blocks, bool absorbs, cudaStream_t s,
+                      const DevGrid* one_grid = nullptr);
     // Waits for the enqueued waves and enqueues more until no packet is left; then records
     // `end` (if given) on the phase's stream.  timeout_ms < 0 waits without limit.
     cudaError_t finish(int timeout_ms, cudaEvent_t end, bool* timed_out);
     // A captured begin() (pool reset and n waves) was launched as a graph on stream s.
-    void replayed(cudaStream_t s, int n) { pending_ = true; stream_ = s; waves_ = n; }
+    void replayed(cudaStream_t s, int n) { pending_ = true; stream_ = s; waves_ = n; tail_only_ = n == 0; }
     bool pending() const { return pending_; }
     int waves() const { return waves_; }
     size_t pool_capacity() const { return cap_pool_; }
@@ -54,6 +55,7 @@ public:
 private:
     cudaError_t enqueue(int n);
     cudaError_t enqueue_tail();
+    cudaError_t record_copied();
 
     Packet* pk_ = nullptr;
     int* free_ = nullptr;             // [pool] records freed in a wave, [pool] records at their
@@ -66,9 +68,7 @@ private:
     double* jL_[2] = {nullptr, nullptr};
     size_t cap_jobs_ = 0;
     unsigned* bins_ = nullptr;        // [2][JOB_BINS] counts, [2][JOB_BINS] first places (walk order)
-    uint2* jkey_ = nullptr;
-    int* spath_ = nullptr;
-    int4* speel_ = nullptr;
+    uint2* order_ = nullptr;          // peel-off jobs in walk order; at its end, the path jobs' packets
     size_t cap_order_ = 0;
     bool order_on_ = false;           // the running phase walks its jobs in spatial order
     bool path_tau_ = false;
@@ -90,6 +90,7 @@ private:
     bool timed_ = false;               // the running phase records ev_
     int tail_div_ = 16;
     bool ckpt_on_ = true;              // path-walk checkpoints (environment variable SKG_CKPT=0: off)
+    bool tail_only_ = false;           // the phase is the tail pass alone
     bool tail_ran_ = false;            // the phase ended with the tail pass
     cudaEvent_t tail_ev_[2] = {nullptr, nullptr};
 };
