@@ -1159,7 +1159,7 @@ struct skg_batch {
     int* h_ells = nullptr;
     cudaEvent_t copied = nullptr;          // the previous launch's tables have been read
     cudaGraphExec_t graph = nullptr;
-    int g_type = -1, g_bk = -1, g_prec = -1, g_blocks = -1;
+    int g_type = -1, g_bk = -1, g_prec = -1, g_blocks = -1, g_gen = -1;
     size_t g_npool = 0;
     bool g_absorbs = false, g_fits = false;
     int g_waves = 0;                       // waves captured in the graph
@@ -1334,7 +1334,8 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
         };
         CK(cudaEventRecord(b->ev0, s));
         if (flags & SKG_BATCH_GRAPH) {
-            bool same = b->graph && !b->g_stale && b->g_absorbs == absorbs && b->g_fits == (total <= npool) && b->g_type == gtype && b->g_bk == gbk && b->g_prec == precision &&
+            bool same = b->graph && !b->g_stale && b->g_absorbs == absorbs && b->g_fits == (total <= npool) &&
+                        b->g_gen == b->waves.generation() && b->g_type == gtype && b->g_bk == gbk && b->g_prec == precision &&
                         b->g_blocks == blocks && b->g_npool == npool;
             if (!same) {
                 if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
@@ -1347,7 +1348,7 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
                 cudaGraphDestroy(gr);
                 CK(e);
                 b->g_type = gtype; b->g_bk = gbk; b->g_prec = precision; b->g_blocks = blocks; b->g_npool = npool;
-                b->g_absorbs = absorbs; b->g_fits = total <= npool;
+                b->g_absorbs = absorbs; b->g_fits = total <= npool; b->g_gen = b->waves.generation();
                 b->g_waves = b->waves.waves(); b->g_stale = false;
             }
             CK(cudaGraphLaunch(b->graph, s));

@@ -49,8 +49,11 @@ namespace skg {
 // own state alone, and the path's long end (path_end_kernel) holds none of them.  Octree disk, 2*10^7
 // packets: traversal pass 179.6 ms against 209.8 with the end of the path and the re-walk inside the
 // path-job kernel (220 bytes of spills at 64 registers); fit-variant batch 46.2 against 53.5 ms.
-#ifndef SKG_VOR_PATH_MIN_BLOCKS
-#define SKG_VOR_PATH_MIN_BLOCKS 3
+// blocks per SM of the path and re-walk kernels: 3 (80 registers, no spills) against 4 (64, spilling
+// 64-112 bytes): traversal pass of the k-d tree disk with absorption 21.3 against 22.8 ms, Cartesian
+// disk with absorption 6.75 against 7.35, re-walks of the octree disk 1.4 ms of 157 less
+#ifndef SKG_PATH_MIN_BLOCKS
+#define SKG_PATH_MIN_BLOCKS 3
 #endif
 // programmatic dependent launch of the peel-off-job kernel after the path-job kernel
 #ifndef SKG_PDL
@@ -852,11 +855,31 @@ __global__ void __launch_bounds__(256) order_kernel(const WaveParams W) {
 // ---------------------------------------------------------------------------------------------
 // traversal pass
 
+// 1 - e^-x for x >= 0, to about one unit in the last place: the Taylor series up to x^10 below 1/16
+// (its next term is below 10^-19 of the sum), expm1 above.  A path step's optical depth is small, and the
+// series takes ten FP64 operations and no branches.
+SKG_D double one_minus_exp(double x) {
+    if (x < 0.0625) {
+        double p = -1.0 / 3628800;
+        p = fma(p, x, 1.0 / 362880);
+        p = fma(p, x, -1.0 / 40320);
+        p = fma(p, x, 1.0 / 5040);
+        p = fma(p, x, -1.0 / 720);
+        p = fma(p, x, 1.0 / 120);
+        p = fma(p, x, -1.0 / 24);
+        p = fma(p, x, 1.0 / 6);
+        p = fma(p, x, -0.5);
+        p = fma(p, x, 1.0);
+        return p * x;
+    }
+    return -expm1(-x);
+}
+
 // Absorption in cell m of a path step: simulateescapeandabsorption (MonteCarloSimulation.cpp:441-462)
 // with OligoDustSystem::absorb / PanDustSystem::absorb.  The tables are wavelength-major on the
 // device ([ell][m]): a wave carries the packets of one or two wavelengths (packets are handed out
 // wavelength by wavelength), so its tallies fall in one slice of the table that stays in L2.  v1 = L e^-tau on entry (a running product,
-// one expm1 per absorbing step: L e^-tau (1 - e^-dtau) = -v1 expm1(-dtau)); v2 accumulates L_sca with
+// each step absorbs v1 (1 - e^-dtau)); v2 accumulates L_sca with
 // the local albedo when there are several dust components.  Returns 1 when a tally was stored.
 template<typename R>
 SKG_D int absorb_step(const DevScene& S, int phase, int m, int ell, double dtau, double& v1, double& v2) {
@@ -865,9 +888,8 @@ SKG_D int absorb_step(const DevScene& S, int phase, int m, int ell, double dtau,
     double* labs = (phase == SKG_PHASE_STELLAR) ? S.labs_stel : S.labs_dust;
     if (S.ncomp == 1) {
         if (!store) return 0;
-        const double em = expm1(-dtau);
-        const double Lintm = -v1 * em;
-        v1 += v1 * em;
+        const double Lintm = v1 * one_minus_exp(dtau);
+        v1 -= Lintm;
         atomicAdd(labs + (size_t)ell * S.ncells + m, (1.0 - S.albedo[ell]) * Lintm);
         return 1;
     }
@@ -877,9 +899,8 @@ SKG_D int absorb_step(const DevScene& S, int phase, int m, int ell, double dtau,
         ksca += rh * S.ksca[h * S.nlambda + ell]; kext += rh * S.kext[h * S.nlambda + ell];
     }
     const double alb = (kext > 0.0) ? ksca / kext : 0.0;
-    const double em = expm1(-dtau);
-    const double Lintm = -v1 * em;
-    v1 += v1 * em;
+    const double Lintm = v1 * one_minus_exp(dtau);
+    v1 -= Lintm;
     v2 += alb * Lintm;
     if (!store) return 0;
     atomicAdd(labs + (size_t)ell * S.ncells + m, (1.0 - alb) * Lintm);
@@ -965,7 +986,8 @@ SKG_D bool resume_ckpt(const WaveParams& W, const DevGrid& g, int p, int nck, do
 enum TravMode : int { TRAV_PATH = 1, TRAV_TAU = 2, TRAV_REWALK = 3 };
 // Resident blocks per SM of each instantiation.
 template<int MODE, template<typename> class Stepper> struct TravBlocks { static constexpr int value = SKG_TRAV_MIN_BLOCKS; };
-template<> struct TravBlocks<TRAV_PATH, VoronoiStepper> { static constexpr int value = SKG_VOR_PATH_MIN_BLOCKS; };
+template<template<typename> class Stepper> struct TravBlocks<TRAV_PATH, Stepper> { static constexpr int value = SKG_PATH_MIN_BLOCKS; };
+template<template<typename> class Stepper> struct TravBlocks<TRAV_REWALK, Stepper> { static constexpr int value = SKG_PATH_MIN_BLOCKS; };
 
 template<typename R, template<typename> class Stepper>
 struct HasCkpt { static constexpr bool value = SKG_CKPT && Resumable<Stepper<R>>::value; };
@@ -1021,7 +1043,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
     int p = 0, slot = 0, ell = 0;
     double tau = 0;                   // optical depth walked
     // TRAV_PATH: v1 = L e^-tau (the luminosity that reaches the current cell, kept as a running
-    // product: one expm1 per absorbing cell step), v2 = L_sca (several dust components);
+    // product), v2 = L_sca (several dust components);
     // TRAV_REWALK: v1 = path length walked, v2 = the interaction optical depth
     double v1 = 0, v2 = 0;
     float kext1 = -1.f;
@@ -1029,6 +1051,8 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
     unsigned long long c_nbr = 0;
     Stepper<R> st;
     int nck = 0;                      // checkpoints of the path walk
+    double* labs = nullptr;           // TRAV_PATH: tallies of the job's wavelength (one dust component), if kept
+    double kabs = 0;                  // 1 - albedo
 
     while (true) {
         const unsigned want = __ballot_sync(FULL, j < 0);
@@ -1095,7 +1119,15 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                         if (MODE == TRAV_PATH || (job0 == 0 && j < (int)npath)) {
                             if (w.hint == -2) W.pk[p].pos_cell = st.cell0;
                         }
-                        if (MODE == TRAV_PATH) { v1 = W.pk[p].L; v2 = 0; nck = 0; }
+                        if (MODE == TRAV_PATH) {
+                            v1 = W.pk[p].L; v2 = 0; nck = 0;
+                            const DevScene& S = *s_scene[slot];
+                            labs = nullptr;
+                            if (S.ncomp == 1 && (phase == SKG_PHASE_STELLAR ? S.store_abs != 0 : phase == SKG_PHASE_DUST_SELFABS)) {
+                                labs = (phase == SKG_PHASE_STELLAR ? S.labs_stel : S.labs_dust) + (size_t)ell * S.ncells;
+                                kabs = 1.0 - S.albedo[ell];
+                            }
+                        }
                     }
                 }
                 used = min(have, used + __popc(want));
@@ -1120,7 +1152,14 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                 if (MODE == TRAV_TAU) {
                     tau += dtau;
                 } else if (MODE == TRAV_PATH) {
-                    c_abs += absorb_step<R>(S, phase, m, ell, dtau, v1, v2);
+                    if (labs) {
+                        const double Lintm = v1 * one_minus_exp(dtau);
+                        v1 -= Lintm;
+                        atomicAdd(labs + m, kabs * Lintm);
+                        c_abs++;
+                    } else if (kext1 < 0.f) {
+                        c_abs += absorb_step<R>(S, phase, m, ell, dtau, v1, v2);
+                    }
                     tau += dtau;
                     if constexpr (CKPT) {
                         if (W.ckpt && nck < SKG_CKPT_N && st.steps >= (nck + 1) * SKG_CKPT_STRIDE && !st.done) {
@@ -1573,6 +1612,7 @@ static bool order_pays(int grid_type, size_t pool, size_t walk_bytes) {
 
 cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes) {
     cudaError_t e;
+    const size_t had[5] = {cap_pool_, cap_ckpt_, cap_jobs_, cap_order_, bins_ != nullptr};
     order_on_ = order_pays(grid_type, pool, walk_bytes);
     if (!ctr_) {
         if ((e = cudaMalloc(&ctr_, NCTR * sizeof(unsigned))) != cudaSuccess) return e;
@@ -1615,6 +1655,8 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t 
         if ((e = cudaMalloc(&order_, jobs * sizeof(uint2))) != cudaSuccess) return e;
         cap_order_ = jobs;
     }
+    const size_t has[5] = {cap_pool_, cap_ckpt_, cap_jobs_, cap_order_, bins_ != nullptr};
+    if (std::memcmp(had, has, sizeof(had)) != 0) generation_++;
     return cudaSuccess;
 }
 

@@ -42,6 +42,8 @@ public:
     bool pending() const { return pending_; }
     int waves() const { return waves_; }
     size_t pool_capacity() const { return cap_pool_; }
+    // changes when reserve() has moved a buffer (a captured launch then holds freed memory)
+    int generation() const { return generation_; }
     // With timing on, each wave's two kernels are bracketed by events (not inside graph capture).
     bool timing = false;
     // Device time of the finished phase's event passes and traversal passes (ms).
@@ -67,6 +69,7 @@ private:
     double* jtau_[2] = {nullptr, nullptr};
     double* jL_[2] = {nullptr, nullptr};
     size_t cap_jobs_ = 0;
+    int generation_ = 0;
     unsigned* bins_ = nullptr;        // [2][JOB_BINS] counts, [2][JOB_BINS] first places (walk order)
     uint2* order_ = nullptr;          // peel-off jobs in walk order; at its end, the path jobs' packets
     size_t cap_order_ = 0;
