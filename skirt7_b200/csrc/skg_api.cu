@@ -247,7 +247,18 @@ DevGrid make_grid(Allocs& A, const skg_grid& g, cudaStream_t s) {
         G.vnbr = upload(A, g.vnbr_ids, (size_t)tot, s);
         // FP32 bisector planes: n = p_i - p_r, w = n . (p_i + p_r)/2 (computed in FP64, stored FP32);
         // walls -1..-6 as axis planes with outward normals
-        std::vector<float4> pl((size_t)tot);
+        std::vector<int2> po(n);
+        int64_t ptot = 0;
+        for (int m = 0; m < n; m++) {
+            po[m].x = (int)ptot;
+            ptot += (g.vnbr_offsets[m + 1] - g.vnbr_offsets[m] + 1) & ~(int64_t)1;
+            REQUIRE(ptot < (1ll << 31), "too many Voronoi neighbour entries");
+            po[m].y = (int)ptot;
+        }
+        std::vector<float4> pl((size_t)ptot, make_float4(0.f, 0.f, 0.f, 0.f));
+        // with each plane the neighbour and its own entries, so that the FP32 walk reaches the next
+        // cell's planes with one load
+        std::vector<int4> nx4((size_t)ptot, make_int4(-1, 0, 0, 0));
         for (int m = 0; m < n; m++) {
             const double* pr = g.sites + 3 * (size_t)m;
             for (int64_t q = g.vnbr_offsets[m]; q < g.vnbr_offsets[m + 1]; q++) {
@@ -273,17 +284,13 @@ DevGrid make_grid(Allocs& A, const skg_grid& g, cudaStream_t s) {
                         default: throw Failure{SKG_ERR_INVALID, "invalid Voronoi wall id"};
                     }
                 }
-                pl[q] = make_float4((float)nx, (float)ny, (float)nz, (float)w);
+                const size_t at = (size_t)po[m].x + (size_t)(q - g.vnbr_offsets[m]);
+                pl[at] = make_float4((float)nx, (float)ny, (float)nz, (float)w);
+                nx4[at] = (mi >= 0) ? make_int4(mi, po[mi].x, po[mi].y, off[mi + 1] - off[mi]) : make_int4(mi, 0, 0, 0);
             }
         }
         G.vplane = upload(A, pl.data(), pl.size(), s);
-        // per entry the neighbour with its own entry range, so that the FP32 walk reaches the next
-        // cell's planes with one load
-        std::vector<int4> nx4((size_t)tot);
-        for (int64_t q = 0; q < tot; q++) {
-            int mi = g.vnbr_ids[q];
-            nx4[q] = (mi >= 0) ? make_int4(mi, off[mi], off[mi + 1], 0) : make_int4(mi, 0, 0, 0);
-        }
+        G.vpoff = upload(A, po.data(), po.size(), s);
         G.vnext = upload(A, nx4.data(), nx4.size(), s);
         G.nb = g.nb;
         size_t nb3 = (size_t)g.nb * g.nb * g.nb;
@@ -607,6 +614,33 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
             }
             H.group_start[ng] = pos;
             H.ngroups = ng;
+        }
+
+        // Voronoi: the planes ahead of each peel-off direction (about half of every list; 270 bytes per
+        // cell and group, so for scenes of few groups)
+        if (ctx->grid.type == SKG_GRID_VORONOI && sc->ncomp > 0 && H.ngroups >= 1 && H.ngroups <= 4 &&
+            (int64_t)H.ngroups * nc < (1ll << 26)) {
+            const size_t n = (size_t)H.ngroups * nc;
+            Allocs T;
+            T.stream = s;
+            int* cnt = T.alloc<int>(n + 1);
+            int* first = T.alloc<int>(n + 1);
+            const size_t sb = offset_scan_scratch_bytes((int)(n + 1));
+            char* scratch = T.alloc<char>(sb);
+            int2* po = A.alloc<int2>(n);
+            int total = 0;
+            if (cnt && first && scratch && po) {
+                CK(launch_group_counts(ctx->grid, H.gkx, H.gky, H.gkz, H.ngroups, cnt, s));
+                CK(launch_offset_scan(cnt, first, (int)(n + 1), scratch, sb, s));
+                CK(cudaMemcpyAsync(&total, first + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+                CK(cudaStreamSynchronize(s));
+                float4* gp = total > 0 ? A.alloc<float4>((size_t)total) : nullptr;
+                int4* gn = gp ? A.alloc<int4>((size_t)total) : nullptr;
+                if (gn) {
+                    CK(launch_group_planes(ctx->grid, H.gkx, H.gky, H.gkz, H.ngroups, first, gp, gn, po, s));
+                    ctx->grid.gplane = gp; ctx->grid.gnext = gn; ctx->grid.gpoff = po;
+                }
+            }
         }
 
         H.min_weight_reduction = sc->min_weight_reduction > 0 ? sc->min_weight_reduction : 1e4;

@@ -64,7 +64,7 @@ struct DevGrid {
     int lattice;
     float lorg[3], lunit[3];
 
-    // Voronoi: sites (3 doubles / float4), CSR neighbours, FP32 bisector planes per CSR entry
+    // Voronoi: sites (3 doubles / float4), CSR neighbours, FP32 bisector planes per neighbour entry
     // vplane[q] = (n.x, n.y, n.z, n.p) with n = p_i - p_r and p the bisector midpoint; walls are
     // encoded as axis planes, so s = (n.p - n.r)/(n.k) for every entry with n.k > 0.
     int nsites;
@@ -72,8 +72,16 @@ struct DevGrid {
     const float4* sitef;
     const int*    vnoff;
     const int*    vnbr;
+    // Each cell's entries start at an even place and are an even number (an odd list ends with a zero
+    // plane, which no ray crosses), so that two planes come in one 32-byte load; vpoff[m] = (first, end).
     const float4* vplane;
-    const int4*   vnext;       // per CSR entry: (neighbour, its first entry, its end entry, 0)
+    const int4*   vnext;       // per entry: (neighbour, its first entry, its end entry, its neighbour count)
+    const int2*   vpoff;
+    // The same lists for the peel-off direction of each group (scenes of few groups; null otherwise): only
+    // the planes ahead of that direction (n.k > 0), in the same order; gpoff[group * nsites + m].
+    const float4* gplane;
+    const int4*   gnext;
+    const int2*   gpoff;
     int nb;
     const int*    boff;
     const int*    bids;
@@ -1004,6 +1012,16 @@ struct TreeLatticeStepper<float> {
     }
 };
 
+// 32 bytes in one load (sm_100: 256-bit global loads)
+struct Eight { float a[8]; };
+SKG_D Eight load32(const void* p) {
+    Eight r;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(r.a[0]), "=f"(r.a[1]), "=f"(r.a[2]), "=f"(r.a[3]), "=f"(r.a[4]), "=f"(r.a[5]), "=f"(r.a[6]), "=f"(r.a[7])
+        : "l"(p));
+    return r;
+}
+
 // The lattice walk on the octant records: the walls ahead, the density and the ropes of the exit
 // walls of the walk's direction octant come ready from one 32-byte record, where the lattice record
 // has to be decoded every step (three codes to walls, the rope to a reference).  The walls are the
@@ -1029,11 +1047,9 @@ struct TreeOctantStepper<float> {
 
     SKG_D void load(const DevGrid& g) {
         const uint4* p = g.orec + 2 * (size_t)(unsigned)idx;
-        uint32_t a0, a1, a2, a3, a4, a5, a6, a7;
-        asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3), "=r"(a4), "=r"(a5), "=r"(a6), "=r"(a7) : "l"(p));
-        wx = __uint_as_float(a0); wy = __uint_as_float(a1); wz = __uint_as_float(a2); wrho = __uint_as_float(a3);
-        gx_ = (int)a4; gy_ = (int)a5; gz_ = (int)a6;
+        const Eight r = load32(p);
+        wx = r.a[0]; wy = r.a[1]; wz = r.a[2]; wrho = r.a[3];
+        gx_ = __float_as_int(r.a[4]); gy_ = __float_as_int(r.a[5]); gz_ = __float_as_int(r.a[6]);
     }
     // does cell c hold the point? (its lattice record)
     SKG_D static bool holds(const DevGrid& g, int c, float px, float py, float pz) {
@@ -1122,9 +1138,6 @@ struct TreeOctantStepper<float> {
 
 // =============================================================================================
 // Voronoi
-#ifndef SKG_VOR_NODIV
-#define SKG_VOR_NODIV 1
-#endif
 template<typename R> SKG_D V3<R> site_pos(const DevGrid& g, int m);
 template<> SKG_D V3<double> site_pos<double>(const DevGrid& g, int m) {
     const double* p = g.site + 3 * (size_t)m; return mk3(p[0], p[1], p[2]);
@@ -1163,6 +1176,8 @@ struct VoronoiStepper {
     R x, y, z, kx, ky, kz;
     int mr;
     int qb, qe;                 // neighbour entries of the current cell (FP32 walk; qe < 0: not read yet)
+    int nnb;                    // its number of neighbours
+    int group = -1;             // FP32 walk: the direction group whose lists it scans (-1: the full lists)
     Pend<R> pd;
     bool done;
     int steps;
@@ -1261,58 +1276,75 @@ SKG_D bool VoronoiStepper<double>::walk(const DevGrid& g, int& m, double& ds) {
     return false;
 }
 
-// FP32: precomputed bisector planes, one 16-byte load per neighbour entry
+SKG_D float vor_den(float nx, float ny, float nz, float kx, float ky, float kz) { return nx * kx + ny * ky + nz * kz; }
+
+// planes a lane has in flight while it scans a cell's walls, in pairs.  The scan waits on its loads (a
+// 10^6-site grid holds 0.5 GB of planes), one 16-byte plane in a line of its own each: two planes per load halve the L1
+// work, a batch of loads at once the waiting, and the group lists halve the planes of a peel-off.
+// 2*10^6 packets on 10^6 sites: 243 ms a pass before; 2, 4 and 5 pairs at 4 blocks per SM 169, 154 and 156 ms,
+// 5 and 6 pairs at 3 blocks 154 and 149 ms; 10^5 packets on 2*10^4 sites 12.4 before, 9.9 with 4, 9.2 with 6
+#ifndef SKG_VOR_PAIRS
+#define SKG_VOR_PAIRS 6
+#endif
+
+// FP32: precomputed bisector planes, two per 32-byte load, a batch of loads in flight at once (one
+// batch holds most of the lists of a direction group)
 template<>
 SKG_D bool VoronoiStepper<float>::walk(const DevGrid& g, int& m, float& ds) {
-    if (qe < 0 && !done) { qb = g.vnoff[mr]; qe = g.vnoff[mr + 1]; }
+    const float4* const planes = group < 0 ? g.vplane : g.gplane;
+    const int4* const nexts = group < 0 ? g.vnext : g.gnext;
+    auto enter = [&]() {                       // the lists of cell mr
+        const int2 o = group < 0 ? __ldg(g.vpoff + mr) : __ldg(g.gpoff + (size_t)group * g.nsites + mr);
+        qb = o.x; qe = o.y;
+        nnb = g.vnoff[mr + 1] - g.vnoff[mr];
+    };
+    if (qe < 0 && !done) enter();
     while (!done) {
         if (++steps > g.max_steps) { done = true; return false; }
         int qbest = -1;
-        const int q0 = qb, q1 = qe;
-#if SKG_VOR_NODIV
         // the nearest wall ahead without a division per entry: a candidate s = num/den (den =
         // n.k > 0) is nearer than the best so far when num * bden < bnum * den
         float bnum = 1.f, bden = 0.f;
-#pragma unroll 4
-        for (int q = q0; q < q1; q++) {
-            const float4 pl = __ldg(g.vplane + q);
-            const float den = pl.x * kx + pl.y * ky + pl.z * kz;
-            const float num = pl.w - (pl.x * x + pl.y * y + pl.z * z);
-            if (den > 0.f && num > 0.f && num * bden < bnum * den) { bnum = num; bden = den; qbest = q; }
-        }
-        scanned += q1 - q0;
-        const float sq = (qbest >= 0) ? bnum / bden : FLT_MAX;
-#else
-        float sq = FLT_MAX;
-#pragma unroll 4
-        for (int q = q0; q < q1; q++) {
-            float4 pl = __ldg(g.vplane + q);
-            float ndotk = pl.x * kx + pl.y * ky + pl.z * kz;
-            scanned++;
-            if (ndotk > 0.f) {
-                float si = (pl.w - (pl.x * x + pl.y * y + pl.z * z)) / ndotk;
-                if (si > 0.f && si < sq) { sq = si; qbest = q; }
+#pragma unroll 1
+        for (int q = qb; q < qe; q += 2 * SKG_VOR_PAIRS) {
+            Eight e[SKG_VOR_PAIRS];
+#pragma unroll
+            for (int i = 0; i < SKG_VOR_PAIRS; i++) {
+                if (q + 2 * i < qe) e[i] = load32(planes + q + 2 * i);
+                else for (int c = 0; c < 8; c++) e[i].a[c] = 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 2 * SKG_VOR_PAIRS; i++) {
+                const float* pl = e[i >> 1].a + 4 * (i & 1);
+                const float den = vor_den(pl[0], pl[1], pl[2], kx, ky, kz);
+                const float num = pl[3] - (pl[0] * x + pl[1] * y + pl[2] * z);
+                if (den > 0.f && num > 0.f && num * bden < bnum * den) { bnum = num; bden = den; qbest = q + i; }
             }
         }
-#endif
+        scanned += nnb;
+        const float sq = (qbest >= 0) ? bnum / bden : FLT_MAX;
         if (qbest < 0) {
             x += kx * g.epsf; y += ky * g.epsf; z += kz * g.epsf;
             mr = voronoi_cell_index<float>(g, x, y, z);
             fallbacks++;
             if (mr < 0) done = true;
-            else { qb = g.vnoff[mr]; qe = g.vnoff[mr + 1]; }
+            else enter();
             continue;
         }
         m = mr;
         x += (sq + g.epsf) * kx; y += (sq + g.epsf) * ky; z += (sq + g.epsf) * kz;
-        const int4 e = __ldg(g.vnext + qbest);
-        mr = e.x; qb = e.y; qe = e.z;
+        const int4 e = __ldg(nexts + qbest);
+        mr = e.x; qb = e.y; qe = e.z; nnb = e.w;
         if (mr < 0) done = true;
         ds = (mr >= 0) ? sq + g.epsf : sq;   // the nudge is credited to this segment (exact total length)
         return true;
     }
     return false;
 }
+
+// does a stepper have lists of its own per peel-off direction?
+template<class St> struct HasGroups { static constexpr bool value = false; };
+template<> struct HasGroups<VoronoiStepper<float>> { static constexpr bool value = true; };
 
 // The cell of a start position strictly inside the box, as the FP32 walks' own search finds it
 // (-2: left to the walk).

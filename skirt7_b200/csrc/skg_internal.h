@@ -39,6 +39,14 @@ cudaError_t launch_emission_sources(const DevScene* dS, int nlambda, int ncells,
 size_t emission_scan_scratch_bytes(int ncells);
 cudaError_t launch_sum(const double* x, int64_t n, double* out, cudaStream_t s);
 cudaError_t launch_octant_records(const DevGrid& g, void* out, cudaStream_t s);   // out: 16 uint4 per cell
+// Voronoi lists per peel-off direction: padded counts per (group, cell) (cnt[ngroups * ncells] = 0), their
+// exclusive sums, then the lists at those offsets
+cudaError_t launch_group_counts(const DevGrid& g, const double* kx, const double* ky, const double* kz, int ngroups,
+                                int* cnt, cudaStream_t s);
+size_t offset_scan_scratch_bytes(int n);
+cudaError_t launch_offset_scan(const int* cnt, int* first, int n, void* scratch, size_t scratch_bytes, cudaStream_t s);
+cudaError_t launch_group_planes(const DevGrid& g, const double* kx, const double* ky, const double* kz, int ngroups,
+                                const int* first, void* planes, void* nexts, void* ranges, cudaStream_t s);
 cudaError_t launch_embed_density(const DevGrid& g, const float* rhof, cudaStream_t s);
 
 // skg_host.cpp

@@ -159,7 +159,7 @@ template<typename R> struct __align__(16) WalkJob {
     float kext1;                      // kappa_ext at its wavelength (one dust component), else -1
     int hint;                         // cell of the start, if known
     int out;                          // where its optical depth goes
-    int p, slot, ell;                 // packet, simulation, wavelength
+    int p, slot, ell;                 // packet, simulation (direction group from bit 8 on grids with lists per group), wavelength
 };
 
 // Counters of a wave's jobs and lists.

@@ -141,6 +141,10 @@ struct Req {
 // the remaining tables.
 int64_t footprint(const SceneCopy& s) {
     int64_t b = s.ncells * (int64_t)(12 * std::max(s.sc.ncomp, 1) + 96) + (int64_t)s.host_bytes() + (16 << 20);
+    // walk records: one per direction octant of a tree, the planes with their neighbours and the lists of
+    // up to four peel-off directions of a Voronoi grid
+    if (s.sc.grid.type == SKG_GRID_OCTREE || s.sc.grid.type == SKG_GRID_BINTREE) b += s.ncells * 256;
+    if (s.sc.grid.type == SKG_GRID_VORONOI) b += s.ncells * (int64_t)(32 * 18 + (s.instr.size() <= 4 ? 300 * (int64_t)s.instr.size() : 1200));
     for (const auto& in : s.instr) {
         int64_t nc = 1;
         if (in.type == SKG_INSTR_FRAME && in.stellar_comps) nc = 1 + std::max(s.sc.nstellar, 0);

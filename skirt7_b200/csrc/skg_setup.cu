@@ -241,6 +241,69 @@ cudaError_t launch_octant_records(const DevGrid& g, void* out, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// The planes ahead of a peel-off direction, per cell: n.k > 0, formed as the walk forms it.
+struct GroupDirs { float kx[4], ky[4], kz[4]; };
+static GroupDirs group_dirs(const double* kx, const double* ky, const double* kz, int n) {
+    GroupDirs d = {};
+    for (int q = 0; q < n && q < 4; q++) { d.kx[q] = (float)kx[q]; d.ky[q] = (float)ky[q]; d.kz[q] = (float)kz[q]; }
+    return d;
+}
+__global__ void group_counts_kernel(const DevGrid g, const GroupDirs d, int ngroups, int* cnt) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t > (int64_t)ngroups * g.nsites) return;
+    int c = 0;
+    if (t < (int64_t)ngroups * g.nsites) {
+        const int q = (int)(t / g.nsites), m = (int)(t - (int64_t)q * g.nsites);
+        const int2 o = g.vpoff[m];
+        for (int i = o.x; i < o.y; i++) {
+            const float4 p = g.vplane[i];
+            c += vor_den(p.x, p.y, p.z, d.kx[q], d.ky[q], d.kz[q]) > 0.f;
+        }
+    }
+    cnt[t] = (c + 1) & ~1;
+}
+__global__ void group_planes_kernel(const DevGrid g, const GroupDirs d, int ngroups, const int* __restrict__ first,
+                                    float4* planes, int4* nexts, int2* ranges) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (int64_t)ngroups * g.nsites) return;
+    const int q = (int)(t / g.nsites), m = (int)(t - (int64_t)q * g.nsites);
+    const int2 o = g.vpoff[m];
+    const int end = first[t + 1];
+    int at = first[t];
+    ranges[t] = make_int2(at, end);
+    for (int i = o.x; i < o.y; i++) {
+        const float4 p = g.vplane[i];
+        if (!(vor_den(p.x, p.y, p.z, d.kx[q], d.ky[q], d.kz[q]) > 0.f)) continue;
+        const int4 nx = g.vnext[i];
+        planes[at] = p;
+        const int64_t f = (int64_t)q * g.nsites + max(nx.x, 0);
+        nexts[at] = nx.x >= 0 ? make_int4(nx.x, first[f], first[f + 1], nx.w) : nx;
+        at++;
+    }
+    for (; at < end; at++) { planes[at] = make_float4(0.f, 0.f, 0.f, 0.f); nexts[at] = make_int4(-1, 0, 0, 0); }
+}
+cudaError_t launch_group_counts(const DevGrid& g, const double* kx, const double* ky, const double* kz, int ngroups,
+                                int* cnt, cudaStream_t s) {
+    const int64_t n = (int64_t)ngroups * g.nsites + 1;
+    group_counts_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(g, group_dirs(kx, ky, kz, ngroups), ngroups, cnt);
+    return cudaGetLastError();
+}
+size_t offset_scan_scratch_bytes(int n) {
+    size_t bytes = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, bytes, (const int*)nullptr, (int*)nullptr, n);
+    return bytes;
+}
+cudaError_t launch_offset_scan(const int* cnt, int* first, int n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+    return cub::DeviceScan::ExclusiveSum(scratch, scratch_bytes, cnt, first, n, s);
+}
+cudaError_t launch_group_planes(const DevGrid& g, const double* kx, const double* ky, const double* kz, int ngroups,
+                                const int* first, void* planes, void* nexts, void* ranges, cudaStream_t s) {
+    const int64_t n = (int64_t)ngroups * g.nsites;
+    group_planes_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(g, group_dirs(kx, ky, kz, ngroups), ngroups, first,
+                                                                    (float4*)planes, (int4*)nexts, (int2*)ranges);
+    return cudaGetLastError();
+}
+
 // Sum of a vector (absorbed-luminosity totals for the self-absorption convergence test).
 __global__ void sum_kernel(const double* __restrict__ x, int64_t n, double* out) {
     __shared__ double sh[256];

@@ -987,6 +987,7 @@ enum TravMode : int { TRAV_PATH = 1, TRAV_TAU = 2, TRAV_REWALK = 3 };
 // Resident blocks per SM of each instantiation.
 template<int MODE, template<typename> class Stepper> struct TravBlocks { static constexpr int value = SKG_TRAV_MIN_BLOCKS; };
 template<template<typename> class Stepper> struct TravBlocks<TRAV_PATH, Stepper> { static constexpr int value = SKG_PATH_MIN_BLOCKS; };
+template<> struct TravBlocks<TRAV_TAU, VoronoiStepper> { static constexpr int value = 3; };   // 12 planes in flight
 template<template<typename> class Stepper> struct TravBlocks<TRAV_REWALK, Stepper> { static constexpr int value = SKG_PATH_MIN_BLOCKS; };
 
 template<typename R, template<typename> class Stepper>
@@ -1086,6 +1087,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                     w.ell = K.ell; w.hint = K.pos_cell;
                     w.slot = ONE ? 0 : P.items[K.item].slot;
                     const DevScene& S = *s_scene[w.slot];
+                    if (HasGroups<Stepper<R>>::value && MODE == TRAV_TAU) w.slot |= grp << 8;
                     w.kext1 = (S.ncomp == 1) ? (float)S.kext[w.ell] : -1.f;
                     w.x = (R)K.x; w.y = (R)K.y; w.z = (R)K.z;
                     if (MODE != TRAV_TAU || grp == JOB_MAIN) { w.kx = (R)K.kx; w.ky = (R)K.ky; w.kz = (R)K.kz; }
@@ -1100,9 +1102,11 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                 const int r = used + __popc(want & ((1u << lane) - 1));
                 if (j < 0 && r < have) {
                     const WalkJob<R> w = mine[r];
-                    j = w.out; p = w.p; slot = w.slot; ell = w.ell; kext1 = w.kext1;
+                    j = w.out; p = w.p; slot = w.slot & 255; ell = w.ell; kext1 = w.kext1;
                     tau = 0;
                     const DevGrid& g = grid_of(slot);
+                    if constexpr (HasGroups<Stepper<R>>::value)
+                        st.group = (MODE == TRAV_TAU && (w.slot >> 8) != JOB_MAIN && g.gplane) ? w.slot >> 8 : -1;
                     // entry segments outside the grid (m = -1) carry no optical depth: only the
                     // re-walk, which measures length, takes them
                     if (MODE == TRAV_REWALK) {
@@ -1604,10 +1608,11 @@ static bool ckpt_grid(int grid_type) {
 // records come from L1 and L2, for the cost of the counting sort.  Worth it when the wave has enough
 // jobs to be dense and the records are more than what stays close anyway: phases of 2*10^7 packets on
 // a 3*10^6-leaf octree (96 MB of records) 306 against 293 ms, of 2*10^6 on 10^6 Voronoi cells (512 MB)
-// 262 against 254 ms; below these bounds the sort costs more than it gives (2.4*10^5 packets on a small octree
-// 4.1 against 4.7 ms; Cartesian densities are a few MB: a batch of 24 fit variants 53.5 against 56.2 ms).
+// 262 against 254 ms, of 10^6 on the octree 20.7 against 18.3, on
+// Voronoi cells 100 against 93, on a 10^6-leaf k-d tree 12.9 against 12.6; below these bounds the sort costs more than it gives
+// (2.4*10^5 packets on a small octree 4.1 against 4.7 ms, 6*10^5 on the k-d tree 9.4 against 9.6; Cartesian densities are a few MB: a batch of 24 fit variants 53.5 against 56.2 ms).
 static bool order_pays(int grid_type, size_t pool, size_t walk_bytes) {
-    return grid_type != SKG_GRID_CARTESIAN && pool >= ((size_t)3 << 19) && pool < ((size_t)1 << 28) && walk_bytes >= ((size_t)8 << 20);
+    return grid_type != SKG_GRID_CARTESIAN && pool >= ((size_t)3 << 18) && pool < ((size_t)1 << 28) && walk_bytes >= ((size_t)8 << 20);
 }
 
 cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes) {
