@@ -378,9 +378,9 @@ struct skg_ctx {
     std::vector<double> lambda, dlambda;
     // dust emission
     int nT = 0;
-    double *Tv = nullptr, *planckabs = nullptr, *labsbol = nullptr, *spectra = nullptr, *temperature = nullptr;
+    double *Tv = nullptr, *planckabs = nullptr, *planck_tab = nullptr, *temperature = nullptr;
     double *emit_Lv = nullptr, *emit_cdf = nullptr, *emit_Ltot = nullptr, *sumbuf = nullptr;
-    void* scan_scratch = nullptr; size_t scan_bytes = 0;
+    double* cdf_sums = nullptr;
     std::string error;
 };
 
@@ -672,14 +672,12 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
             ctx->nT = NT + 1;
             ctx->Tv = upload(A, Tv.data(), Tv.size(), s);
             ctx->planckabs = upload(A, pa.data(), pa.size(), s);
-            ctx->labsbol = zeros<double>(A, nc, s);
-            ctx->spectra = zeros<double>(A, (size_t)nc * nl, s);
+            ctx->planck_tab = zeros<double>(A, 3 * (size_t)nl, s);
             ctx->temperature = zeros<double>(A, nc, s);
             ctx->emit_Lv = zeros<double>(A, (size_t)nc * nl, s);
             ctx->emit_cdf = zeros<double>(A, (size_t)(nc + 1) * nl, s);
             ctx->emit_Ltot = zeros<double>(A, nl, s);
-            ctx->scan_bytes = emission_scan_scratch_bytes((int)nc);
-            ctx->scan_scratch = A.alloc<char>(ctx->scan_bytes);
+            ctx->cdf_sums = zeros<double>(A, (size_t)nl * emission_tiles((int)nc), s);
             H.emit_Lv = ctx->emit_Lv; H.emit_cdf = ctx->emit_cdf; H.emit_Ltot = ctx->emit_Ltot;
         }
         ctx->sumbuf = zeros<double>(A, 2, s);
@@ -1019,10 +1017,10 @@ int skg_calc_dust_emission(skg_ctx* ctx, double* temperature) {
         CK(cudaSetDevice(ctx->device));
         REQUIRE(ctx->emit_cdf != nullptr, "dust emission is not enabled for this scene");
         cudaStream_t s = ctx->stream;
-        CK(launch_dust_emission(ctx->grid, ctx->ds, ctx->Tv, ctx->planckabs, ctx->nT, ctx->labsbol, ctx->spectra,
+        CK(launch_dust_emission(ctx->grid, ctx->ds, ctx->Tv, ctx->planckabs, ctx->nT, ctx->planck_tab, ctx->emit_Lv,
                                 ctx->temperature, s));
-        CK(launch_emission_sources(ctx->ds, ctx->nlambda, (int)ctx->ncells, ctx->labsbol, ctx->spectra, ctx->emit_Lv,
-                                   ctx->emit_cdf, ctx->emit_Ltot, ctx->scan_scratch, ctx->scan_bytes, s));
+        CK(launch_emission_sources(ctx->nlambda, (int)ctx->ncells, ctx->emit_Lv, ctx->emit_cdf, ctx->emit_Ltot,
+                                   ctx->cdf_sums, s));
         if (temperature) CK(cudaMemcpyAsync(temperature, ctx->temperature, ctx->ncells * sizeof(double), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         return SKG_OK;

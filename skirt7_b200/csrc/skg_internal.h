@@ -30,13 +30,11 @@ cudaError_t launch_node_mass(const void* dgeoms, const double* norms, int ncomp,
                              int nnodes, int nsamples, uint64_t seed, uint64_t node_offset,
                              double* mass, double* rhomin, double* rhomax, cudaStream_t s);
 cudaError_t launch_dust_emission(const DevGrid& g, const DevScene* dS, const double* Tv,
-                                 const double* planckabs, int nT, double* labsbol, double* spectra,
+                                 const double* planckabs, int nT, double* tab /* [3 nlambda] */, double* emit_Lv,
                                  double* temperature, cudaStream_t s);
-cudaError_t launch_emission_sources(const DevScene* dS, int nlambda, int ncells, const double* labsbol,
-                                    const double* spectra, double* emit_Lv, double* emit_cdf,
-                                    double* emit_Ltot, void* scratch, size_t scratch_bytes,
-                                    cudaStream_t s);
-size_t emission_scan_scratch_bytes(int ncells);
+size_t emission_tiles(int ncells);
+cudaError_t launch_emission_sources(int nlambda, int ncells, const double* emit_Lv, double* emit_cdf,
+                                    double* emit_Ltot, double* sums /* [nlambda][emission_tiles] */, cudaStream_t s);
 cudaError_t launch_sum(const double* x, int64_t n, double* out, cudaStream_t s);
 cudaError_t launch_octant_records(const DevGrid& g, void* out, cudaStream_t s);   // out: 16 uint4 per cell
 // Voronoi lists per peel-off direction: padded counts per (group, cell) (cnt[ngroups * ncells] = 0), their

@@ -84,10 +84,19 @@ cudaError_t launch_node_mass(const void* dgeoms, const double* norms, int ncomp,
 //   L_ell = kappa_abs(ell) B_ell(T) dlambda, normalised to unit sum     GreyBodyDustEmissivity.cpp:21-45,
 //                                                                       DustLib.cpp:135-148
 // The mix's 1/mu factors cancel between the Planck table and the sum, as in the reference.
-SKG_D double planck_B(double lambda, double T) {   // PlanckFunction.cpp:24-33
+
+// Per wavelength, from the mix: tab[ell] = kappa_abs 2 h c^2 / lambda^5 dlambda and tab[nl + ell] =
+// h c / (lambda k), so that L_ell = tab[ell] / (exp(tab[nl + ell] / T) - 1) (PlanckFunction.cpp:24-33); and
+// tab[2 nl + ell] = 1 where the wavelength counts for the absorbed energy, 0 where J is not finite.
+__global__ void planck_table_kernel(const DevScene* __restrict__ Sp, double* tab) {
+    const DevScene& S = *Sp;
     const double h = 6.62606957e-34, c = 2.99792458e8, k = 1.3806488e-23;
-    double x = h * c / (lambda * k * T);
-    return 2.0 * h * c * c / pow(lambda, 5) / (exp(x) - 1.0);
+    for (int ell = blockIdx.x * blockDim.x + threadIdx.x; ell < S.nlambda; ell += gridDim.x * blockDim.x) {
+        const double lambda = S.lambda[ell], kabs = S.kext[ell] * (1.0 - S.albedo[ell]);
+        tab[ell] = kabs * (2.0 * h * c * c / pow(lambda, 5)) * S.dlambda[ell];
+        tab[S.nlambda + ell] = h * c / (lambda * k);
+        tab[2 * S.nlambda + ell] = (kabs > 0.0 && S.dlambda[ell] != 0.0) ? 1.0 : 0.0;
+    }
 }
 
 SKG_D double cell_volume(const DevGrid& g, int m) {
@@ -101,92 +110,145 @@ SKG_D double cell_volume(const DevGrid& g, int m) {
     return (b[3] - b[0]) * (b[4] - b[1]) * (b[5] - b[2]);
 }
 
-__global__ void dust_emission_kernel(const DevGrid g, const DevScene* __restrict__ Sp, const double* __restrict__ Tv,
-                                     const double* __restrict__ planckabs, int nT, double* labsbol,
-                                     double* spectra, double* temperature) {
+// Temperature of every cell and its luminosity per wavelength, emit_Lv[ell][m] = Labsbol[m] L_ell
+// (PanMonteCarloSimulation.cpp:197-203).  One thread per cell; the spectrum is formed twice, once for
+// its sum and once for the result: with the wavelengths' constants in a table an entry costs an exp and a division, less than
+// writing the spectra out and reading them back twice (a pow and three divisions per entry
+// before: 4.2 ms per call for 10^6 cells and 40 wavelengths, with the sums below).
+__global__ void __launch_bounds__(128) dust_emission_kernel(const DevGrid g, const DevScene* __restrict__ Sp,
+                                                            const double* __restrict__ Tv,
+                                                            const double* __restrict__ planckabs, int nT,
+                                                            const double* __restrict__ tab, double* __restrict__ emit_Lv,
+                                                            double* temperature) {
     const DevScene& S = *Sp;
-    int m = blockIdx.x * blockDim.x + threadIdx.x;
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= S.ncells) return;
     const int nl = S.nlambda;
-    double lb = 0, pa = 0;
-    double fac = 4.0 * M_PI * cell_volume(g, m);
-    double rho = S.rho[m];
+    const size_t nc = (size_t)S.ncells;
+    const double* const ls = S.labs_stel + m;
+    const double* const ld = S.labs_dust + m;
+    double lb = 0, la = 0;
+#pragma unroll 4
     for (int ell = 0; ell < nl; ell++) {
-        double la = S.labs_stel[(size_t)ell * S.ncells + m] + S.labs_dust[(size_t)ell * S.ncells + m];
-        lb += la;
-        double kabs = S.kext[ell] * (1.0 - S.albedo[ell]);
-        double J = la / (kabs * rho * fac) / S.dlambda[ell];
-        if (!isfinite(J)) J = 0.0;
-        pa += kabs * J * S.dlambda[ell];
+        const double v = ls[ell * nc] + ld[ell * nc];
+        lb += v;
+        la += v * __ldg(tab + 2 * nl + ell);
     }
-    labsbol[m] = lb;
-    int p = dlocate_clip(planckabs, nT, pa);
-    double T = Tv[p] + ((pa - planckabs[p]) / (planckabs[p + 1] - planckabs[p])) * (Tv[p + 1] - Tv[p]);
+    const double q = S.rho[m] * (4.0 * M_PI * cell_volume(g, m));
+    double pa = la / q;                            // sum of kappa_abs J dlambda
+    if (!isfinite(pa)) pa = 0.0;
+    const int p = dlocate_clip(planckabs, nT, pa);
+    const double T = Tv[p] + ((pa - planckabs[p]) / (planckabs[p + 1] - planckabs[p])) * (Tv[p + 1] - Tv[p]);
     if (temperature) temperature[m] = T;
     double total = 0;
-    const size_t nc = (size_t)S.ncells;
-    for (int ell = 0; ell < nl; ell++) {
-        double kabs = S.kext[ell] * (1.0 - S.albedo[ell]);
-        double v = (T > 0) ? kabs * planck_B(S.lambda[ell], T) * S.dlambda[ell] : 0.0;
-        spectra[ell * nc + m] = v; total += v;
-    }
-    if (total > 0) for (int ell = 0; ell < nl; ell++) spectra[ell * nc + m] /= total;
+    const double invT = 1.0 / T;
+    if (T > 0)
+        for (int ell = 0; ell < nl; ell++) total += __ldg(tab + ell) / (exp(__ldg(tab + nl + ell) * invT) - 1.0);
+    const double f = (total > 0 && lb > 0.0) ? lb / total : 0.0;
+    for (int ell = 0; ell < nl; ell++)
+        emit_Lv[ell * nc + m] = f > 0 ? f * (__ldg(tab + ell) / (exp(__ldg(tab + nl + ell) * invT) - 1.0)) : 0.0;
 }
 
 cudaError_t launch_dust_emission(const DevGrid& g, const DevScene* dS, const double* Tv, const double* planckabs,
-                                 int nT, double* labsbol, double* spectra, double* temperature, cudaStream_t s) {
+                                 int nT, double* tab, double* emit_Lv, double* temperature, cudaStream_t s) {
     int th = 128;
     int bl = (g.ncells + th - 1) / th;
     if (bl == 0) return cudaSuccess;
-    dust_emission_kernel<<<bl, th, 0, s>>>(g, dS, Tv, planckabs, nT, labsbol, spectra, temperature);
+    planck_table_kernel<<<1, 128, 0, s>>>(dS, tab);
+    dust_emission_kernel<<<bl, th, 0, s>>>(g, dS, Tv, planckabs, nT, tab, emit_Lv, temperature);
     return cudaGetLastError();
 }
 
-// emit_Lv[ell][m] = Labsbol[m] * spectrum[ell][m]   (PanMonteCarloSimulation.cpp:197-203)
-__global__ void emission_weights_kernel(int nl, int nc, const double* __restrict__ labsbol,
-                                        const double* __restrict__ spectra, double* emit_Lv) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)nl * nc) return;
-    int ell = (int)(t / nc), m = (int)(t - (int64_t)ell * nc);
-    double lb = labsbol[m];
-    emit_Lv[t] = (lb > 0.0) ? lb * spectra[t] : 0.0;
+// The cumulative cell luminosities, normalised per wavelength (NR::cdf, NR.hpp:388-394: P_0 = 0,
+// P_{i+1} = sum_{j<=i} p_j / sum p): sums of tiles of cells, their offsets per wavelength, then the
+// tiles again with their offset and the normalisation -- three launches for all wavelengths, the
+// luminosities read twice and the result written once (a library scan per wavelength and a pass to
+// normalise before: 80 launches for 40 wavelengths).
+constexpr int CDF_TILE = 2048;                     // 8 warps of 8 rows of 32 cells
+SKG_D double warp_incl(double v, int lane) {
+    for (int d = 1; d < 32; d <<= 1) { const double t = __shfl_up_sync(0xffffffffu, v, d); if (lane >= d) v += t; }
+    return v;
 }
-// NR::cdf normalisation (NR.hpp:388-394): P_0 = 0, P_{i+1} = sum_{j<=i} p_j / sum p
-__global__ void cdf_totals_kernel(int nl, int nc, double* cdf, double* Ltot) {
-    int ell = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ell >= nl) return;
-    Ltot[ell] = cdf[(size_t)ell * (nc + 1) + nc];
-    cdf[(size_t)ell * (nc + 1)] = 0.0;
-}
-__global__ void cdf_normalise_kernel(int nl, int nc, double* cdf, const double* __restrict__ Ltot) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)nl * (nc + 1)) return;
-    int ell = (int)(t / (nc + 1));
-    double tot = Ltot[ell];
-    if (t - (int64_t)ell * (nc + 1) == 0) return;
-    cdf[t] = (tot > 0) ? cdf[t] / tot : 0.0;
-}
-
-size_t emission_scan_scratch_bytes(int ncells) {
-    size_t bytes = 0;
-    cub::DeviceScan::InclusiveSum(nullptr, bytes, (const double*)nullptr, (double*)nullptr, ncells);
-    return bytes;
-}
-
-cudaError_t launch_emission_sources(const DevScene*, int nl, int nc, const double* labsbol, const double* spectra,
-                                    double* emit_Lv, double* emit_cdf, double* emit_Ltot, void* scratch,
-                                    size_t scratch_bytes, cudaStream_t s) {
-    int64_t tot = (int64_t)nl * nc;
-    emission_weights_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(nl, nc, labsbol, spectra, emit_Lv);
-    for (int ell = 0; ell < nl; ell++) {
-        size_t bytes = scratch_bytes;
-        cudaError_t e = cub::DeviceScan::InclusiveSum(scratch, bytes, emit_Lv + (size_t)ell * nc,
-                                                      emit_cdf + (size_t)ell * (nc + 1) + 1, nc, s);
-        if (e != cudaSuccess) return e;
+__global__ void __launch_bounds__(256) cdf_sums_kernel(int nc, const double* __restrict__ Lv, double* sums) {
+    __shared__ double ws[8];
+    const double* x = Lv + (size_t)blockIdx.y * nc;
+    double v = 0;
+    for (int i = 0; i < CDF_TILE / 256; i++) {
+        const int64_t m = (int64_t)blockIdx.x * CDF_TILE + i * 256 + threadIdx.x;
+        if (m < nc) v += x[m];
     }
-    cdf_totals_kernel<<<(nl + 127) / 128, 128, 0, s>>>(nl, nc, emit_cdf, emit_Ltot);
-    int64_t tc = (int64_t)nl * (nc + 1);
-    cdf_normalise_kernel<<<(unsigned)((tc + 255) / 256), 256, 0, s>>>(nl, nc, emit_cdf, emit_Ltot);
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) v += ws[w];
+        sums[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = v;
+    }
+}
+// one block per wavelength: the tiles' sums become their offsets
+__global__ void __launch_bounds__(256) cdf_offsets_kernel(int ntiles, double* sums, double* Ltot) {
+    __shared__ double ws[8], carry;
+    double* x = sums + (size_t)blockIdx.x * ntiles;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) carry = 0;
+    for (int b = 0; b < ntiles; b += 256) {
+        const int i = b + threadIdx.x;
+        const double v = i < ntiles ? x[i] : 0.0;
+        const double inc = warp_incl(v, lane);
+        if (lane == 31) ws[warp] = inc;
+        __syncthreads();
+        double before = carry;
+        for (int w = 0; w < warp; w++) before += ws[w];
+        if (i < ntiles) x[i] = before + (inc - v);
+        __syncthreads();
+        if (threadIdx.x == 255) carry = before + inc;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) Ltot[blockIdx.x] = carry;
+}
+__global__ void __launch_bounds__(256) cdf_kernel(int nc, const double* __restrict__ Lv, const double* __restrict__ offsets,
+                                                  const double* __restrict__ Ltot, double* __restrict__ cdf) {
+    __shared__ double ws[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ell = blockIdx.y;
+    const double* x = Lv + (size_t)ell * nc;
+    double* out = cdf + (size_t)ell * (nc + 1);
+    const int64_t m0 = (int64_t)blockIdx.x * CDF_TILE + warp * (CDF_TILE / 8) + lane;
+    double v[8];
+    double sum = 0;
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const int64_t m = m0 + 32 * r;
+        v[r] = sum + warp_incl(m < nc ? x[m] : 0.0, lane);
+        sum = __shfl_sync(0xffffffffu, v[r], 31);
+    }
+    if (lane == 0) ws[warp] = sum;
+    __syncthreads();
+    double before = offsets[(size_t)ell * gridDim.x + blockIdx.x];
+    for (int w = 0; w < warp; w++) before += ws[w];
+    const double tot = Ltot[ell];
+    const double inv = tot > 0 ? 1.0 / tot : 0.0;
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const int64_t m = m0 + 32 * r;
+        if (m < nc) out[m + 1] = (before + v[r]) * inv;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = 0.0;
+}
+
+size_t emission_tiles(int nc) { return ((size_t)nc + CDF_TILE - 1) / CDF_TILE; }
+
+cudaError_t launch_emission_sources(int nl, int nc, const double* emit_Lv, double* emit_cdf, double* emit_Ltot,
+                                    double* sums, cudaStream_t s) {
+    if (nc <= 0 || nl <= 0) return cudaSuccess;
+    const int tiles = (int)emission_tiles(nc);
+    for (int l0 = 0; l0 < nl; l0 += 65535) {
+        const int n = std::min(nl - l0, 65535);
+        const double* x = emit_Lv + (size_t)l0 * nc;
+        double* t = sums + (size_t)l0 * tiles;
+        cdf_sums_kernel<<<dim3(tiles, n), 256, 0, s>>>(nc, x, t);
+        cdf_offsets_kernel<<<n, 256, 0, s>>>(tiles, t, emit_Ltot + l0);
+        cdf_kernel<<<dim3(tiles, n), 256, 0, s>>>(nc, x, t, emit_Ltot + l0, emit_cdf + (size_t)l0 * (nc + 1));
+    }
     return cudaGetLastError();
 }
 

@@ -173,7 +173,11 @@ class Context:
         self._ck(self.lib.skg_read_density(self.h, rho.ctypes.data_as(A.dp)))
         return rho[: nd * self.ncells].reshape(nd, self.ncells)
 
-    def calc_dust_emission(self):
+    def calc_dust_emission(self, temperature=True):
+        """skg_calc_dust_emission; returns the cells' temperatures (None when not asked for)."""
+        if not temperature:
+            self._ck(self.lib.skg_calc_dust_emission(self.h, None))
+            return None
         T = np.zeros(self.ncells)
         self._ck(self.lib.skg_calc_dust_emission(self.h, T.ctypes.data_as(A.dp)))
         return T
@@ -394,7 +398,7 @@ class MonteCarloSimulation:
             ncmax = self.cycles if self.cycles else 100
             cycle, conv = 1, False
             while cycle <= ncmax and (not conv or self.cycles):
-                ctx.calc_dust_emission()
+                ctx.calc_dust_emission(temperature=False)
                 ctx.reset_dust_absorption()
                 ms = self._run(A.PHASE_DUST_SELFABS, self.packages * factors[stage], self.seed + 1000 * stage + cycle)
                 _, ldust = ctx.absorbed_totals()
@@ -407,7 +411,7 @@ class MonteCarloSimulation:
 
     def rundustemission(self):
         ctx = self.ctx
-        ctx.calc_dust_emission()
+        ctx.calc_dust_emission(temperature=False)
         self.phase_ms["dustemission"] = self._run(A.PHASE_DUST_EMISSION, self.packages * self.emissionBoost,
                                                   self.seed + 7777)
 
