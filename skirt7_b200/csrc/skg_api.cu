@@ -978,21 +978,28 @@ int skg_read_absorption(skg_ctx* ctx, double* labs_stellar, double* labs_dust) {
     if (rc) return rc;
     try {
         const size_t nc = (size_t)ctx->ncells, nl = (size_t)ctx->nlambda, n = nc * nl;
-        // the device tables are wavelength-major ([ell][m]); the caller gets [m][ell]
-        std::vector<double> t;
+        // the device tables are wavelength-major ([ell][m]); the caller gets [m][ell], transposed on the
+        // device in pieces of 64 MB (on the host: 20 ms of a 40 ms pass for 10^6 cells and 10 wavelengths)
+        cudaStream_t s = ctx->stream;
+        Allocs T;
+        T.stream = s;
+        const size_t piece = std::max<size_t>(32, std::min(nc, ((size_t)8 << 20) / nl));
+        double* buf = nullptr;
         auto read = [&](const double* dev, double* out) {
             if (!out) return;
             if (!dev) { std::memset(out, 0, n * sizeof(double)); return; }
-            t.resize(n);
-            CK(cudaMemcpy(t.data(), dev, n * sizeof(double), cudaMemcpyDeviceToHost));
-            const size_t B = 64;                        // cache blocks of the transpose
-            for (size_t m0 = 0; m0 < nc; m0 += B)
-                for (size_t e0 = 0; e0 < nl; e0 += B)
-                    for (size_t m = m0; m < std::min(nc, m0 + B); m++)
-                        for (size_t e = e0; e < std::min(nl, e0 + B); e++) out[m * nl + e] = t[e * nc + m];
+            if (nl == 1) { CK(cudaMemcpyAsync(out, dev, n * sizeof(double), cudaMemcpyDeviceToHost, s)); return; }
+            if (!buf) buf = T.alloc<double>(piece * nl);
+            if (!buf) throw Failure{SKG_ERR_OOM, "device allocation failed"};
+            for (size_t m0 = 0; m0 < nc; m0 += piece) {
+                const size_t k = std::min(piece, nc - m0);
+                CK(launch_cell_major(dev, (int64_t)nc, (int)nl, (int64_t)m0, (int64_t)k, buf, s));
+                CK(cudaMemcpyAsync(out + m0 * nl, buf, k * nl * sizeof(double), cudaMemcpyDeviceToHost, s));
+            }
         };
         read(ctx->hs.labs_stel, labs_stellar);
         read(ctx->hs.labs_dust, labs_dust);
+        CK(cudaStreamSynchronize(s));
         return SKG_OK;
     } catch (const Failure& f) { return fail(ctx, f); }
 }

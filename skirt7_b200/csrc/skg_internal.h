@@ -35,6 +35,7 @@ cudaError_t launch_dust_emission(const DevGrid& g, const DevScene* dS, const dou
 size_t emission_tiles(int ncells);
 cudaError_t launch_emission_sources(int nlambda, int ncells, const double* emit_Lv, double* emit_cdf,
                                     double* emit_Ltot, double* sums /* [nlambda][emission_tiles] */, cudaStream_t s);
+cudaError_t launch_cell_major(const double* in, int64_t nc, int nl, int64_t m0, int64_t n, double* out, cudaStream_t s);
 cudaError_t launch_sum(const double* x, int64_t n, double* out, cudaStream_t s);
 cudaError_t launch_octant_records(const DevGrid& g, void* out, cudaStream_t s);   // out: 16 uint4 per cell
 // Voronoi lists per peel-off direction: padded counts per (group, cell) (cnt[ngroups * ncells] = 0), their

@@ -366,6 +366,28 @@ cudaError_t launch_group_planes(const DevGrid& g, const double* kx, const double
     return cudaGetLastError();
 }
 
+// out[m - m0][ell] = in[ell][m] for the cells m0 .. m0 + n - 1: tiles of 32 cells x 32 wavelengths through
+// shared memory, both sides coalesced.
+__global__ void __launch_bounds__(256) cell_major_kernel(const double* __restrict__ in, int64_t nc, int nl, int64_t m0,
+                                                         int64_t n, double* __restrict__ out) {
+    __shared__ double t[32][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int64_t c0 = (int64_t)blockIdx.x * 32;
+    for (int e0 = 0; e0 < nl; e0 += 32) {
+        for (int r = y; r < 32; r += 8)
+            if (e0 + r < nl && c0 + x < n) t[r][x] = in[(size_t)(e0 + r) * nc + m0 + c0 + x];
+        __syncthreads();
+        for (int r = y; r < 32; r += 8)
+            if (e0 + x < nl && c0 + r < n) out[(size_t)(c0 + r) * nl + e0 + x] = t[x][r];
+        __syncthreads();
+    }
+}
+cudaError_t launch_cell_major(const double* in, int64_t nc, int nl, int64_t m0, int64_t n, double* out, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    cell_major_kernel<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(in, nc, nl, m0, n, out);
+    return cudaGetLastError();
+}
+
 // Sum of a vector (absorbed-luminosity totals for the self-absorption convergence test).
 __global__ void sum_kernel(const double* __restrict__ x, int64_t n, double* out) {
     __shared__ double sh[256];

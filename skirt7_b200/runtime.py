@@ -37,6 +37,7 @@ class Context:
         nc, nb = C.c_int64(), C.c_int64()
         self.lib.skg_ctx_info(self.h, C.byref(nc), C.byref(nb))
         self.ncells, self.device_bytes = nc.value, nb.value
+        self.dust_tallied = False         # may the dust absorption table hold anything but zeros?
 
     def close(self):
         if self.h:
@@ -104,6 +105,7 @@ class Context:
         ells = np.ascontiguousarray(ells, dtype=np.int32)
         opts = A.RunOpts(precision, max_steps, max_scatt, blocks, refill, 1, pool)
         count = npp if count is None else count
+        self.dust_tallied = self.dust_tallied or phase == A.PHASE_DUST_SELFABS
         self._ck(self.lib.skg_run_phase(self.h, phase, ells.ctypes.data_as(A.i32p), len(ells), int(npp), int(first),
                                         int(count), int(seed), C.byref(opts), stream))
 
@@ -123,6 +125,7 @@ class Context:
 
     def reset_tallies(self):
         self._ck(self.lib.skg_reset_tallies(self.h))
+        self.dust_tallied = False
 
     def read_instrument(self, i, out=None):
         """(cube, sed): cube shaped [components, nlambda, nyp, nxp] (None for SED instruments),
@@ -155,9 +158,10 @@ class Context:
         self._ck(self.lib.skg_read_instrument_device(self.h, i, d_cube, d_sed, stream))
 
     def read_absorption(self):
-        ls = np.zeros(self.ncells * self.nlambda)
+        ls = np.empty(self.ncells * self.nlambda)
         ld = np.zeros(self.ncells * self.nlambda)
-        self._ck(self.lib.skg_read_absorption(self.h, ls.ctypes.data_as(A.dp), ld.ctypes.data_as(A.dp)))
+        self._ck(self.lib.skg_read_absorption(self.h, ls.ctypes.data_as(A.dp),
+                                              ld.ctypes.data_as(A.dp) if self.dust_tallied else None))
         return ls.reshape(self.ncells, self.nlambda), ld.reshape(self.ncells, self.nlambda)
 
     def counters(self):
@@ -189,6 +193,7 @@ class Context:
 
     def reset_dust_absorption(self):
         self._ck(self.lib.skg_reset_dust_absorption(self.h))
+        self.dust_tallied = False
 
 
 class Batch:
@@ -209,6 +214,7 @@ class Batch:
         for i, (ctx, ells, npp, first, count, seed) in enumerate(slices):
             e = np.ascontiguousarray(ells, dtype=np.int32)
             keep.append(e)
+            ctx.dust_tallied = ctx.dust_tallied or phase == A.PHASE_DUST_SELFABS
             arr[i] = A.Work(ctx.h.value, e.ctypes.data_as(A.i32p), len(e), int(npp), int(first), int(count), int(seed))
         opts = A.RunOpts(precision, 0, max_scatt, 0, refill, 1, pool)
         A.check(self.lib.skg_batch_run(self.h, phase, arr, n, C.byref(opts), A.BATCH_GRAPH if graph else 0, stream))
