@@ -147,9 +147,8 @@ struct __align__(64) Packet {
     int int_cell;                     // cell of the interaction point (-1 unknown)
     unsigned rngc;                    // next Philox block of the packet's stream
     int flags;                        // bit 0 stellar origin, bit 1 the pending peel-offs follow a scattering
-    int peel_j0, peel_n;              // this packet's peel-off jobs of the last wave
     int nck;                          // checkpoints of the path walk
-    int pad;
+    int pad[3];
 };
 static_assert(sizeof(Packet) == 128, "packet record is two 64-byte lines");
 
@@ -166,8 +165,7 @@ template<typename R> struct __align__(16) WalkJob {
 enum JobCount : int {
     J_PATH = 0,                       // path jobs
     J_PEEL,                           // peel-off jobs
-    J_BUSY,                           // packets with jobs
-    J_FREE, J_INT,                    // records on the free list, on the interaction list
+    J_FREE, J_INT,                    // records on the wave's free list, on its interaction list
     J_REWALK,                         // packets on the re-walk list
     J_TAKEN_PATH, J_TAKEN_TAU, J_TAKEN_REWALK,   // jobs taken by each walk
     J_N = 16
@@ -184,15 +182,12 @@ struct WaveParams {
     double* jtau;                     // peel-off optical depth
     double* jL;                       // peel-off luminosity
     unsigned* jcount;                 // counters of this wave (JobCount)
-    // the previous wave's jobs (peel-off detection)
-    const int2* pjobs;
-    const double* pjtau;
-    const double* pjL;
+    unsigned* jnext;                  // the next wave's counters (J_FREE and J_INT are counted by this wave)
     unsigned* last_busy;              // highest wave index that had jobs
-    int* freelist;                    // records the event pass freed (J_FREE)
-    int* intlist;                     // records it found at their interaction point (J_INT)
-    int2* rlist;                      // the paths that interact: (packet, place in walk order) (J_REWALK;
-                                      // the memory of the lists above, which the launch pass has consumed)
+    const int* freelist;              // records that take a new packet (J_FREE; wave 0: all)
+    const int* intlist;               // records at their interaction point (J_INT)
+    int *freenext, *intnext;          // the next wave's
+    int2* rlist;                      // the paths that interact: (packet, place in walk order) (J_REWALK)
     int tail_lanes;                   // tail pass: packets to a warp
     int path_tau;                     // the path jobs need the optical depth alone (walked with the peel-offs)
     float4* ckpt;                     // per packet record: checkpoints of its path walk

@@ -10,25 +10,26 @@
 //
 // is cut at its traversals.  The packets in flight sit in a pool of 128-byte records.  Each wave
 // runs these kernels:
-//   event_kernel  one thread per record: detects the peel-offs walked in the previous wave and
-//                 lists the packets at their interaction point and the free records;
-//   launch_kernel one thread per listed record: moves a packet to its interaction point, writes
-//                 its scattering peel-offs and scatters it, or launches a new packet into a free
-//                 record; then appends the packet's next traversals to the wave's job list (one
-//                 peel-off job per direction group and one path job);
-//   trav_kernel   persistent, launched twice (the path jobs, then the peel-off jobs in a lean
-//                 instantiation); each lane takes jobs one after another and walks them:
-//                 peel-off  accumulates the optical depth towards an observer
-//                           (DustSystem::opticaldepth, DustSystem.cpp:960-976);
-//                 path      streams kappa*rho*ds into the FP64 cumulative optical depth and the
-//                           per-cell absorption tallies (simulateescapeandabsorption, :432-509),
-//                           applies the escape fraction and the termination test, samples the
-//                           interaction optical depth (simulatepropagation, :513-531) and re-walks
-//                           the path to the segment where the cumulative optical depth passes it,
-//                           interpolating inside it (DustGridPath::pathlength, DustGridPath.cpp:162-173).
-// The traversal kernel holds nothing but the walk, so it keeps few registers, no local memory and
-// a small instruction footprint; the divergent event code runs once per packet per wave in a
-// kernel of its own.  Instruments seen from the same direction share one peel-off traversal
+//   launch_kernel   one thread per packet at its interaction point, then per free record: moves the
+//                   packet there and scatters it, or launches a new packet; then puts the packet's next
+//                   traversals on the wave's lists (one peel-off job per direction group, one path job);
+//   order_kernel    (with its bin kernels, on large waves) the jobs in spatial order;
+//   trav_kernel     persistent; each lane takes jobs one after another and walks them, in an
+//                   instantiation per kind of walk:
+//                   optical depth towards an observer (DustSystem::opticaldepth,
+//                   DustSystem.cpp:960-976) or along a path without absorption;
+//                   path with absorption: streams kappa*rho*ds into the FP64 cumulative optical depth
+//                   and the per-cell tallies (simulateescapeandabsorption, :432-509);
+//                   re-walk of a path to the segment where the cumulative optical depth passes the
+//                   interaction optical depth, interpolating inside it (DustGridPath::pathlength,
+//                   DustGridPath.cpp:162-173);
+//   path_end_kernel between path and re-walk: escape fraction, termination test, sampling of the
+//                   interaction optical depth (simulatepropagation, :513-531); lists the next wave's
+//                   interacting packets and free records;
+//   detect_kernel   one thread per peel-off: the instruments' tallies.
+// The traversal kernels hold nothing but the walk, so they keep few registers, no local memory and
+// a small instruction footprint; the divergent event code runs once per packet per wave in kernels
+// of its own.  Instruments seen from the same direction share one peel-off traversal
 // (identical optical depth; the reference recomputes it per instrument).
 #include "skg_scene.cuh"
 #include "skg_internal.h"
@@ -59,24 +60,6 @@ namespace skg {
 #ifndef SKG_PDL
 #define SKG_PDL 1
 #endif
-// the event pass at 4 blocks of 256 per SM (64 registers, spilling part of the packet record):
-// its divergent, latency-bound code gains more from the warps than it loses to the spills
-// (octree disk, 10^7 packets: 34.6 ms against 45.2 ms at 2 blocks and 126 registers)
-// packets at their interaction point and free records are scattered and relaunched by a pass of
-// their own after the event pass, every lane of its warps doing the same work (octree disk, 10^7
-// packets: phase 177.7 against 194.4 ms in one event pass; Cartesian 87.0 against 90.7 ms)
-#ifndef SKG_LAUNCH_KERNEL
-#define SKG_LAUNCH_KERNEL 1
-#endif
-#ifndef SKG_EVENT_MIN_BLOCKS
-#define SKG_EVENT_MIN_BLOCKS 4
-#endif
-// threads per event-pass block: a block's slot on an SM is held until its slowest record is done,
-// so small blocks free slots sooner (octree disk, 10^7 packets: event pass 29.5 ms with 64 threads,
-// 32.4 with 128, 34.6 with 256)
-#ifndef SKG_EVENT_THREADS
-#define SKG_EVENT_THREADS 64
-#endif
 // a lane whose job ended takes the next one when this many lanes of its warp (or all of them) wait for
 // one.  With the job records staged by the warp a start costs little: 4, 8 and 12 lanes take the octree
 // disk's traversal pass 166.7, 162.3 and 161.5 ms (2*10^7 packets), the fit-variant batch 43.8, 43.3
@@ -90,20 +73,6 @@ namespace skg {
 // interaction optical depth (at most one stride of cell steps) instead of at the path's start
 #ifndef SKG_CKPT
 #define SKG_CKPT 1
-#endif
-// the scatter-and-launch pass's grid: the blocks resident at once (1), or 16 per SM (0);
-// event + launch passes of a 10^7-packet octree-disk phase 13.3 against 14.4 ms
-#ifndef SKG_LAUNCH_OCC
-#define SKG_LAUNCH_OCC 1
-#endif
-// the event pass's grid for pools of at most this many records of a Cartesian grid: the blocks resident at once,
-// striding over the pool (the per-block counter and SED flushes then happen once per resident
-// block); larger pools: one thread per record.  Event pass of a 10^7-packet phase, pool 2^21:
-// Cartesian disk 15.7 against 16.8 ms, a batch of 24 fit variants 560.7 against 566.6 ms (whole
-// batch); pool 2^23 (2·10^6 packets per wavelength): octree disk 156 against 139 ms, k-d tree disk
-// 190 against 188 ms -- so the stride only up to 2^21
-#ifndef SKG_EVENT_STRIDE_POOL
-#define SKG_EVENT_STRIDE_POOL (1 << 21)
 #endif
 // cell steps a lane takes per pass of the traversal loop (the warp's refill vote runs once per
 // pass): optical-depth and re-walk kernels, path kernel.  Octree disk, 2*10^7 packets, traversal pass
@@ -231,8 +200,7 @@ __device__ __forceinline__
 __device__ __noinline__
 #endif
 int detect_group(const DevScene& S, int grp, int ell, double Lpeel, double tau,
-                                         int nscatt_peel, bool stellar, int comp, double x, double y, double z,
-                                         double* psed) {
+                                         int nscatt_peel, bool stellar, int comp, double x, double y, double z) {
     double Lextf = Lpeel * exp(-tau);
     const int nl = S.nlambda;
     int adds = 0;
@@ -240,8 +208,7 @@ int detect_group(const DevScene& S, int grp, int ell, double Lpeel, double tau,
         const int iq = S.group_instr[q];
         const DevInstr& I = S.instr[iq];
         auto sed_add = [&](int c, double v) {
-            if (psed) atomicAdd(psed + S.sed_base[iq] + c * nl + ell, v);
-            else atomicAdd(I.sed + (size_t)c * nl + ell, v);
+            atomicAdd(I.sed + (size_t)c * nl + ell, v);
             adds++;
         };
         int l = (I.type == SKG_INSTR_SED) ? -1 : pixel_on_detector(I, x, y, z);
@@ -454,32 +421,18 @@ SKG_D unsigned peel_bin(const DevGrid& g, int grp, float x, float y, float z) {
            box_bin((x - g.bmid[0]) * g.bscale[0], (y - g.bmid[1]) * g.bscale[1], (z - g.bmid[2]) * g.bscale[2]);
 }
 
-// The direction groups that get a peel-off traversal from (x, y, z), in group order
+// The direction groups that get a peel-off traversal from (x, y, z), as a bit mask
 // (MonteCarloSimulation.cpp:299-357): emission peel-offs carry weight 1, scattering peel-offs the
-// phase-function value, and a negative value ends the list (the reference aborts the peel-off).
-// With WRITE the jobs are stored from j0 on; returns their number.
-template<bool WRITE>
-SKG_D int peel_jobs(const DevScene& S, int ell, bool scat, int cell, double kx, double ky, double kz, double x,
-                    double y, double z, double L, int p, int j0, const WaveParams* W, const DevGrid* grid) {
-    int n = 0;
+// phase-function value, and a negative value ends the list (the reference aborts the peel-off; it
+// takes several dust components).
+SKG_D unsigned peel_groups(const DevScene& S, int ell, bool scat, int cell, double kx, double ky, double kz, double x,
+                           double y, double z) {
+    unsigned need = 0;
     for (int g = 0; g < S.ngroups; g++) {
-        double w = 1.0;
-        if (scat) {
-            w = peel_weight(S, ell, cell, kx, ky, kz, S.gkx[g], S.gky[g], S.gkz[g]);
-            if (w < 0) break;
-        }
-        if (!group_needs_traversal(S, g, x, y, z)) continue;
-        if (WRITE) {
-            W->jobs[j0 + n] = make_int2(p, g);
-            W->jL[j0 + n] = L * w;
-            if (W->hist) {
-                const unsigned b = peel_bin(*grid, g, (float)x, (float)y, (float)z);
-                W->jkey[j0 + n] = make_uint2(b, atomicAdd(W->hist + JOB_BINS + b, 1u));
-            }
-        }
-        n++;
+        if (scat && S.ncomp != 1 && peel_weight(S, ell, cell, kx, ky, kz, S.gkx[g], S.gky[g], S.gkz[g]) < 0) break;
+        if (group_needs_traversal(S, g, x, y, z)) need |= 1u << g;
     }
-    return n;
+    return need;
 }
 
 constexpr int SED_PRIV = 1024;          // SED bins a block keeps privately (8 KB)
@@ -487,8 +440,8 @@ constexpr int SED_PRIV = 1024;          // SED bins a block keeps privately (8 K
 // A packet at its interaction point: propagate, count its scattering peel-offs, scatter
 // (simulatepropagation :513-531, peeloffscattering :313-357, simulatescattering :535-543).
 template<typename R>
-SKG_D void scatter_packet(const RunParams& P, int phase, bool peel_on, Packet& K, int& state, int& npeel, int& nmain,
-                          bool& scat_peel, double& kx0, double& ky0, double& kz0, unsigned long long* s_cnt) {
+SKG_D void scatter_packet(const RunParams& P, int phase, bool peel_on, Packet& K, int& state, unsigned& need,
+                          double& kx0, double& ky0, double& kz0) {
     const WorkItem& It = P.items[K.item];
     const DevScene& S = *P.scenes[It.slot];
     const R si = (R)K.s_int;                        // PhotonPackage::propagate
@@ -499,8 +452,7 @@ SKG_D void scatter_packet(const RunParams& P, int phase, bool peel_on, Packet& K
     if (K.s_int > 0) K.pos_cell = (K.int_cell >= 0) ? K.int_cell : -2;
     kx0 = K.kx; ky0 = K.ky; kz0 = K.kz;
     if (peel_on) {
-        scat_peel = true;
-        npeel = peel_jobs<false>(S, K.ell, true, K.int_cell, kx0, ky0, kz0, K.x, K.y, K.z, K.L, 0, 0, nullptr, nullptr);
+        need = peel_groups(S, K.ell, true, K.int_cell, kx0, ky0, kz0, K.x, K.y, K.z);
     }
     Philox rng;
     rng.init(It.seed, K.id, (uint32_t)K.ell | ((uint32_t)phase << 24));
@@ -509,8 +461,6 @@ SKG_D void scatter_packet(const RunParams& P, int phase, bool peel_on, Packet& K
     K.rngc = rng.c0;
     K.kx = (double)(R)kn.x; K.ky = (double)(R)kn.y; K.kz = (double)(R)kn.z;
     K.nscatt++;
-    atomicAdd(&s_cnt[C_SCATT], 1ull);
-    nmain = 1;
     state = PK_WAIT;
 }
 
@@ -519,7 +469,7 @@ SKG_D void scatter_packet(const RunParams& P, int phase, bool peel_on, Packet& K
 // packet; a record finds none once the work counter is past the batch's packets.
 template<typename R>
 SKG_D void take_packets(const RunParams& P, const BatchHeader& H, int phase, bool peel_on, int lane, bool need,
-                        Packet& K, int& state, int& npeel, int& nmain, unsigned long long* s_cnt) {
+                        Packet& K, int& state, unsigned& groups, unsigned& launched) {
     const unsigned FULL = 0xffffffffu;
     while (__any_sync(FULL, need)) {
         const unsigned want = __ballot_sync(FULL, need);
@@ -540,7 +490,7 @@ SKG_D void take_packets(const RunParams& P, const BatchHeader& H, int phase, boo
                 const int ell = P.ells[It.ell0 + ei];
                 Philox rng;
                 rng.init(It.seed, ip, (uint32_t)ell | ((uint32_t)phase << 24));
-                atomicAdd(&s_cnt[C_PACKETS], 1ull);
+                launched++;
                 const DevScene& S = *P.scenes[It.slot];
                 const Launched o = launch_packet(P.grids[It.slot], S, phase, ell, It.npp_total, rng);
                 if (o.ok) {
@@ -549,12 +499,9 @@ SKG_D void take_packets(const RunParams& P, const BatchHeader& H, int phase, boo
                     K.L = o.L; K.Lth = o.Lth; K.s_int = 0;
                     K.id = ip; K.item = it; K.ell = ell; K.nscatt = 0;
                     K.pos_cell = -2; K.int_cell = -1; K.rngc = rng.c0;
-                    K.flags = pk_flags(o); K.peel_n = 0;
-                    npeel = peel_on ? peel_jobs<false>(S, ell, false, -1, 0, 0, 0, K.x, K.y, K.z, K.L, 0, 0, nullptr,
-                                                       nullptr)
-                                    : 0;
-                    nmain = S.ncomp > 0 ? 1 : 0;            // without dust the life cycle ends here
-                    state = nmain ? PK_WAIT : PK_TERM;
+                    K.flags = pk_flags(o);
+                    groups = peel_on ? peel_groups(S, ell, false, -1, 0, 0, 0, K.x, K.y, K.z) : 0;
+                    state = S.ncomp > 0 ? PK_WAIT : PK_TERM;    // without dust the life cycle ends here
                     need = false;
                 }
             }
@@ -562,223 +509,242 @@ SKG_D void take_packets(const RunParams& P, const BatchHeader& H, int phase, boo
     }
 }
 
-// Appends a packet's jobs (all lanes of the warp call this), one reservation per warp for each
-// kind: the path jobs (the longest) from index 0, a packet's peel-off jobs contiguous from index
-// npool on; counts the packets with work.
-SKG_D void append_jobs(const WaveParams& W, int p, Packet& K, int npeel, int nmain, bool scat_peel, double kx0,
-                       double ky0, double kz0, int lane) {
+// Places for every thread's n[i] entries behind the counters at[i] (all threads of a block of 256
+// call this, as often as one another): one atomic per block and counter, where one per warp made
+// the launches of a wave of 2^21 records wait on a few words of L2.
+template<int N> struct BlockPlaces { unsigned warp[2][N][8], base[2][N]; int turn; };
+template<int N>
+SKG_D void reserve_places(BlockPlaces<N>& sh, int& turn, const unsigned (&n)[N], unsigned* const (&at)[N], unsigned (&place)[N]) {
     const unsigned FULL = 0xffffffffu;
-    int inm = nmain, inp = npeel;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int tm = __shfl_up_sync(FULL, inm, o), tp = __shfl_up_sync(FULL, inp, o);
-        if (lane >= o) { inm += tm; inp += tp; }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = turn;
+    turn ^= 1;                        // (a warp is never two calls ahead of another)
+    unsigned inc[N];
+    for (int i = 0; i < N; i++) {
+        inc[i] = n[i];
+        for (int d = 1; d < 32; d <<= 1) { const unsigned v = __shfl_up_sync(FULL, inc[i], d); if (lane >= d) inc[i] += v; }
+        if (lane == 31) sh.warp[t][i][warp] = inc[i];
     }
-    const int totm = __shfl_sync(FULL, inm, 31), totp = __shfl_sync(FULL, inp, 31);
-    unsigned bm = 0, bp = 0;
-    if (lane == 31) {
-        if (totm > 0) bm = atomicAdd(W.jcount + J_PATH, (unsigned)totm);
-        if (totp > 0) bp = atomicAdd(W.jcount + J_PEEL, (unsigned)totp);
+    __syncthreads();
+    if (threadIdx.x < N) {
+        unsigned sum = 0;
+        for (int w = 0; w < 8; w++) { const unsigned v = sh.warp[t][threadIdx.x][w]; sh.warp[t][threadIdx.x][w] = sum; sum += v; }
+        unsigned* p = at[0];
+        for (int i = 1; i < N; i++) if ((int)threadIdx.x == i) p = at[i];
+        sh.base[t][threadIdx.x] = sum ? atomicAdd(p, sum) : 0;
     }
-    bm = __shfl_sync(FULL, bm, 31);
-    bp = __shfl_sync(FULL, bp, 31);
-    const unsigned busy = __ballot_sync(FULL, npeel + nmain > 0);
-    if (lane == 0 && busy) {
-        atomicAdd(W.jcount + J_BUSY, (unsigned)__popc(busy));
-        atomicMax(W.last_busy, (unsigned)W.wave);
-    }
-    if (npeel > 0) {
-        const int j0 = W.npool + (int)(bp + inp - npeel);
-        const DevScene& S = *W.R.scenes[W.R.items[K.item].slot];
-        peel_jobs<true>(S, K.ell, scat_peel, K.int_cell, kx0, ky0, kz0, K.x, K.y, K.z, K.L, p, j0, &W,
-                        W.R.grids + W.R.items[K.item].slot);
-        K.peel_j0 = j0;
-    }
-    K.peel_n = npeel;
-    if (nmain) {
-        const unsigned j = bm + inm - 1;
-        W.jobs[j] = make_int2(p, JOB_MAIN);
+    __syncthreads();
+    for (int i = 0; i < N; i++) place[i] = sh.base[t][i] + sh.warp[t][i][warp] + inc[i] - n[i];
+}
+
+// Writes a packet's jobs at their places: its path job (path >= 0), its peel-off jobs from j0 on.
+SKG_D void write_jobs(const WaveParams& W, int p, const Packet& K, unsigned need, bool path, bool scat, double kx0,
+                      double ky0, double kz0, unsigned jm, unsigned j0) {
+    const int slot = W.R.items[K.item].slot;
+    const DevScene& S = *W.R.scenes[slot];
+    for (unsigned m = need; m; m &= m - 1, j0++) {
+        const int g = __ffs(m) - 1;
+        const double w = scat ? peel_weight(S, K.ell, K.int_cell, kx0, ky0, kz0, S.gkx[g], S.gky[g], S.gkz[g]) : 1.0;
+        W.jobs[j0] = make_int2(p, g);
+        W.jL[j0] = K.L * w;
         if (W.hist) {
-            const unsigned b = path_bin(W.R.grids[W.R.items[K.item].slot], (float)K.x, (float)K.y, (float)K.z, (float)K.kx,
-                                        (float)K.ky, (float)K.kz);
-            W.jkey[j] = make_uint2(b, atomicAdd(W.hist + b, 1u));
+            const unsigned b = peel_bin(W.R.grids[slot], g, (float)K.x, (float)K.y, (float)K.z);
+            W.jkey[j0] = make_uint2(b, atomicAdd(W.hist + JOB_BINS + b, 1u));
+        }
+    }
+    if (path) {
+        W.jobs[jm] = make_int2(p, JOB_MAIN);
+        if (W.hist) {
+            const unsigned b = path_bin(W.R.grids[slot], (float)K.x, (float)K.y, (float)K.z, (float)K.kx, (float)K.ky,
+                                        (float)K.kz);
+            W.jkey[jm] = make_uint2(b, atomicAdd(W.hist + b, 1u));
         }
     }
 }
 
-template<typename R, bool STRIDE>
-__global__ void __launch_bounds__(SKG_EVENT_THREADS, SKG_EVENT_MIN_BLOCKS * 256 / SKG_EVENT_THREADS) event_kernel(const WaveParams W) {
-    __shared__ unsigned long long s_cnt[C_N];
-    __shared__ double s_sed[SED_PRIV];
-    const RunParams& P = W.R;
-    const BatchHeader H = *P.hdr;
-    // a launch of one simulation tallies its SED bins per block and adds them once at the end
-    const int sed_bins = (H.nslots == 1) ? P.scenes[0]->sed_bins : 0;
-    double* const psed = (sed_bins > 0 && sed_bins <= SED_PRIV) ? s_sed : nullptr;
-    if (threadIdx.x < C_N) s_cnt[threadIdx.x] = 0;
-    if (psed) for (int t = threadIdx.x; t < sed_bins; t += blockDim.x) s_sed[t] = 0.0;
-    __syncthreads();
-#if !SKG_LAUNCH_KERNEL
-    const int phase = H.phase;
-    const bool peel_on = phase != SKG_PHASE_DUST_SELFABS;
-#endif
-    const int lane = threadIdx.x & 31;
-#if SKG_LAUNCH_KERNEL
-    const unsigned FULL = 0xffffffffu;
-#endif
-    // STRIDE: the resident blocks stride over the pool; otherwise one thread per record
-#pragma unroll 1
-    for (int base = blockIdx.x * blockDim.x, it = 0; STRIDE ? base < W.npool : it == 0;
-         base += gridDim.x * blockDim.x, it++) {
-    const int p = base + threadIdx.x;
-
-    Packet K;
-    int state = PK_DONE;
-    if (p < W.npool) { K = W.pk[p]; state = K.state; }
-    const bool was_live = state != PK_DONE;
-    if (state == PK_WAIT) {                       // a path job that was not walked: drop the packet
-        atomicOr(P.err, ERR_CAPACITY); atomicAdd(&s_cnt[C_ERR], 1ull); state = PK_TERM;
-    }
-
-    // 1. the peel-offs walked in the previous wave (Instrument::detect of every group member)
-    if (was_live && K.peel_n > 0) {
-        const DevScene& S = *P.scenes[P.items[K.item].slot];
-        const int nsp = (K.flags & 2) ? K.nscatt : 0;   // the peel-off copy counts the scattering
-        int pix = 0;
-        for (int i = 0; i < K.peel_n; i++) {
-            const int j = K.peel_j0 + i;
-            pix += detect_group(S, W.pjobs[j].y, K.ell, W.pjL[j], W.pjtau[j], nsp, (K.flags & 1) != 0,
-                                pk_comp(K), K.x, K.y, K.z, psed);
-        }
-        atomicAdd(&s_cnt[C_PIX], (unsigned long long)pix);
-        atomicAdd(&s_cnt[C_PEEL], (unsigned long long)K.peel_n);
-        K.peel_n = 0;
-    }
-
-    // 2. a packet at its interaction point: propagate, count its scattering peel-offs, scatter
-    int npeel = 0, nmain = 0;
-    bool scat_peel = false;
-    double kx0 = 0, ky0 = 0, kz0 = 0;              // direction before the scattering
-#if SKG_LAUNCH_KERNEL
-    // (in the launch pass, with every lane of its warps scattering)
-    {
-        const bool inter = p < W.npool && state == PK_INTERACT;
-        const unsigned im = __ballot_sync(FULL, inter);
-        if (im) {
-            const int leader = __ffs(im) - 1;
-            unsigned base = 0;
-            if (lane == leader) base = atomicAdd(W.jcount + J_INT, (unsigned)__popc(im));
-            base = __shfl_sync(FULL, base, leader);
-            if (inter) W.intlist[base + __popc(im & ((1u << lane) - 1))] = p;
-        }
-    }
-#else
-    if (state == PK_INTERACT)
-        scatter_packet<R>(P, phase, peel_on, K, state, npeel, nmain, scat_peel, kx0, ky0, kz0, s_cnt);
-#endif
-
-#if SKG_LAUNCH_KERNEL
-    // 3. free records go on the wave's free list: the launch pass gives them new packets, every
-    //    lane of its warps launching (here a warp's launches would run beside its scatterings)
-    {
-        const bool freed = p < W.npool && (state == PK_EMPTY || state == PK_TERM);
-        const unsigned fm = __ballot_sync(FULL, freed);
-        if (fm) {
-            const int leader = __ffs(fm) - 1;
-            unsigned base = 0;
-            if (lane == leader) base = atomicAdd(W.jcount + J_FREE, (unsigned)__popc(fm));
-            base = __shfl_sync(FULL, base, leader);
-            if (freed) W.freelist[base + __popc(fm & ((1u << lane) - 1))] = p;
-        }
-    }
-#else
-    // 3. free records take new packets
-    take_packets<R>(P, H, phase, peel_on, lane, state == PK_EMPTY || state == PK_TERM, K, state, npeel, nmain, s_cnt);
-#endif
-
-#if SKG_LAUNCH_KERNEL
-    // every live record is now on one of the two lists, and the scatter-and-launch pass rewrites
-    // it (jobs, state, the cleared peel-off count): this pass only read it
-    (void)npeel; (void)nmain; (void)scat_peel; (void)kx0; (void)ky0; (void)kz0; (void)was_live;
-#else
-    // 4. append the jobs
-    append_jobs(W, p, K, npeel, nmain, scat_peel, kx0, ky0, kz0, lane);
-    if (p < W.npool && was_live) {
-        K.flags = (K.flags & ~2) | (scat_peel ? 2 : 0);
-        K.state = state;
-        W.pk[p] = K;
-    }
-#endif
-    }   // records of this block
-    __syncthreads();
-    if (threadIdx.x < C_N && s_cnt[threadIdx.x]) atomicAdd(P.counters + threadIdx.x, s_cnt[threadIdx.x]);
-    if (psed) {
-        const DevScene& S0 = *P.scenes[0];
-        for (int t = threadIdx.x; t < sed_bins; t += blockDim.x) {
-            const double v = s_sed[t];
-            if (v == 0.0) continue;
-            int i = 0;
-            while (i + 1 < S0.ninstr && S0.sed_base[i + 1] <= t) i++;
-            atomicAdd(S0.instr[i].sed + (t - S0.sed_base[i]), v);
-        }
-    }
-}
-
-// Scatter-and-launch pass: one thread per record the event pass found at its interaction point
-// (propagation, scattering peel-offs, scattering), then one per record it freed (StellarSystem::launch
-// and the samplers, or the dust-emission launch), every lane of a warp doing the same work; the
-// packets' jobs are appended as the event pass does.
+// Scatter-and-launch pass: one thread per packet at its interaction point (propagation, scattering
+// peel-offs, scattering), then one per free record (StellarSystem::launch and the samplers, or the
+// dust-emission launch), every lane of a warp doing the same work.  The packets' jobs go on the
+// wave's lists: path jobs from index 0, a packet's peel-off jobs together from index npool on.  A free record
+// that finds no packet is done.
 template<typename R>
-__global__ void __launch_bounds__(SKG_EVENT_THREADS) launch_kernel(const WaveParams W) {
-    __shared__ unsigned long long s_cnt[C_N];
+__global__ void __launch_bounds__(256) launch_kernel(const WaveParams W) {
+    __shared__ BlockPlaces<3> sh;
     const RunParams& P = W.R;
     const BatchHeader H = *P.hdr;
-    if (threadIdx.x < C_N) s_cnt[threadIdx.x] = 0;
-    __syncthreads();
     const int phase = H.phase;
     const bool peel_on = phase != SKG_PHASE_DUST_SELFABS;
     const int lane = threadIdx.x & 31;
-    const unsigned nint = W.jcount[J_INT];
+    int turn = 0;
+    unsigned c_scatt = 0, c_packets = 0;
+    unsigned* const at[3] = {W.jcount + J_PATH, W.jcount + J_PEEL, W.jnext + J_FREE};
+    const unsigned nint = W.wave ? W.jcount[J_INT] : 0;
     for (unsigned b0 = blockIdx.x * blockDim.x; b0 < nint; b0 += gridDim.x * blockDim.x) {
         const unsigned i = b0 + threadIdx.x;
         const bool mine = i < nint;
         const int p = mine ? W.intlist[i] : 0;
         Packet K;
-        int state = PK_DONE, npeel = 0, nmain = 0;
-        bool scat_peel = false;
+        int state = PK_DONE;
+        unsigned need = 0;
         double kx0 = 0, ky0 = 0, kz0 = 0;
         if (mine) {
             K = W.pk[p];
-            state = K.state;
-            scatter_packet<R>(P, phase, peel_on, K, state, npeel, nmain, scat_peel, kx0, ky0, kz0, s_cnt);
+            scatter_packet<R>(P, phase, peel_on, K, state, need, kx0, ky0, kz0);
+            c_scatt++;
         }
-        append_jobs(W, p, K, npeel, nmain, scat_peel, kx0, ky0, kz0, lane);
+        const unsigned n[3] = {mine ? 1u : 0u, (unsigned)__popc(need), 0u};
+        unsigned place[3];
+        reserve_places(sh, turn, n, at, place);
         if (mine) {
-            K.flags = (K.flags & ~2) | (scat_peel ? 2 : 0);   // the pending peel-offs follow a scattering
+            write_jobs(W, p, K, need, true, true, kx0, ky0, kz0, place[0], W.npool + place[1]);
+            K.flags |= 2;                         // the pending peel-offs follow a scattering
             K.state = state;
             W.pk[p] = K;
         }
     }
-    const unsigned nfree = W.jcount[J_FREE];
+    // (every record is free at first)
+    const unsigned nfree = W.wave ? W.jcount[J_FREE] : (unsigned)W.npool;
     for (unsigned b0 = blockIdx.x * blockDim.x; b0 < nfree; b0 += gridDim.x * blockDim.x) {
         const unsigned i = b0 + threadIdx.x;
         const bool mine = i < nfree;
-        const int p = mine ? W.freelist[i] : 0;
+        const int p = !mine ? 0 : W.wave ? W.freelist[i] : (int)i;
         Packet K;
-        int state = PK_DONE, npeel = 0, nmain = 0;
-        if (mine) { K = W.pk[p]; state = K.state; }
-        take_packets<R>(P, H, phase, peel_on, lane, mine, K, state, npeel, nmain, s_cnt);
+        int state = PK_DONE;
+        unsigned need = 0;
+        take_packets<R>(P, H, phase, peel_on, lane, mine, K, state, need, c_packets);
         // the start cell once per packet, all lanes together (otherwise each of its walks looks for it)
-        if (sizeof(R) == 4 && mine && nmain + npeel > 0)
+        if (sizeof(R) == 4 && mine && state != PK_DONE)
             K.pos_cell = start_cell(P.grids[P.items[K.item].slot], (float)K.x, (float)K.y, (float)K.z);
-        append_jobs(W, p, K, npeel, nmain, false, 0, 0, 0, lane);
+        // (a packet without a path leaves its record free for the next wave)
+        const bool path = mine && state == PK_WAIT, ends = mine && state == PK_TERM;
+        const unsigned n[3] = {path ? 1u : 0u, (unsigned)__popc(need), ends ? 1u : 0u};
+        unsigned place[3];
+        reserve_places(sh, turn, n, at, place);
+        if (path || ends) write_jobs(W, p, K, need, path, false, 0, 0, 0, place[0], W.npool + place[1]);
+        if (ends) W.freenext[place[2]] = p;
         if (mine) {
-            K.flags &= ~2;
+            K.nck = 0; K.pad[0] = K.pad[1] = K.pad[2] = 0;
             K.state = state;
-            W.pk[p] = K;
+            if (state == PK_DONE) W.pk[p].state = PK_DONE; else W.pk[p] = K;
         }
     }
+    c_scatt = __reduce_add_sync(0xffffffffu, c_scatt);
+    c_packets = __reduce_add_sync(0xffffffffu, c_packets);
+    if (lane == 0 && c_scatt) atomicAdd(P.counters + C_SCATT, (unsigned long long)c_scatt);
+    if (lane == 0 && c_packets) atomicAdd(P.counters + C_PACKETS, (unsigned long long)c_packets);
+}
+
+// Adds v to the SED bin key (-1: none) of every lane, the lanes of a bin summed first: the packets of
+// a wave share one or two wavelengths, so the lanes' bins are few, and FP64 atomics of a warp on one
+// shared-memory word take turns.  All lanes of the warp call this.
+SKG_D void sed_add(double* sed, int key, double v) {
+    const unsigned FULL = 0xffffffffu;
+    unsigned left = __ballot_sync(FULL, key >= 0);
+    while (left) {
+        const int k0 = __shfl_sync(FULL, key, __ffs(left) - 1);
+        double sum = key == k0 ? v : 0.0;
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(FULL, sum, d);
+        if ((threadIdx.x & 31) == 0) atomicAdd(sed + k0, sum);
+        left &= ~__ballot_sync(FULL, key == k0);
+    }
+}
+
+// Detection pass: one thread per peel-off job of the wave, right after its walks (a pass over all records of the pool in
+// the next wave before, with the records' lists: event and launch passes of the octree disk, 2*10^7 packets, 35.4 ms a
+// phase against 26.5; Cartesian disk, 10^6, 2.40 against 1.25; a batch of 24 fit variants 35.1 against 30.6 ms in all) (Instrument::detect of every member of its
+// direction group; detect_group has the rules).  A launch of one simulation tallies its SED bins per
+// block and adds them once at the end.
+__global__ void __launch_bounds__(256) detect_kernel(const WaveParams W) {
+    __shared__ double s_sed[SED_PRIV];
+    const RunParams& P = W.R;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int sed_bins = (P.hdr->nslots == 1) ? P.scenes[0]->sed_bins : 0;
+    const bool priv = sed_bins > 0 && sed_bins <= SED_PRIV;
+    if (priv) for (int t = threadIdx.x; t < sed_bins; t += blockDim.x) s_sed[t] = 0.0;
     __syncthreads();
-    if (threadIdx.x < C_N && s_cnt[threadIdx.x]) atomicAdd(P.counters + threadIdx.x, s_cnt[threadIdx.x]);
+    unsigned pix = 0, peels = 0;
+    const unsigned n = W.jcount[J_PEEL];
+    for (unsigned b0 = blockIdx.x * blockDim.x; b0 < n; b0 += gridDim.x * blockDim.x) {
+        const unsigned i = b0 + threadIdx.x;
+        const bool on = i < n;
+        if (!priv) {
+            if (on) {
+                const unsigned j = W.npool + i;
+                const int2 jb = W.jobs[j];
+                const Packet& K = W.pk[jb.x];
+                const int fl = K.flags;
+                pix += detect_group(*P.scenes[P.items[K.item].slot], jb.y, K.ell, W.jL[j], W.jtau[j], (fl & 2) ? K.nscatt : 0,
+                                    (fl & 1) != 0, pk_comp(K), K.x, K.y, K.z);
+                peels++;
+            }
+            continue;
+        }
+        const DevScene& S = *P.scenes[0];
+        const int nl = S.nlambda;
+        int q0 = 0, q1 = 0, ell = 0, nsp = 0, fl = 0, comp = -1;
+        double L = 0, Lext = 0, x = 0, y = 0, z = 0;
+        if (on) {
+            const unsigned j = W.npool + i;
+            const int2 jb = W.jobs[j];
+            const Packet& K = W.pk[jb.x];
+            q0 = S.group_start[jb.y]; q1 = S.group_start[jb.y + 1];
+            fl = K.flags; nsp = (fl & 2) ? K.nscatt : 0; ell = K.ell; comp = pk_comp(K);
+            x = K.x; y = K.y; z = K.z;
+            L = W.jL[j];
+            Lext = L * exp(-W.jtau[j]);
+            peels++;
+        }
+        const int members = __reduce_max_sync(FULL, q1 - q0);
+        for (int q = 0; q < members; q++) {
+            int key[3] = {-1, -1, -1};
+            double v[3] = {0, 0, 0};
+            if (q0 + q < q1) {
+                const int iq = S.group_instr[q0 + q];
+                const DevInstr& I = S.instr[iq];
+                const int c0 = S.sed_base[iq] + ell;
+                const int l = (I.type == SKG_INSTR_SED) ? -1 : pixel_on_detector(I, x, y, z);
+                const size_t fp = (size_t)I.nxp * I.nyp;
+                if (I.type != SKG_INSTR_FRAME) { key[0] = c0; v[0] = Lext; pix++; }
+                if (l >= 0) { atomicAdd(I.cube + (size_t)ell * fp + l, Lext); pix++; }
+                if (I.type == SKG_INSTR_FRAME) {
+                    // the frame of the packet's stellar component (component 1 + comp)
+                    if (l >= 0 && I.ncomp > 1 && comp >= 0) {
+                        atomicAdd(I.cube + ((size_t)(1 + comp) * nl + ell) * fp + l, Lext); pix++;
+                    }
+                } else if (I.type == SKG_INSTR_FULL) {
+                    auto add = [&](int s, int c, double value) {
+                        key[s] = c0 + c * nl; v[s] = value; pix++;
+                        if (l >= 0) { atomicAdd(I.cube + ((size_t)c * nl + ell) * fp + l, value); pix++; }
+                    };
+                    if (fl & 1) {
+                        if (nsp == 0) { add(1, SKG_FULL_TRA, L); if (S.ncomp) add(2, SKG_FULL_STRDIR, Lext); }
+                        else {
+                            add(1, SKG_FULL_STRSCA, Lext);
+                            if (nsp <= I.nscatt_levels) add(2, SKG_FULL_NBASE + nsp - 1, Lext);
+                        }
+                    } else {
+                        add(1, nsp == 0 ? SKG_FULL_DUSDIR : SKG_FULL_DUSSCA, Lext);
+                    }
+                }
+            }
+            __syncwarp();
+            for (int s = 0; s < 3; s++) sed_add(s_sed, key[s], v[s]);
+        }
+    }
+    pix = __reduce_add_sync(FULL, pix);
+    peels = __reduce_add_sync(FULL, peels);
+    if (lane == 0 && pix) atomicAdd(P.counters + C_PIX, (unsigned long long)pix);
+    if (lane == 0 && peels) atomicAdd(P.counters + C_PEEL, (unsigned long long)peels);
+    if (!priv) return;
+    __syncthreads();
+    const DevScene& S0 = *P.scenes[0];
+    for (int t = threadIdx.x; t < sed_bins; t += blockDim.x) {
+        const double v = s_sed[t];
+        if (v == 0.0) continue;
+        int i = 0;
+        while (i + 1 < S0.ninstr && S0.sed_base[i + 1] <= t) i++;
+        atomicAdd(S0.instr[i].sed + (t - S0.sed_base[i]), v);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1218,17 +1184,21 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
 }
 
 // The ends of the wave's paths, one thread per path job in walk order: escape fraction, termination
-// test and interaction optical depth (after_path); the packets that interact go on the re-walk list.
+// test and interaction optical depth (after_path).  The packets that interact go on the re-walk list
+// and on the next wave's interaction list, the records of the others on its free list.
 // In a kernel of its own every lane of a warp does this long FP64 work at once, and the walks need
 // no registers for it.
-__global__ void __launch_bounds__(128) path_end_kernel(const WaveParams W) {
+__global__ void __launch_bounds__(256) path_end_kernel(const WaveParams W) {
+    __shared__ BlockPlaces<3> sh;
     const RunParams& P = W.R;
     const unsigned n = W.jcount[J_PATH];
-    const int lane = threadIdx.x & 31;
     const int phase = P.hdr->phase;
+    int turn = 0;
+    unsigned* const at[3] = {W.jcount + J_REWALK, W.jnext + J_INT, W.jnext + J_FREE};
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n + W.jcount[J_PEEL] > 0) *W.last_busy = (unsigned)W.wave;
     for (unsigned b0 = blockIdx.x * blockDim.x; b0 < n; b0 += gridDim.x * blockDim.x) {
         const unsigned i = b0 + threadIdx.x;
-        bool again = false;
+        bool again = false, inter = false;
         int p = 0;
         if (i < n) {
             p = W.hist ? W.spath[i] : W.jobs[i].x;
@@ -1237,15 +1207,16 @@ __global__ void __launch_bounds__(128) path_end_kernel(const WaveParams W) {
             double L = K.L, tau_int = 0;
             const int rc = after_path(W, S, p, phase, K.ell, W.jtau[i], W.path_tau ? 0.0 : W.jL[i], L, tau_int);
             if (rc < 0) atomicAdd(P.counters + C_ERR, 1ull);
-            if (rc == 1) { W.jtau[i] = tau_int; again = true; }
+            again = rc == 1;
+            inter = again || (rc == 0 && K.state == PK_INTERACT);
+            if (again) W.jtau[i] = tau_int;
         }
-        const unsigned am = __ballot_sync(0xffffffffu, again);
-        if (am) {
-            unsigned base = 0;
-            if (lane == 0) base = atomicAdd(W.jcount + J_REWALK, (unsigned)__popc(am));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (again) W.rlist[base + __popc(am & ((1u << lane) - 1))] = make_int2(p, (int)i);
-        }
+        const unsigned cnt[3] = {again ? 1u : 0u, inter ? 1u : 0u, i < n && !inter ? 1u : 0u};
+        unsigned place[3];
+        reserve_places(sh, turn, cnt, at, place);
+        if (again) W.rlist[place[0]] = make_int2(p, (int)i);
+        if (inter) W.intnext[place[1]] = p;
+        else if (i < n) W.freenext[place[2]] = p;
     }
 }
 
@@ -1296,8 +1267,7 @@ SKG_D void tail_peel(const DevGrid& g, const DevScene& S, const Packet& K, bool 
         const double tau = tail_tau<R, Stepper>(g, S, K.ell, (R)K.x, (R)K.y, (R)K.z, (R)S.gkx[grp], (R)S.gky[grp],
                                                 (R)S.gkz[grp], K.pos_cell, cnt, err);
         cnt[C_PEEL]++;
-        cnt[C_PIX] += detect_group(S, grp, K.ell, K.L * w, tau, nsp, (K.flags & 1) != 0, pk_comp(K), K.x, K.y, K.z,
-                                   nullptr);
+        cnt[C_PIX] += detect_group(S, grp, K.ell, K.L * w, tau, nsp, (K.flags & 1) != 0, pk_comp(K), K.x, K.y, K.z);
     }
 }
 
@@ -1378,21 +1348,6 @@ __global__ void __launch_bounds__(128) tail_kernel(const WaveParams W) {
     const bool peel_on = phase != SKG_PHASE_DUST_SELFABS;
     unsigned long long cnt[C_N];
     for (int c = 0; c < C_N; c++) cnt[c] = 0;
-    if (state == PK_WAIT) {                       // a path job that was not walked (as the event pass)
-        atomicOr(P.err, ERR_CAPACITY); cnt[C_ERR]++; state = PK_TERM;
-    }
-    // the peel-offs walked in the last wave
-    if (K.peel_n > 0) {
-        const DevScene& S = *P.scenes[P.items[K.item].slot];
-        const int nsp = (K.flags & 2) ? K.nscatt : 0;
-        for (int i = 0; i < K.peel_n; i++) {
-            const int j = K.peel_j0 + i;
-            cnt[C_PIX] += detect_group(S, W.pjobs[j].y, K.ell, W.pjL[j], W.pjtau[j], nsp, (K.flags & 1) != 0,
-                                       pk_comp(K), K.x, K.y, K.z, nullptr);
-        }
-        cnt[C_PEEL] += K.peel_n;
-        K.peel_n = 0;
-    }
     while (true) {
         if (state == PK_INTERACT) {
             const WorkItem& It = P.items[K.item];
@@ -1442,7 +1397,7 @@ __global__ void __launch_bounds__(128) tail_kernel(const WaveParams W) {
         K.L = o.L; K.Lth = o.Lth; K.s_int = 0;
         K.id = ip; K.item = it; K.ell = ell; K.nscatt = 0;
         K.pos_cell = -2; K.int_cell = -1; K.rngc = rng.c0;
-        K.flags = pk_flags(o); K.peel_n = 0;
+        K.flags = pk_flags(o);
         if (peel_on) tail_peel<R, Stepper>(P.grids[It.slot], S, K, false, 0, 0, 0, 0, cnt, P.err);
         state = S.ncomp > 0 ? PK_WAIT : PK_TERM;   // without dust the life cycle ends here
     }
@@ -1480,47 +1435,23 @@ int resident_blocks(size_t smem) {
 }
 
 template<typename R, template<typename> class Stepper, bool ONE>
-cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaEvent_t mid, cudaStream_t s) {
+cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaEvent_t mid, cudaEvent_t walked, cudaStream_t s) {
     const size_t smem = (size_t)nslots * sizeof(DevGrid);
-    const int need = (W.npool + SKG_EVENT_THREADS - 1) / SKG_EVENT_THREADS;
-    // (Cartesian grids only: the octree's event pass, detections into three 512^2 frames, is slower
-    // strided at any pool size -- 2^21: 52.2 against 44.8 ms over 150 launches -- its heavier
-    // records unevenly spread over the resident blocks)
-    constexpr bool cart = std::is_same<Stepper<R>, CartStepper<R>>::value || std::is_same<Stepper<R>, CartUniStepper<R>>::value;
-    if (cart && W.npool <= SKG_EVENT_STRIDE_POOL) {
-        static int esms = 0, eper = 1;
-        if (esms == 0) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&esms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&eper, event_kernel<R, true>, SKG_EVENT_THREADS, 0);
-            if (eper <= 0) eper = 1;
-        }
-        event_kernel<R, true><<<std::min(need, esms * eper), SKG_EVENT_THREADS, 0, s>>>(W);
-    } else {
-        event_kernel<R, false><<<need, SKG_EVENT_THREADS, 0, s>>>(W);
+    const int need = (W.npool + 255) / 256;
+    // grid-stride passes over at most the blocks resident at once
+    static int lper = 0, dper = 0;
+    if (lper == 0) {
+        int d = 0, l = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, detect_kernel, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l, launch_kernel<R>, 256, 0);
+        dper = std::max(d, 1); lper = std::max(l, 1);
     }
-#if SKG_LAUNCH_KERNEL
-    {
-        // a grid-stride pass: SKG_LAUNCH_OCC sizes it to the blocks that are resident at once
-        static int sms = 0, per = 16;
-        if (sms == 0) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-#if SKG_LAUNCH_OCC
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, launch_kernel<R>, SKG_EVENT_THREADS, 0);
-            if (per <= 0) per = 1;
-#endif
-        }
-        launch_kernel<R><<<sms * per, SKG_EVENT_THREADS, 0, s>>>(W);
-        if (W.hist) {
-            bin_sums_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0 + 2 * JOB_BINS);
-            bins_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0, W.bin0 + 2 * JOB_BINS);
-            order_kernel<<<std::min(sms * 8, (W.npool + 255) / 256), 256, 0, s>>>(W);
-        }
+    launch_kernel<R><<<std::min(need, dev_sms() * lper), 256, 0, s>>>(W);
+    if (W.hist) {
+        bin_sums_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0 + 2 * JOB_BINS);
+        bins_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0, W.bin0 + 2 * JOB_BINS);
+        order_kernel<<<std::min(dev_sms() * 8, need), 256, 0, s>>>(W);
     }
-#endif
     if (mid) cudaEventRecord(mid, s);
     auto blocks = [&](int resident) { return trav_blocks > 0 ? trav_blocks : resident; };
     if (W.path_tau) {
@@ -1540,8 +1471,10 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
         cudaError_t e = cudaLaunchKernelEx(&cfg, trav_kernel<R, Stepper, TRAV_TAU, ONE>, W);
         if (e != cudaSuccess) return e;
     }
-    path_end_kernel<<<std::min(need * SKG_EVENT_THREADS / 128 + 1, dev_sms() * 16), 128, 0, s>>>(W);
+    path_end_kernel<<<std::min(need, dev_sms() * 8), 256, 0, s>>>(W);
     trav_kernel<R, Stepper, TRAV_REWALK, ONE><<<resident_blocks<R, Stepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
+    if (walked) cudaEventRecord(walked, s);
+    detect_kernel<<<std::min(need * 2, dev_sms() * dper), 256, 0, s>>>(W);
     return cudaGetLastError();
 }
 
@@ -1552,7 +1485,7 @@ cudaError_t enqueue_tail(const WaveParams& W, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-using WaveFn = cudaError_t (*)(const WaveParams&, int, int, cudaEvent_t, cudaStream_t);
+using WaveFn = cudaError_t (*)(const WaveParams&, int, int, cudaEvent_t, cudaEvent_t, cudaStream_t);
 using TailFn = cudaError_t (*)(const WaveParams&, cudaStream_t);
 struct PassFns { WaveFn wave; TailFn tail; };
 
@@ -1589,10 +1522,9 @@ WaveRunner::~WaveRunner() {
     for (cudaEvent_t e : ev_) cudaEventDestroy(e);
     for (cudaEvent_t e : tail_ev_) if (e) cudaEventDestroy(e);
     // (a runner that never reserved frees nothing: no device-wide synchronisation)
-    for (void* p : {(void*)pk_, (void*)free_, (void*)ckpt_, (void*)ctr_, (void*)bins_, (void*)order_})
+    for (void* p : {(void*)pk_, (void*)lists_[0], (void*)lists_[1], (void*)rlist_, (void*)ckpt_, (void*)ctr_, (void*)bins_,
+                    (void*)order_, (void*)jobs_, (void*)jtau_, (void*)jL_})
         if (p) cudaFree(p);
-    for (int b = 0; b < 2; b++)
-        for (void* p : {(void*)jobs_[b], (void*)jtau_[b], (void*)jL_[b]}) if (p) cudaFree(p);
     if (h_ctr_) cudaFreeHost(h_ctr_);
     if (copied_) cudaEventDestroy(copied_);
 }
@@ -1625,9 +1557,12 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t 
         if ((e = cudaEventCreateWithFlags(&copied_, cudaEventDisableTiming)) != cudaSuccess) return e;
     }
     if (pool > cap_pool_) {
-        cudaFree(pk_); pk_ = nullptr; cudaFree(free_); free_ = nullptr; cap_pool_ = 0;
+        for (void** q : {(void**)&pk_, (void**)&lists_[0], (void**)&lists_[1], (void**)&rlist_}) { cudaFree(*q); *q = nullptr; }
+        cap_pool_ = 0;
         if ((e = cudaMalloc(&pk_, pool * sizeof(Packet))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&free_, 2 * pool * sizeof(int))) != cudaSuccess) return e;
+        for (int b = 0; b < 2; b++)
+            if ((e = cudaMalloc(&lists_[b], 2 * pool * sizeof(int))) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&rlist_, pool * sizeof(int2))) != cudaSuccess) return e;
         cap_pool_ = pool;
     }
     if (SKG_CKPT && ckpt_grid(grid_type) && pool > cap_ckpt_) {
@@ -1642,16 +1577,11 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t 
     const size_t jobs = pool * (size_t)(ngroups + 1);
     if (jobs > cap_jobs_) {
 
-        for (int b = 0; b < 2; b++) {
-            cudaFree(jobs_[b]); cudaFree(jtau_[b]); cudaFree(jL_[b]);
-            jobs_[b] = nullptr; jtau_[b] = nullptr; jL_[b] = nullptr;
-        }
+        for (void** q : {(void**)&jobs_, (void**)&jtau_, (void**)&jL_}) { cudaFree(*q); *q = nullptr; }
         cap_jobs_ = 0;
-        for (int b = 0; b < 2; b++) {
-            if ((e = cudaMalloc(&jobs_[b], jobs * sizeof(int2))) != cudaSuccess) return e;
-            if ((e = cudaMalloc(&jtau_[b], jobs * sizeof(double))) != cudaSuccess) return e;
-            if ((e = cudaMalloc(&jL_[b], jobs * sizeof(double))) != cudaSuccess) return e;
-        }
+        if ((e = cudaMalloc(&jobs_, jobs * sizeof(int2))) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&jtau_, jobs * sizeof(double))) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&jL_, jobs * sizeof(double))) != cudaSuccess) return e;
         cap_jobs_ = jobs;
     }
     if (order_on_ && jobs > cap_order_) {
@@ -1672,26 +1602,28 @@ cudaError_t WaveRunner::enqueue(int n) {
         const int w = waves_ + i, b = w & 1;
         WaveParams W;
         W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = w;
-        W.jobs = jobs_[b]; W.jtau = jtau_[b]; W.jL = jL_[b]; W.jcount = ctr_ + J_N * b;
-        W.pjobs = jobs_[b ^ 1]; W.pjtau = jtau_[b ^ 1]; W.pjL = jL_[b ^ 1];
+        W.jobs = jobs_; W.jtau = jtau_; W.jL = jL_;
+        W.jcount = ctr_ + J_N * b; W.jnext = ctr_ + J_N * (b ^ 1);
         W.last_busy = ctr_ + 2 * J_N;
-        W.freelist = free_; W.intlist = free_ + npool_; W.rlist = reinterpret_cast<int2*>(free_); W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+        W.freelist = lists_[b]; W.intlist = lists_[b] + npool_; W.freenext = lists_[b ^ 1]; W.intnext = lists_[b ^ 1] + npool_;
+        W.rlist = rlist_; W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
         W.g0 = g0_;
         W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
         // (a job's key lies where its optical depth will)
-        W.jkey = reinterpret_cast<uint2*>(jtau_[b]); W.speel = order_;
+        W.jkey = reinterpret_cast<uint2*>(jtau_); W.speel = order_;
         W.spath = reinterpret_cast<int*>(order_ + (cap_order_ - npool_));
-        if ((e = cudaMemsetAsync(ctr_ + J_N * b, 0, J_N * sizeof(unsigned), stream_)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(ctr_ + J_N * (b ^ 1), 0, J_N * sizeof(unsigned), stream_)) != cudaSuccess) return e;
         if (timed_) {
-            while (ev_.size() < 3 * (size_t)(w + 1)) {
+            while (ev_.size() < 4 * (size_t)(w + 1)) {
                 cudaEvent_t x;
                 if ((e = cudaEventCreate(&x)) != cudaSuccess) return e;
                 ev_.push_back(x);
             }
-            if ((e = cudaEventRecord(ev_[3 * w], stream_)) != cudaSuccess) return e;
+            if ((e = cudaEventRecord(ev_[4 * w], stream_)) != cudaSuccess) return e;
         }
-        if ((e = fn(W, nslots_, trav_blocks_, timed_ ? ev_[3 * w + 1] : nullptr, stream_)) != cudaSuccess) return e;
-        if (timed_ && (e = cudaEventRecord(ev_[3 * w + 2], stream_)) != cudaSuccess) return e;
+        if ((e = fn(W, nslots_, trav_blocks_, timed_ ? ev_[4 * w + 1] : nullptr, timed_ ? ev_[4 * w + 2] : nullptr, stream_)) !=
+            cudaSuccess) return e;
+        if (timed_ && (e = cudaEventRecord(ev_[4 * w + 3], stream_)) != cudaSuccess) return e;
     }
     waves_ += n;
     if ((e = cudaMemcpyAsync(h_ctr_, ctr_, NCTR * sizeof(unsigned), cudaMemcpyDeviceToHost, stream_)) != cudaSuccess) return e;
@@ -1724,24 +1656,22 @@ cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, 
     cudaStreamIsCapturing(s, &cs);
     timed_ = timing && cs == cudaStreamCaptureStatusNone;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(pk_, 0, npool * sizeof(Packet), s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(ctr_, 0, NCTR * sizeof(unsigned), s)) != cudaSuccess) return e;
     pending_ = true;
     tail_only_ = tail_div_ > 0 && fits && npool <= (size_t)(grid_type == SKG_GRID_CARTESIAN ? SKG_TAIL_ONLY_CART : SKG_TAIL_ONLY);
     if (!tail_only_) return enqueue(estimate);
+    if ((e = cudaMemsetAsync(pk_, 0, npool * sizeof(Packet), s)) != cudaSuccess) return e;   // (wave 0 writes every record)
     if ((e = enqueue_tail()) != cudaSuccess) return e;
     return record_copied();
 }
 
 cudaError_t WaveRunner::enqueue_tail() {
-    const int b = (waves_ + 1) & 1;               // the last wave's jobs hold the pending peel-offs
     WaveParams W;
     W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = waves_;
-    W.jobs = nullptr; W.jtau = nullptr; W.jL = nullptr; W.jcount = ctr_ + J_N * (b ^ 1);
-    W.pjobs = jobs_[b]; W.pjtau = jtau_[b]; W.pjL = jL_[b];
+    W.jobs = nullptr; W.jtau = nullptr; W.jL = nullptr; W.jcount = nullptr; W.jnext = nullptr;
     W.last_busy = ctr_ + 2 * J_N;
     W.tail_lanes = waves_ ? 32 : std::min(32, std::max(1, npool_ / (dev_sms() * 16)));
-    W.freelist = nullptr; W.intlist = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+    W.freelist = nullptr; W.intlist = nullptr; W.freenext = nullptr; W.intnext = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
     W.hist = nullptr; W.bin0 = nullptr; W.jkey = nullptr; W.spath = nullptr; W.speel = nullptr;
     cudaError_t e;
     if (timed_) {
@@ -1772,10 +1702,12 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
             std::this_thread::sleep_for(std::chrono::microseconds(50));
         }
         if (tail_only_) { pending_ = false; break; }
-        const unsigned busy = h_ctr_[J_N * ((waves_ - 1) & 1) + J_BUSY];
+        // packets with jobs in the last wave (without dust a packet has peel-offs alone)
+        const unsigned* c = h_ctr_ + J_N * ((waves_ - 1) & 1);
+        const unsigned busy = c[J_PATH] ? c[J_PATH] : c[J_PEEL];
         if (busy == 0) {
             pending_ = false;
-            estimate = (int)h_ctr_[2 * J_N] + 3;        // the last busy wave, the detection wave, one spare
+            estimate = (int)h_ctr_[2 * J_N] + 2;        // the last busy wave, the empty one, one spare
             break;
         }
         if (tail_div_ > 0 && (size_t)busy * (size_t)tail_div_ <= (size_t)npool_) {
@@ -1800,10 +1732,12 @@ cudaError_t WaveRunner::times(float* event_ms, float* trav_ms) const {
     if (timed_ && !pending_) {
         for (int w = 0; w < waves_; w++) {
             float x = 0, y = 0;
-            cudaError_t e = cudaEventElapsedTime(&x, ev_[3 * w], ev_[3 * w + 1]);
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&y, ev_[3 * w + 1], ev_[3 * w + 2]);
+            cudaError_t e = cudaEventElapsedTime(&x, ev_[4 * w], ev_[4 * w + 1]);
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&y, ev_[4 * w + 1], ev_[4 * w + 2]);
             if (e != cudaSuccess) return e;
             a += x; t += y;
+            if ((e = cudaEventElapsedTime(&x, ev_[4 * w + 2], ev_[4 * w + 3])) != cudaSuccess) return e;
+            a += x;
         }
         if (tail_ran_) {
             float y = 0;

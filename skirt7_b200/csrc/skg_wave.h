@@ -1,12 +1,12 @@
 // skg_wave.h -- host side of the wavefront packet tracer (kernels in skg_tracer.cu).
 //
-// A phase runs as a sequence of waves on one stream.  Wave w: an event pass over the packet pool
-// (detect the previous wave's peel-offs, launch new packets into free records, move scattered
-// packets to their interaction point, scatter, and write the next traversals as jobs) followed by
-// a traversal pass that walks every job of the wave.  The number of waves is not known in
-// advance: begin() enqueues an estimate, finish() reads how many packets still had work after the
-// last enqueued wave and enqueues more until none has -- or, once few have, the tail pass, which
-// finishes every remaining packet in one launch.
+// A phase runs as a sequence of waves on one stream.  Wave w: a launch pass (scatter the packets that
+// the previous wave brought to their interaction point, launch new packets into the records that it freed, and write the
+// next traversals as jobs), the walks of every job, and a detection pass over the peel-offs.
+// The number of waves is not known in advance: begin() enqueues an estimate, finish() reads how many
+// packets still had work in the last enqueued wave and enqueues more until none has -- or, once few
+// have, the tail pass, which finishes every remaining packet in one launch.  Phases of few packets
+// are the tail pass alone.
 #pragma once
 #include "skg_scene.cuh"
 
@@ -60,14 +60,15 @@ private:
     cudaError_t record_copied();
 
     Packet* pk_ = nullptr;
-    int* free_ = nullptr;             // [pool] records freed in a wave, [pool] records at their
-                                      // interaction point (the scatter-and-launch pass's work)
+    int* lists_[2] = {nullptr, nullptr};   // [pool] free records, [pool] records at their interaction
+                                      // point: a wave's, and the next wave's (which it fills)
+    int2* rlist_ = nullptr;           // [pool] paths to re-walk
     float4* ckpt_ = nullptr;          // [pool][checkpoints][2] path-walk checkpoints
     size_t cap_ckpt_ = 0;
     size_t cap_pool_ = 0;
-    int2* jobs_[2] = {nullptr, nullptr};
-    double* jtau_[2] = {nullptr, nullptr};
-    double* jL_[2] = {nullptr, nullptr};
+    int2* jobs_ = nullptr;
+    double* jtau_ = nullptr;
+    double* jL_ = nullptr;
     size_t cap_jobs_ = 0;
     int generation_ = 0;
     unsigned* bins_ = nullptr;        // [2][JOB_BINS] counts, [2][JOB_BINS] first places (walk order)
@@ -76,7 +77,7 @@ private:
     bool order_on_ = false;           // the running phase walks its jobs in spatial order
     bool path_tau_ = false;
     static constexpr int NCTR = 2 * J_N + 1;
-    unsigned* ctr_ = nullptr;         // [J_N b + JobCount]: counters of job buffer b; [2 J_N]: last busy wave
+    unsigned* ctr_ = nullptr;         // [J_N (w & 1) + JobCount]: counters of wave w; [2 J_N]: last busy wave
     unsigned* h_ctr_ = nullptr;       // pinned copy read by finish()
     cudaEvent_t copied_ = nullptr;
 
@@ -89,7 +90,7 @@ private:
     int tree_walk_ = TW_ROPE;
     int npool_ = 0;
     int waves_ = 0;
-    std::vector<cudaEvent_t> ev_;      // 3 per wave: before the event pass, between, after the traversal
+    std::vector<cudaEvent_t> ev_;      // 4 per wave: before the launch pass, the walks, the detection, and after it
     bool timed_ = false;               // the running phase records ev_
     int tail_div_ = 16;
     bool ckpt_on_ = true;              // path-walk checkpoints (environment variable SKG_CKPT=0: off)
