@@ -286,7 +286,9 @@ DevGrid make_grid(Allocs& A, const skg_grid& g, cudaStream_t s) {
                 }
                 const size_t at = (size_t)po[m].x + (size_t)(q - g.vnbr_offsets[m]);
                 pl[at] = make_float4((float)nx, (float)ny, (float)nz, (float)w);
-                nx4[at] = (mi >= 0) ? make_int4(mi, po[mi].x, po[mi].y, off[mi + 1] - off[mi]) : make_int4(mi, 0, 0, 0);
+                const int np = mi >= 0 ? po[mi].y - po[mi].x : 0;
+                nx4[at] = (mi >= 0) ? make_int4(mi, po[mi].x, np < 32768 ? np | (off[mi + 1] - off[mi]) << 16 : -1, 0)
+                                    : make_int4(mi, 0, 0, 0);
             }
         }
         G.vplane = upload(A, pl.data(), pl.size(), s);
@@ -527,7 +529,8 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
                 CK(cudaStreamSynchronize(s));
             }
             H.rhof = rf;
-            if (sc->ncomp == 1 && (ctx->grid.lrec || ctx->grid.prec)) CK(launch_embed_density(ctx->grid, rf, s));
+            if (sc->ncomp == 1) ctx->grid.rho1 = rf;
+            if (sc->ncomp == 1 && (ctx->grid.lrec || ctx->grid.prec || ctx->grid.vnext)) CK(launch_embed_density(ctx->grid, rf, s));
         }
 
         // octant records of the FP32 walk (256 bytes per cell; without them it takes the lattice records)

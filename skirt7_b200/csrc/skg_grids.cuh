@@ -23,6 +23,7 @@ struct DevGrid {
     float  epsf;                // FP32 nudge (a few ulps of the domain size)
     int ncells;
     int max_steps;
+    const float* rho1;          // cell densities of a single dust component (FP32; null otherwise)
     float bmid[3], bscale[3];   // middle of the box and 1 / its half widths (bins of the walk order)
 
     // Cartesian planes
@@ -75,7 +76,8 @@ struct DevGrid {
     // Each cell's entries start at an even place and are an even number (an odd list ends with a zero
     // plane, which no ray crosses), so that two planes come in one 32-byte load; vpoff[m] = (first, end).
     const float4* vplane;
-    const int4*   vnext;       // per entry: (neighbour, its first entry, its end entry, its neighbour count)
+    const int4*   vnext;       // per entry: (neighbour, its first entry, its entries | its neighbour count << 16 (-1: see
+                               // vpoff), bits of its density (one dust component))
     const int2*   vpoff;
     // The same lists for the peel-off direction of each group (scenes of few groups; null otherwise): only
     // the planes ahead of that direction (n.k > 0), in the same order; gpoff[group * nsites + m].
@@ -444,8 +446,9 @@ struct CartUniStepper<float> {
     bool done;
     int steps;
     int cell0;
+    float rho;                  // density of the last segment's cell (-1: to be read from the scene)
+    float rho_ahead;            // of the current cell: loaded as the walk enters it, a step before its use
     static constexpr int fallbacks = 0;
-    static constexpr float rho = -1.f;
     SKG_D int nscanned() const { return 0; }
 
     SKG_D static void axis(float org, float h, float o, float k, int c, int n, float& c0, float& dt, float& q, float& tn,
@@ -476,10 +479,12 @@ struct CartUniStepper<float> {
         my = dy < 0.f ? -g.nz : g.nz;
         mx = (dx < 0.f ? -g.nz : g.nz) * g.ny;
         cell = e.k + g.nz * (e.j + g.ny * e.i);
+        rho = -1.f;
+        rho_ahead = g.rho1 ? __ldg(g.rho1 + cell) : -1.f;
     }
     static constexpr bool resumable = false;
     SKG_D bool next(const DevGrid& g, int& m, float& ds) {
-        if (pd.pop(ds)) { m = -1; return true; }
+        if (pd.pop(ds)) { m = -1; rho = 0.f; return true; }
         return walk(g, m, ds);
     }
     // One cell step: the nearest wall (the reference's tie order x, y, z) and, predicated, its axis's
@@ -489,12 +494,14 @@ struct CartUniStepper<float> {
         while (!done) {
             if (++steps > g.max_steps) { done = true; return false; }
             m = cell;
+            rho = rho_ahead;
             const float t = fminf(fminf(tx, ty), tz);
             const bool ax = tx <= t, ay = !ax && ty <= t;
             if (ax) { qx += copysignf(1.f, dtx); tx = fmaf(qx, dtx, cx); cell += mx; }
             else if (ay) { qy += copysignf(1.f, dty); ty = fmaf(qy, dty, cy); cell += my; }
             else { qz += copysignf(1.f, dtz); tz = fmaf(qz, dtz, cz); cell += mz; }
             done = t >= tend;
+            if (!done && g.rho1) rho_ahead = __ldg(g.rho1 + cell);
             const float d = t - tc;
             tc = t;
             if (d > 0.f) { ds = d; return true; }   // DustGridPath::addSegment drops ds <= 0
@@ -1185,7 +1192,8 @@ struct VoronoiStepper {
     int scanned;
     SKG_D int nscanned() const { return scanned; }
     int cell0;
-    static constexpr float rho = -1.f;
+    float rho = -1.f;           // FP32 walk: density of the last segment's cell (-1: to be read from the scene)
+    float rho_ahead = -1.f;     // of the current cell
 
     // hint: the cell holding the start position (the interaction point lies in the cell of its
     // segment); accepted for a position strictly inside the domain
@@ -1220,7 +1228,7 @@ struct VoronoiStepper {
     }
 
     SKG_D bool next(const DevGrid& g, int& m, R& ds) {
-        if (pd.pop(ds)) { m = -1; return true; }
+        if (pd.pop(ds)) { m = -1; rho = 0.f; return true; }
         return walk(g, m, ds);
     }
     // the segments inside the grid (after the entry segments have been taken)
@@ -1297,6 +1305,7 @@ SKG_D bool VoronoiStepper<float>::walk(const DevGrid& g, int& m, float& ds) {
         const int2 o = group < 0 ? __ldg(g.vpoff + mr) : __ldg(g.gpoff + (size_t)group * g.nsites + mr);
         qb = o.x; qe = o.y;
         nnb = g.vnoff[mr + 1] - g.vnoff[mr];
+        rho_ahead = g.rho1 ? __ldg(g.rho1 + mr) : -1.f;
     };
     if (qe < 0 && !done) enter();
     while (!done) {
@@ -1334,8 +1343,11 @@ SKG_D bool VoronoiStepper<float>::walk(const DevGrid& g, int& m, float& ds) {
         m = mr;
         x += (sq + g.epsf) * kx; y += (sq + g.epsf) * ky; z += (sq + g.epsf) * kz;
         const int4 e = __ldg(nexts + qbest);
-        mr = e.x; qb = e.y; qe = e.z; nnb = e.w;
+        rho = rho_ahead;
+        mr = e.x; qb = e.y; qe = qb + (e.z & 0xffff); nnb = e.z >> 16;
+        rho_ahead = g.rho1 ? __int_as_float(e.w) : -1.f;
         if (mr < 0) done = true;
+        else if (e.z == -1) enter();
         ds = (mr >= 0) ? sq + g.epsf : sq;   // the nudge is credited to this segment (exact total length)
         return true;
     }

@@ -266,9 +266,24 @@ __global__ void embed_density_lattice_kernel(uint4* prec, int ncells, const floa
     if (m >= ncells) return;
     prec[2 * (size_t)m].x = __float_as_uint(rhof[m]);
 }
+// And the density of the neighbour behind each Voronoi wall: all of cell m's entries, padding included.
+__global__ void embed_density_voronoi_kernel(const int2* __restrict__ ranges, int4* next, int ncells,
+                                             const float* __restrict__ rhof) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= ncells) return;
+    const int2 o = ranges[m];
+    for (int q = o.x; q < o.y; q++) {
+        const int mi = next[q].x;
+        if (mi >= 0) next[q].w = __float_as_int(rhof[mi]);
+    }
+}
 cudaError_t launch_embed_density(const DevGrid& g, const float* rhof, cudaStream_t s) {
     int n = g.ncells;
     if (n <= 0) return cudaSuccess;
+    if (g.vnext) {
+        embed_density_voronoi_kernel<<<(n + 127) / 128, 128, 0, s>>>(g.vpoff, const_cast<int4*>(g.vnext), n, rhof);
+        return cudaGetLastError();
+    }
     if (g.lattice) embed_density_lattice_kernel<<<(n + 255) / 256, 256, 0, s>>>(const_cast<uint4*>(g.prec), n, rhof);
     else embed_density_kernel<<<(n + 255) / 256, 256, 0, s>>>(const_cast<float4*>(g.lrec), n, rhof);
     return cudaGetLastError();
@@ -339,7 +354,8 @@ __global__ void group_planes_kernel(const DevGrid g, const GroupDirs d, int ngro
         const int4 nx = g.vnext[i];
         planes[at] = p;
         const int64_t f = (int64_t)q * g.nsites + max(nx.x, 0);
-        nexts[at] = nx.x >= 0 ? make_int4(nx.x, first[f], first[f + 1], nx.w) : nx;
+        const int np = first[f + 1] - first[f];
+        nexts[at] = nx.x < 0 ? nx : make_int4(nx.x, first[f], nx.z == -1 ? -1 : np | (nx.z & ~0xffff), nx.w);
         at++;
     }
     for (; at < end; at++) { planes[at] = make_float4(0.f, 0.f, 0.f, 0.f); nexts[at] = make_int4(-1, 0, 0, 0); }

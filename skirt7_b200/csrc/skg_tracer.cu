@@ -567,7 +567,10 @@ SKG_D void write_jobs(const WaveParams& W, int p, const Packet& K, unsigned need
 // wave's lists: path jobs from index 0, a packet's peel-off jobs together from index npool on.  A free record
 // that finds no packet is done.
 template<typename R>
-__global__ void __launch_bounds__(256) launch_kernel(const WaveParams W) {
+#ifndef SKG_LB
+#define SKG_LB 3
+#endif
+__global__ void __launch_bounds__(256, SKG_LB) launch_kernel(const WaveParams W) {
     __shared__ BlockPlaces<3> sh;
     const RunParams& P = W.R;
     const BatchHeader H = *P.hdr;
