@@ -93,11 +93,11 @@ namespace skg {
 // phases of at most this many packets (Cartesian, other grids) run in the tail pass alone: with a few
 // lanes of every warp busy a wave lasts as long as its longest walk, about 100 us each on a small Cartesian grid, and a
 // phase takes some twenty of them.  Waves against the tail pass alone, ms per phase: 40x40x20 Cartesian
-// grid 10^4 packets 2.10 / 0.90, 4*10^4 2.37 / 1.92, 8*10^4 2.66 / 2.55; 100x100x50 4*10^4 3.37 / 3.28, 8*10^4 3.60 /
-// 4.50; octree with four observers 4*10^3 1.70 / 1.00, 10^4 1.80 / 1.73, 2*10^4 1.87 / 2.75; 10^6 Voronoi
-// cells 10^4 28.8 / 28.2, 2*10^4 34.2 / 42.5
+// grid 10^4 packets 1.76 / 1.00, 2*10^4 1.83 / 1.49, 4*10^4 1.98 / 2.23; 100x100x50 2*10^4 2.40 / 2.12, 4*10^4 2.77 /
+// 3.48; octree with four observers 4*10^3 1.52 / 1.00, 10^4 1.59 / 1.70; 10^6-leaf k-d tree 10^4 2.97 / 2.96;
+// Voronoi, 2*10^4 cells, 4*10^3 5.08 / 3.48, 10^4 5.61 / 5.54; 10^6 cells 4*10^3 22.0 / 16.3, 10^4 24.1 / 24.9
 #ifndef SKG_TAIL_ONLY_CART
-#define SKG_TAIL_ONLY_CART (1 << 15)
+#define SKG_TAIL_ONLY_CART 20000
 #endif
 #ifndef SKG_TAIL_ONLY
 #define SKG_TAIL_ONLY (1 << 13)
@@ -566,11 +566,10 @@ SKG_D void write_jobs(const WaveParams& W, int p, const Packet& K, unsigned need
 // dust-emission launch), every lane of a warp doing the same work.  The packets' jobs go on the
 // wave's lists: path jobs from index 0, a packet's peel-off jobs together from index npool on.  A free record
 // that finds no packet is done.
+// (3 blocks per SM, 80 registers: launch pass of the octree disk, 10^7 packets, 8.7 ms at 2 blocks and 120
+// registers, 7.8 at 3; 4 no faster)
 template<typename R>
-#ifndef SKG_LB
-#define SKG_LB 3
-#endif
-__global__ void __launch_bounds__(256, SKG_LB) launch_kernel(const WaveParams W) {
+__global__ void __launch_bounds__(256, 3) launch_kernel(const WaveParams W) {
     __shared__ BlockPlaces<3> sh;
     const RunParams& P = W.R;
     const BatchHeader H = *P.hdr;
@@ -1335,8 +1334,12 @@ SKG_D void tail_path(const WaveParams& W, const DevGrid& g, const DevScene& S, i
     K.s_int = s; K.int_cell = -1; K.state = PK_INTERACT;
 }
 
+// (4 blocks per SM, 128 registers: 10^4 packets on a 40x40x20 grid 0.90 ms against 1.40 at 2 blocks, 1.15 at 3;
+// the Voronoi walk 9.9 ms at 3 against 12.9 at 4, 10^3 packets on 10^6 cells)
+template<template<typename> class Stepper> struct TailBlocks { static constexpr int value = 4; };
+template<> struct TailBlocks<VoronoiStepper> { static constexpr int value = 3; };
 template<typename R, template<typename> class Stepper>
-__global__ void __launch_bounds__(128) tail_kernel(const WaveParams W) {
+__global__ void __launch_bounds__(128, TailBlocks<Stepper>::value) tail_kernel(const WaveParams W) {
     const RunParams& P = W.R;
     // tail_lanes packets to a warp: few packets run side by side in few lanes, which then seldom
     // wait for one another's branches
@@ -1482,14 +1485,22 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
 }
 
 template<typename R, template<typename> class Stepper>
-cudaError_t enqueue_tail(const WaveParams& W, cudaStream_t s) {
+cudaError_t enqueue_tail(WaveParams W, cudaStream_t s) {
+    if (W.wave == 0) {                // the whole phase: spread the packets over the warps resident at once
+        static int per = 0;
+        if (per == 0) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tail_kernel<R, Stepper>, 128, 0);
+            per = std::max(per, 1);
+        }
+        W.tail_lanes = std::min(32, std::max(1, (W.npool + dev_sms() * per * 4 - 1) / (dev_sms() * per * 4)));
+    }
     const int warps = (W.npool + W.tail_lanes - 1) / W.tail_lanes;
     tail_kernel<R, Stepper><<<(warps + 3) / 4, 128, 0, s>>>(W);
     return cudaGetLastError();
 }
 
 using WaveFn = cudaError_t (*)(const WaveParams&, int, int, cudaEvent_t, cudaEvent_t, cudaStream_t);
-using TailFn = cudaError_t (*)(const WaveParams&, cudaStream_t);
+using TailFn = cudaError_t (*)(WaveParams, cudaStream_t);
 struct PassFns { WaveFn wave; TailFn tail; };
 
 template<typename R, template<typename> class Stepper, bool ONE = false>
@@ -1673,7 +1684,7 @@ cudaError_t WaveRunner::enqueue_tail() {
     W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = waves_;
     W.jobs = nullptr; W.jtau = nullptr; W.jL = nullptr; W.jcount = nullptr; W.jnext = nullptr;
     W.last_busy = ctr_ + 2 * J_N;
-    W.tail_lanes = waves_ ? 32 : std::min(32, std::max(1, npool_ / (dev_sms() * 16)));
+    W.tail_lanes = 32;
     W.freelist = nullptr; W.intlist = nullptr; W.freenext = nullptr; W.intnext = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
     W.hist = nullptr; W.bin0 = nullptr; W.jkey = nullptr; W.spath = nullptr; W.speel = nullptr;
     cudaError_t e;
