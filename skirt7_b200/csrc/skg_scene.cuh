@@ -189,6 +189,7 @@ struct WaveParams {
     int *freenext, *intnext;          // the next wave's
     int2* rlist;                      // the paths that interact: (packet, place in walk order) (J_REWALK)
     int tail_lanes;                   // tail pass: packets to a warp
+    int rewalk_lattice;               // octant walk: the re-walks on the lattice records
     int path_tau;                     // the path jobs need the optical depth alone (walked with the peel-offs)
     float4* ckpt;                     // per packet record: checkpoints of its path walk
     // walk order of the wave's jobs (order_kernel); hist == nullptr: as appended

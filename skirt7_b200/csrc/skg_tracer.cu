@@ -1478,7 +1478,18 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
         if (e != cudaSuccess) return e;
     }
     path_end_kernel<<<std::min(need, dev_sms() * 8), 256, 0, s>>>(W);
-    trav_kernel<R, Stepper, TRAV_REWALK, ONE><<<resident_blocks<R, Stepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
+    // On large trees the few cells of the re-walks come from the lattice records, one table for all
+    // directions: a wave's re-walks touch most of the eight octant tables once, and their records come
+    // from DRAM (2.9 GB per launch on the 3*10^6-leaf octree).  2*10^7 packets there 190 -> 186 ms a
+    // pass; 32 MB of records the same either way, a small octree 2.9 -> 3.0 ms.
+    if constexpr (std::is_same<Stepper<R>, TreeOctantStepper<float>>::value) {
+        if (W.rewalk_lattice) {
+            trav_kernel<float, TreeLatticeStepper, TRAV_REWALK, ONE>
+                <<<resident_blocks<float, TreeLatticeStepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
+        }
+    }
+    if (!W.rewalk_lattice)
+        trav_kernel<R, Stepper, TRAV_REWALK, ONE><<<resident_blocks<R, Stepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
     if (walked) cudaEventRecord(walked, s);
     detect_kernel<<<std::min(need * 2, dev_sms() * dper), 256, 0, s>>>(W);
     return cudaGetLastError();
@@ -1564,6 +1575,7 @@ static bool order_pays(int grid_type, size_t pool, size_t walk_bytes) {
 cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t walk_bytes) {
     cudaError_t e;
     const size_t had[5] = {cap_pool_, cap_ckpt_, cap_jobs_, cap_order_, bins_ != nullptr};
+    big_records_ = walk_bytes >= ((size_t)64 << 20);
     order_on_ = order_pays(grid_type, pool, walk_bytes);
     if (!ctr_) {
         if ((e = cudaMalloc(&ctr_, NCTR * sizeof(unsigned))) != cudaSuccess) return e;
@@ -1622,6 +1634,7 @@ cudaError_t WaveRunner::enqueue(int n) {
         W.freelist = lists_[b]; W.intlist = lists_[b] + npool_; W.freenext = lists_[b ^ 1]; W.intnext = lists_[b ^ 1] + npool_;
         W.rlist = rlist_; W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
         W.g0 = g0_;
+        W.rewalk_lattice = tree_walk_ == TW_OCTANT && grid_type_ != SKG_GRID_CARTESIAN && precision_ == SKG_PREC_FP32 && big_records_;
         W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
         // (a job's key lies where its optical depth will)
         W.jkey = reinterpret_cast<uint2*>(jtau_); W.speel = order_;
@@ -1686,6 +1699,7 @@ cudaError_t WaveRunner::enqueue_tail() {
     W.last_busy = ctr_ + 2 * J_N;
     W.tail_lanes = 32;
     W.freelist = nullptr; W.intlist = nullptr; W.freenext = nullptr; W.intnext = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+    W.rewalk_lattice = 0;
     W.hist = nullptr; W.bin0 = nullptr; W.jkey = nullptr; W.spath = nullptr; W.speel = nullptr;
     cudaError_t e;
     if (timed_) {

@@ -75,6 +75,7 @@ private:
     uint2* order_ = nullptr;          // peel-off jobs in walk order; at its end, the path jobs' packets
     size_t cap_order_ = 0;
     bool order_on_ = false;           // the running phase walks its jobs in spatial order
+    bool big_records_ = false;        // the walks' records of one direction exceed half the L2
     bool path_tau_ = false;
     static constexpr int NCTR = 2 * J_N + 1;
     unsigned* ctr_ = nullptr;         // [J_N (w & 1) + JobCount]: counters of wave w; [2 J_N]: last busy wave
