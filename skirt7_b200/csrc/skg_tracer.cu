@@ -23,10 +23,10 @@
 //                   re-walk of a path to the segment where the cumulative optical depth passes the
 //                   interaction optical depth, interpolating inside it (DustGridPath::pathlength,
 //                   DustGridPath.cpp:162-173);
-//   path_end_kernel between path and re-walk: escape fraction, termination test, sampling of the
-//                   interaction optical depth (simulatepropagation, :513-531); lists the next wave's
-//                   interacting packets and free records;
-//   detect_kernel   one thread per peel-off: the instruments' tallies.
+//   end_kernel      between the walks and the re-walks: per path the escape fraction, the termination
+//                   test and the sampling of the interaction optical depth (simulatepropagation, :513-531),
+//                   with the next wave's lists of interacting packets and free records; per peel-off the
+//                   instruments' tallies.
 // The traversal kernels hold nothing but the walk, so they keep few registers, no local memory and
 // a small instruction footprint; the divergent event code runs once per packet per wave in kernels
 // of its own.  Instruments seen from the same direction share one peel-off traversal
@@ -47,7 +47,7 @@ namespace skg {
 #define SKG_TRAV_MIN_BLOCKS 4
 #endif
 // The walks of a wave run in kernels of their own (TravMode below): each holds the registers of its
-// own state alone, and the path's long end (path_end_kernel) holds none of them.  Octree disk, 2*10^7
+// own state alone, and the path's long end (end_kernel) holds none of them.  Octree disk, 2*10^7
 // packets: traversal pass 179.6 ms against 209.8 with the end of the path and the re-walk inside the
 // path-job kernel (220 bytes of spills at 64 registers); fit-variant batch 46.2 against 53.5 ms.
 // blocks per SM of the path and re-walk kernels: 3 (80 registers, no spills) against 4 (64, spilling
@@ -655,8 +655,7 @@ SKG_D void sed_add(double* sed, int key, double v) {
 // phase against 26.5; Cartesian disk, 10^6, 2.40 against 1.25; a batch of 24 fit variants 35.1 against 30.6 ms in all) (Instrument::detect of every member of its
 // direction group; detect_group has the rules).  A launch of one simulation tallies its SED bins per
 // block and adds them once at the end.
-__global__ void __launch_bounds__(256) detect_kernel(const WaveParams W) {
-    __shared__ double s_sed[SED_PRIV];
+SKG_D void detect_peels(const WaveParams& W, double* s_sed) {
     const RunParams& P = W.R;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -947,8 +946,7 @@ SKG_D bool resume_ckpt(const WaveParams& W, const DevGrid& g, int p, int nck, do
 }
 
 // The walks of a wave, each in an instantiation that holds its own state alone:
-//   TRAV_PATH    the path jobs of phases that keep absorption or of several dust components (and, on
-//                steppers that resume, of every phase: they write checkpoints)
+//   TRAV_PATH    the path jobs of phases that keep absorption or of several dust components
 //   TRAV_TAU     jobs that need the optical depth alone: the peel-offs, and the path jobs otherwise
 //   TRAV_REWALK  the paths that interact, to the interaction optical depth
 enum TravMode : int { TRAV_PATH = 1, TRAV_TAU = 2, TRAV_REWALK = 3 };
@@ -1088,11 +1086,10 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                         }
                     } else {
                         st.init(g, w.x, w.y, w.z, w.kx, w.ky, w.kz, w.hint);
-                        if (MODE == TRAV_PATH || (job0 == 0 && j < (int)npath)) {
-                            if (w.hint == -2) W.pk[p].pos_cell = st.cell0;
-                        }
+                        nck = 0;
+                        if ((MODE == TRAV_PATH || j < (int)npath) && w.hint == -2) W.pk[p].pos_cell = st.cell0;
                         if (MODE == TRAV_PATH) {
-                            v1 = W.pk[p].L; v2 = 0; nck = 0;
+                            v1 = W.pk[p].L; v2 = 0;
                             const DevScene& S = *s_scene[slot];
                             labs = nullptr;
                             if (S.ncomp == 1 && (phase == SKG_PHASE_STELLAR ? S.store_abs != 0 : phase == SKG_PHASE_DUST_SELFABS)) {
@@ -1111,6 +1108,15 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
 
         const DevGrid& g = grid_of(slot);
         const DevScene& S = *s_scene[slot];
+        // a checkpoint of a path's walk every SKG_CKPT_STRIDE steps
+        auto checkpoint = [&](bool path) {
+            if constexpr (CKPT) {
+                if (path && W.ckpt && nck < SKG_CKPT_N && st.steps >= (nck + 1) * SKG_CKPT_STRIDE && !st.done) {
+                    save_ckpt(W, p, nck, st, tau);
+                    nck++;
+                }
+            }
+        };
         // cell steps: several of them before the warp looks at refills again.  (Walking
         // four steps ahead and loading their densities together, for the walks whose records do
         // not carry the density, was slower: Cartesian traversal pass 83 against 64 ms, Voronoi
@@ -1123,6 +1129,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                 const double dtau = step_dtau<R>(S, st, kext1, m, ell, ds);
                 if (MODE == TRAV_TAU) {
                     tau += dtau;
+                    if constexpr (CKPT) checkpoint(j < (int)npath);
                 } else if (MODE == TRAV_PATH) {
                     if (labs) {
                         const double Lintm = v1 * one_minus_exp(dtau);
@@ -1133,12 +1140,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                         c_abs += absorb_step<R>(S, phase, m, ell, dtau, v1, v2);
                     }
                     tau += dtau;
-                    if constexpr (CKPT) {
-                        if (W.ckpt && nck < SKG_CKPT_N && st.steps >= (nck + 1) * SKG_CKPT_STRIDE && !st.done) {
-                            save_ckpt(W, p, nck, st, tau);
-                            nck++;
-                        }
-                    }
+                    if constexpr (CKPT) checkpoint(true);
                 } else {
                     const double tn = tau + dtau, sn = v1 + (double)ds;
                     if (tn > v2) {
@@ -1162,7 +1164,8 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
                     K.s_int = v1; K.int_cell = -1; K.state = PK_INTERACT;
                 } else {
                     W.jtau[j] = tau;
-                    if (MODE == TRAV_PATH) { W.jL[j] = v2; if (CKPT) W.pk[p].nck = nck; }
+                    if (MODE == TRAV_PATH) W.jL[j] = v2;
+                    if (CKPT && (MODE == TRAV_PATH || j < (int)npath)) W.pk[p].nck = nck;
                 }
                 j = -1;
                 break;
@@ -1188,10 +1191,9 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
 // The ends of the wave's paths, one thread per path job in walk order: escape fraction, termination
 // test and interaction optical depth (after_path).  The packets that interact go on the re-walk list
 // and on the next wave's interaction list, the records of the others on its free list.
-// In a kernel of its own every lane of a warp does this long FP64 work at once, and the walks need
-// no registers for it.
-__global__ void __launch_bounds__(256) path_end_kernel(const WaveParams W) {
-    __shared__ BlockPlaces<3> sh;
+// Outside the walks every lane of a warp does this long FP64 work at once, and the walks need no
+// registers for it.
+SKG_D void end_paths(const WaveParams& W, BlockPlaces<3>& sh) {
     const RunParams& P = W.R;
     const unsigned n = W.jcount[J_PATH];
     const int phase = P.hdr->phase;
@@ -1220,6 +1222,15 @@ __global__ void __launch_bounds__(256) path_end_kernel(const WaveParams W) {
         if (inter) W.intnext[place[1]] = p;
         else if (i < n) W.freenext[place[2]] = p;
     }
+}
+
+// The ends of the paths and the detections of a wave in one launch, after its walks (as two, a batch of
+// 24 fit variants 27.3 against 26.4 ms, an octree phase of 2.4*10^5 packets 2.92 against 2.83).
+__global__ void __launch_bounds__(256) end_kernel(const WaveParams W) {
+    __shared__ BlockPlaces<3> sh;
+    __shared__ double s_sed[SED_PRIV];
+    end_paths(W, sh);
+    detect_peels(W, s_sed);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1441,14 +1452,14 @@ int resident_blocks(size_t smem) {
 }
 
 template<typename R, template<typename> class Stepper, bool ONE>
-cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaEvent_t mid, cudaEvent_t walked, cudaStream_t s) {
+cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaEvent_t mid, cudaStream_t s) {
     const size_t smem = (size_t)nslots * sizeof(DevGrid);
     const int need = (W.npool + 255) / 256;
     // grid-stride passes over at most the blocks resident at once
     static int lper = 0, dper = 0;
     if (lper == 0) {
         int d = 0, l = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, detect_kernel, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, end_kernel, 256, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l, launch_kernel<R>, 256, 0);
         dper = std::max(d, 1); lper = std::max(l, 1);
     }
@@ -1477,7 +1488,7 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
         cudaError_t e = cudaLaunchKernelEx(&cfg, trav_kernel<R, Stepper, TRAV_TAU, ONE>, W);
         if (e != cudaSuccess) return e;
     }
-    path_end_kernel<<<std::min(need, dev_sms() * 8), 256, 0, s>>>(W);
+    end_kernel<<<std::min(need, dev_sms() * dper), 256, 0, s>>>(W);
     // On large trees the few cells of the re-walks come from the lattice records, one table for all
     // directions: a wave's re-walks touch most of the eight octant tables once, and their records come
     // from DRAM (2.9 GB per launch on the 3*10^6-leaf octree).  2*10^7 packets there 190 -> 186 ms a
@@ -1490,8 +1501,6 @@ cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaE
     }
     if (!W.rewalk_lattice)
         trav_kernel<R, Stepper, TRAV_REWALK, ONE><<<resident_blocks<R, Stepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
-    if (walked) cudaEventRecord(walked, s);
-    detect_kernel<<<std::min(need * 2, dev_sms() * dper), 256, 0, s>>>(W);
     return cudaGetLastError();
 }
 
@@ -1510,7 +1519,7 @@ cudaError_t enqueue_tail(WaveParams W, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-using WaveFn = cudaError_t (*)(const WaveParams&, int, int, cudaEvent_t, cudaEvent_t, cudaStream_t);
+using WaveFn = cudaError_t (*)(const WaveParams&, int, int, cudaEvent_t, cudaStream_t);
 using TailFn = cudaError_t (*)(WaveParams, cudaStream_t);
 struct PassFns { WaveFn wave; TailFn tail; };
 
@@ -1641,16 +1650,15 @@ cudaError_t WaveRunner::enqueue(int n) {
         W.spath = reinterpret_cast<int*>(order_ + (cap_order_ - npool_));
         if ((e = cudaMemsetAsync(ctr_ + J_N * (b ^ 1), 0, J_N * sizeof(unsigned), stream_)) != cudaSuccess) return e;
         if (timed_) {
-            while (ev_.size() < 4 * (size_t)(w + 1)) {
+            while (ev_.size() < 3 * (size_t)(w + 1)) {
                 cudaEvent_t x;
                 if ((e = cudaEventCreate(&x)) != cudaSuccess) return e;
                 ev_.push_back(x);
             }
-            if ((e = cudaEventRecord(ev_[4 * w], stream_)) != cudaSuccess) return e;
+            if ((e = cudaEventRecord(ev_[3 * w], stream_)) != cudaSuccess) return e;
         }
-        if ((e = fn(W, nslots_, trav_blocks_, timed_ ? ev_[4 * w + 1] : nullptr, timed_ ? ev_[4 * w + 2] : nullptr, stream_)) !=
-            cudaSuccess) return e;
-        if (timed_ && (e = cudaEventRecord(ev_[4 * w + 3], stream_)) != cudaSuccess) return e;
+        if ((e = fn(W, nslots_, trav_blocks_, timed_ ? ev_[3 * w + 1] : nullptr, stream_)) != cudaSuccess) return e;
+        if (timed_ && (e = cudaEventRecord(ev_[3 * w + 2], stream_)) != cudaSuccess) return e;
     }
     waves_ += n;
     if ((e = cudaMemcpyAsync(h_ctr_, ctr_, NCTR * sizeof(unsigned), cudaMemcpyDeviceToHost, stream_)) != cudaSuccess) return e;
@@ -1676,7 +1684,7 @@ cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, 
     trav_blocks_ = trav_blocks; stream_ = s; npool_ = (int)npool; waves_ = 0; tail_ran_ = false;
     const char* td = std::getenv("SKG_TAIL_DIV");
     tail_div_ = td ? std::atoi(td) : tail_div;
-    path_tau_ = !absorbs && !(precision == SKG_PREC_FP32 && ckpt_grid(grid_type));
+    path_tau_ = !absorbs;
     const char* ck = std::getenv("SKG_CKPT");
     ckpt_on_ = !(ck && std::atoi(ck) == 0) && ckpt_ && cap_ckpt_ >= (size_t)npool;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1760,12 +1768,10 @@ cudaError_t WaveRunner::times(float* event_ms, float* trav_ms) const {
     if (timed_ && !pending_) {
         for (int w = 0; w < waves_; w++) {
             float x = 0, y = 0;
-            cudaError_t e = cudaEventElapsedTime(&x, ev_[4 * w], ev_[4 * w + 1]);
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&y, ev_[4 * w + 1], ev_[4 * w + 2]);
+            cudaError_t e = cudaEventElapsedTime(&x, ev_[3 * w], ev_[3 * w + 1]);
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&y, ev_[3 * w + 1], ev_[3 * w + 2]);
             if (e != cudaSuccess) return e;
             a += x; t += y;
-            if ((e = cudaEventElapsedTime(&x, ev_[4 * w + 2], ev_[4 * w + 3])) != cudaSuccess) return e;
-            a += x;
         }
         if (tail_ran_) {
             float y = 0;

@@ -2,7 +2,7 @@
 //
 // A phase runs as a sequence of waves on one stream.  Wave w: a launch pass (scatter the packets that
 // the previous wave brought to their interaction point, launch new packets into the records that it freed, and write the
-// next traversals as jobs), the walks of every job, and a detection pass over the peel-offs.
+// next traversals as jobs), the walks of every job, their ends (escape, termination, detection) and the re-walks.
 // The number of waves is not known in advance: begin() enqueues an estimate, finish() reads how many
 // packets still had work in the last enqueued wave and enqueues more until none has -- or, once few
 // have, the tail pass, which finishes every remaining packet in one launch.  Phases of few packets
@@ -91,7 +91,7 @@ private:
     int tree_walk_ = TW_ROPE;
     int npool_ = 0;
     int waves_ = 0;
-    std::vector<cudaEvent_t> ev_;      // 4 per wave: before the launch pass, the walks, the detection, and after it
+    std::vector<cudaEvent_t> ev_;      // 3 per wave: before the launch pass, before the walks, after the ends and re-walks
     bool timed_ = false;               // the running phase records ev_
     int tail_div_ = 16;
     bool ckpt_on_ = true;              // path-walk checkpoints (environment variable SKG_CKPT=0: off)
