@@ -75,13 +75,14 @@ namespace skg {
 #define SKG_CKPT 1
 #endif
 // cell steps a lane takes per pass of the traversal loop (the warp's refill vote runs once per
-// pass): optical-depth and re-walk kernels, path kernel.  Octree disk, 2*10^7 packets, traversal pass
-// at 3 and 5: 162.3 and 156.8 ms; Cartesian disk 7.30 and 7.19, k-d tree disk 23.4 and 22.7 ms
+// pass): optical-depth and re-walk kernels, path kernel.  2*10^7 packets of the octree disk, ms per pass
+// at 5 and 4, 8 and 6, 12 and 8, 16 and 12: 185.3, 180.8, 178.1, 177.9; fit-variant batch 26.4, 25.9, 26.0,
+// 26.1 (device); k-d tree disk with absorption 25.4, 24.9, 24.6, 24.5; Voronoi disk 132.7, 132.2, 132.6, 131.2
 #ifndef SKG_INNER_STEPS
-#define SKG_INNER_STEPS 5
+#define SKG_INNER_STEPS 12
 #endif
 #ifndef SKG_INNER_PATH
-#define SKG_INNER_PATH 4
+#define SKG_INNER_PATH 8
 #endif
 #ifndef SKG_CKPT_N
 #define SKG_CKPT_N 32
@@ -1121,7 +1122,10 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
         // four steps ahead and loading their densities together, for the walks whose records do
         // not carry the density, was slower: Cartesian traversal pass 83 against 64 ms, Voronoi
         // peel-off walks 298 against 258 ms; the walk is issue-bound, not waiting on those loads.)
-#pragma unroll 1
+#ifndef SKG_UR
+#define SKG_UR 1
+#endif
+#pragma unroll SKG_UR
         for (int is = 0; is < (MODE == TRAV_PATH ? SKG_INNER_PATH : SKG_INNER_STEPS); is++) {
             int m; R ds;
             if (st.walk(g, m, ds)) {
