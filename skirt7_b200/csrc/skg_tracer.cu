@@ -1122,10 +1122,7 @@ __global__ void __launch_bounds__(256, (TravBlocks<MODE, Stepper>::value)) trav_
         // four steps ahead and loading their densities together, for the walks whose records do
         // not carry the density, was slower: Cartesian traversal pass 83 against 64 ms, Voronoi
         // peel-off walks 298 against 258 ms; the walk is issue-bound, not waiting on those loads.)
-#ifndef SKG_UR
-#define SKG_UR 1
-#endif
-#pragma unroll SKG_UR
+#pragma unroll 1
         for (int is = 0; is < (MODE == TRAV_PATH ? SKG_INNER_PATH : SKG_INNER_STEPS); is++) {
             int m; R ds;
             if (st.walk(g, m, ds)) {
