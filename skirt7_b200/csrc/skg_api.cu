@@ -214,7 +214,8 @@ DevGrid make_grid(Allocs& A, const skg_grid& g, cudaStream_t s) {
         // rope-linked tree for the FP32 walk
         {
             RopeTree rt;
-            // SKG_TREE_RECORDS=rope keeps the 64-byte leaf records for trees that fit the lattice
+            // SKG_TREE_RECORDS=rope keeps the 64-byte leaf records for trees that fit the lattice,
+            // =lattice the lattice records without the octant records
             const char* rec = std::getenv("SKG_TREE_RECORDS");
             build_rope_tree(g, rt, !(rec && std::strcmp(rec, "rope") == 0));
             if (rt.lattice) {
@@ -534,7 +535,9 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
         }
 
         // octant records of the FP32 walk (256 bytes per cell; without them it takes the lattice records)
-        if (ctx->grid.lattice && ctx->grid.search != SKG_SEARCH_BOOKKEEPING && nc <= (1 << 27)) {
+        const char* kind = std::getenv("SKG_TREE_RECORDS");
+        if (ctx->grid.lattice && ctx->grid.search != SKG_SEARCH_BOOKKEEPING && nc <= (1 << 27) &&
+            !(kind && std::strcmp(kind, "lattice") == 0)) {
             uint4* rec = A.alloc<uint4>(16 * (size_t)nc);
             if (rec) { CK(launch_octant_records(ctx->grid, rec, s)); ctx->grid.orec = rec; }
         }
@@ -745,7 +748,7 @@ int skg_sync(skg_ctx* ctx, int timeout_ms) {
             if (e != cudaErrorNotReady) { cudaGetLastError(); return fail(ctx, Failure{SKG_ERR_CUDA, cudaGetErrorString(e)}); }
             if (timeout_ms >= 0 && std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count() > timeout_ms)
                 return fail(ctx, Failure{SKG_ERR_TIMEOUT, "timed out waiting for the device"});
-            std::this_thread::sleep_for(std::chrono::microseconds(200));
+            wait_a_little(t0, 200);
         }
     }
     ctx->hev_pending = false;
@@ -1416,7 +1419,7 @@ int skg_batch_sync(skg_batch* b, int timeout_ms) {
         if (e != cudaErrorNotReady) { cudaGetLastError(); return bfail(b, Failure{SKG_ERR_CUDA, cudaGetErrorString(e)}); }
         if (timeout_ms >= 0 && std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count() > timeout_ms)
             return bfail(b, Failure{SKG_ERR_TIMEOUT, "timed out waiting for the device"});
-        std::this_thread::sleep_for(std::chrono::microseconds(100));
+        wait_a_little(t0, 100);
     }
     unsigned err = 0;
     cudaMemcpy(&err, b->T.err, sizeof(unsigned), cudaMemcpyDeviceToHost);

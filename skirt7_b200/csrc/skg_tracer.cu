@@ -1736,7 +1736,7 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
                 if (timed_out) *timed_out = true;
                 return cudaSuccess;
             }
-            std::this_thread::sleep_for(std::chrono::microseconds(50));
+            wait_a_little(t0, 50);
         }
         if (tail_only_) { pending_ = false; break; }
         // packets with jobs in the last wave (without dust a packet has peel-offs alone)
