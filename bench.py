@@ -11,7 +11,7 @@ other configurations of the hot path with the same machinery:
                     cycles and the dust-emission phase (emission spectra recomputed before
                     each dust phase)
 
-One step = the workload's phases (a sequence of waves: an event pass and a traversal pass each)
+One step = the workload's phases (a sequence of waves: a launch pass and a traversal pass each)
 over all wavelengths with --packets packets per wavelength per GPU (by default the
 configuration's count: 10^7, 10^8 for the Voronoi workload).  A step ends when its phases have finished (the host has seen the last
 wave's counters), so every step times exactly its own waves.  Ranks (one process per GPU; with
@@ -566,16 +566,16 @@ def main():
                          "traffic_basis": ("scaled, not measured in this run: ncu DRAM bytes per cell step of "
                                            "this workload's traversal pass (%.2f B, one capture of a stellar "
                                            "phase) x this launch's cell steps" % bps) if bps else None,
-                         "kernel": "trav_kernel, path and peel-off instantiations (traversal pass of the stellar phase)",
-                         "launch": "one traversal pass of a wave (its path-job and peel-off-job kernels)",
+                         "kernel": "trav_kernel instantiations and end_kernel (traversal pass of the stellar phase)",
+                         "launch": "one traversal pass of a wave (walks, ends of paths, detections, re-walks)",
                          "algorithmic_bytes_per_launch": alg_bytes / max(waves, 1),
                          "kernel_ms_per_launch": trav_ms / max(waves, 1), "launches_per_phase": waves,
                          "phase_ms": kms, "event_pass_ms": ev_ms, "traversal_pass_ms": trav_ms},
             "e2e": {"value": e2e, "unit": "packets/s", "h2d_bytes_per_step": len(phases) * (4 * nl + 64),
                     "d2h_bytes_per_step": cubes_bytes, "steps": e2e_steps},
-            # per wave: the event pass, the scatter-and-launch pass and the two traversal kernels
-            # (path jobs, peel-off jobs)
-            "gpu_launches": 4 * waves * len(phases) * args.steps,
+            # per wave: the scatter-and-launch pass, the optical depths, the ends, the re-walks, and on
+            # the tree and Voronoi workloads the three kernels of the walk order
+            "gpu_launches": (4 if wl.gtype == "CartesianDustGrid" else 7) * waves * len(phases) * args.steps,
             "clocks": clk,
             "counters_stellar_phase": c,
         }

@@ -235,7 +235,7 @@ typedef struct skg_counters {
     uint64_t nbr_scanned;                   /* neighbour-list entries scanned (tree/Voronoi) */
     uint64_t fallbacks;                     /* neighbour search fallbacks / re-locations */
     uint64_t errors;                        /* packets retired on a budget or NaN */
-    uint64_t waves;                         /* waves (event pass + traversal pass) of the phase */
+    uint64_t waves;                         /* waves (launch pass + traversal pass) of the phase */
 } skg_counters;
 
 typedef struct skg_ctx skg_ctx;
@@ -421,9 +421,9 @@ int  skg_read_counters(skg_ctx* ctx, skg_counters* out);
 int  skg_sync(skg_ctx* ctx, int timeout_ms);
 /* Device time (ms) of the last skg_run_phase launch (CUDA events on the launching stream). */
 int  skg_last_phase_ms(skg_ctx* ctx, float* ms);
-/* The last phase split by kernel: summed device time (ms) of its event passes (launch, detection,
-   scattering) and of its traversal passes, and its number of waves (each wave is one launch of
-   each).  Finishes the phase first. */
+/* The last phase split by pass: summed device time (ms) of its launch passes (scatterings, launches,
+   walk order) and of its traversal passes (walks, ends of paths, detections, re-walks, the tail pass),
+   and its number of waves (0: the tail pass alone, which small phases are).  Finishes the phase first. */
 int  skg_phase_times(skg_ctx* ctx, float* event_ms, float* traversal_ms, int32_t* waves);
 
 /* ---- dust emission (PanDustSystem::calculatedustemission / DustLib::calculate) --------- */

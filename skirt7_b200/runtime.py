@@ -118,7 +118,8 @@ class Context:
         return ms.value
 
     def phase_times(self):
-        """(event_ms, traversal_ms, waves) of the last phase: summed device time of its two kernels."""
+        """(event_ms, traversal_ms, waves) of the last phase: summed device time of its launch
+        passes and of its traversal passes (waves 0: the tail pass alone)."""
         a, b, w = C.c_float(), C.c_float(), C.c_int32()
         self._ck(self.lib.skg_phase_times(self.h, C.byref(a), C.byref(b), C.byref(w)))
         return a.value, b.value, w.value
