@@ -234,7 +234,7 @@ class Workload:
     # (dram__bytes_read.sum + dram__bytes_write.sum over the traversal launches of a stellar phase
     # of this workload, divided by that phase's cell steps); roofline.traffic scales it by a
     # launch's cell steps, and says so.  Other workloads report no traffic.
-    NCU_DRAM_BYTES_PER_STEP = {"octree_pan": 11.76}
+    NCU_DRAM_BYTES_PER_STEP = {"octree_pan": 9.69}
 
     def frames(self):
         from skirt7_b200 import _abi as A
