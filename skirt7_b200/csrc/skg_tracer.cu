@@ -1608,7 +1608,6 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t 
     }
     if (order_on_ && !bins_) {
         if ((e = cudaMalloc(&bins_, (4 * (size_t)JOB_BINS + 1024) * sizeof(unsigned))) != cudaSuccess) return e;
-        if ((e = cudaMemset(bins_, 0, 4 * JOB_BINS * sizeof(unsigned))) != cudaSuccess) return e;
     }
     const size_t jobs = pool * (size_t)(ngroups + 1);
     if (jobs > cap_jobs_) {
@@ -1693,6 +1692,9 @@ cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, 
     timed_ = timing && cs == cudaStreamCaptureStatusNone;
     cudaError_t e;
     if ((e = cudaMemsetAsync(ctr_, 0, NCTR * sizeof(unsigned), s)) != cudaSuccess) return e;
+    // (the waves leave the counts of the bins at zero; cleared here, on the phase's stream, for the first and for
+    // one that follows a failed phase)
+    if (order_on_ && (e = cudaMemsetAsync(bins_, 0, 2 * JOB_BINS * sizeof(unsigned), s)) != cudaSuccess) return e;
     pending_ = true;
     tail_only_ = tail_div_ > 0 && fits && npool <= (size_t)(grid_type == SKG_GRID_CARTESIAN ? SKG_TAIL_ONLY_CART : SKG_TAIL_ONLY);
     if (!tail_only_) return enqueue(estimate);
