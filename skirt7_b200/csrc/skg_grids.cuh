@@ -458,10 +458,11 @@ struct CartUniStepper<float> {
             c0 = (org - o) * u; dt = h * u;
             q = (float)(k < 0.f ? c : c + 1);
             tn = fmaf(q, dt, c0);
-            end = fminf(end, fmaf(k < 0.f ? 0.f : (float)n, dt, c0));
-        } else {
-            c0 = 0.f; dt = 0.f; q = 0.f; tn = FLT_MAX;
+            const float te = fmaf(k < 0.f ? 0.f : (float)n, dt, c0);
+            if (fabsf(c0) <= FLT_MAX && fabsf(tn) <= FLT_MAX && fabsf(te) <= FLT_MAX) { end = fminf(end, te); return; }
         }
+        // never crossed (nor an axis whose parameters leave FP32's range: boxes of 10^24 m at |k| of 10^-15)
+        c0 = 0.f; dt = 0.f; q = 0.f; tn = FLT_MAX;
     }
     SKG_D void init(const DevGrid& g, float rx, float ry, float rz, float dx, float dy, float dz, int hint = -1) {
         CartStepperRef<float> e;
@@ -469,12 +470,11 @@ struct CartUniStepper<float> {
         pd = e.pd; done = e.done; steps = 0; cell0 = e.cell0;
         tc = 0.f;
         if (done) return;
-        if (isnan(dx) || isnan(dy) || isnan(dz)) { done = true; return; }   // the reference walk stops
+        if (isnan(dx) || isnan(dy) || isnan(dz) || isnan(e.x) || isnan(e.y) || isnan(e.z)) { done = true; return; }   // the reference walk stops
         tend = FLT_MAX;
         axis(g.corg[0], g.cstep[0], e.x, dx, e.i, g.nx, cx, dtx, qx, tx, tend);
         axis(g.corg[1], g.cstep[1], e.y, dy, e.j, g.ny, cy, dty, qy, ty, tend);
         axis(g.corg[2], g.cstep[2], e.z, dz, e.k, g.nz, cz, dtz, qz, tz, tend);
-        if (!(fabsf(tx) <= FLT_MAX && fabsf(ty) <= FLT_MAX && fabsf(tz) <= FLT_MAX)) done = true;
         mz = dz < 0.f ? -1 : 1;
         my = dy < 0.f ? -g.nz : g.nz;
         mx = (dx < 0.f ? -g.nz : g.nz) * g.ny;
