@@ -651,11 +651,12 @@ SKG_D void sed_add(double* sed, int key, double v) {
     }
 }
 
-// Detection pass: one thread per peel-off job of the wave, right after its walks (a pass over all records of the pool in
-// the next wave before, with the records' lists: event and launch passes of the octree disk, 2*10^7 packets, 35.4 ms a
-// phase against 26.5; Cartesian disk, 10^6, 2.40 against 1.25; a batch of 24 fit variants 35.1 against 30.6 ms in all) (Instrument::detect of every member of its
-// direction group; detect_group has the rules).  A launch of one simulation tallies its SED bins per
-// block and adds them once at the end.
+// Detection: one thread per peel-off job of the wave, right after its walks (Instrument::detect of every
+// member of its direction group; detect_group has the rules).  A launch of one simulation tallies its
+// SED bins per block and adds them once at the end.  (A pass over all records of the pool in the next wave
+// before, which also made the record lists: event and launch passes of the octree disk, 2*10^7 packets,
+// 35.4 ms a phase against 26.5; Cartesian disk, 10^6, 2.40 against 1.25; a batch of 24 fit variants 35.1
+// against 30.6 ms in all.)
 SKG_D void detect_peels(const WaveParams& W, double* s_sed) {
     const RunParams& P = W.R;
     const unsigned FULL = 0xffffffffu;
@@ -846,9 +847,9 @@ SKG_D double one_minus_exp(double x) {
 // Absorption in cell m of a path step: simulateescapeandabsorption (MonteCarloSimulation.cpp:441-462)
 // with OligoDustSystem::absorb / PanDustSystem::absorb.  The tables are wavelength-major on the
 // device ([ell][m]): a wave carries the packets of one or two wavelengths (packets are handed out
-// wavelength by wavelength), so its tallies fall in one slice of the table that stays in L2.  v1 = L e^-tau on entry (a running product,
-// each step absorbs v1 (1 - e^-dtau)); v2 accumulates L_sca with
-// the local albedo when there are several dust components.  Returns 1 when a tally was stored.
+// wavelength by wavelength), so its tallies fall in one slice of the table that stays in L2.
+// v1 = L e^-tau on entry (a running product, each step absorbs v1 (1 - e^-dtau)); v2 accumulates L_sca
+// with the local albedo when there are several dust components.  Returns 1 when a tally was stored.
 template<typename R>
 SKG_D int absorb_step(const DevScene& S, int phase, int m, int ell, double dtau, double& v1, double& v2) {
     if (m < 0) return 0;
@@ -1577,7 +1578,8 @@ static bool ckpt_grid(int grid_type) {
 // a 3*10^6-leaf octree (96 MB of records) 306 against 293 ms, of 2*10^6 on 10^6 Voronoi cells (512 MB)
 // 262 against 254 ms, of 10^6 on the octree 20.7 against 18.3, on
 // Voronoi cells 100 against 93, on a 10^6-leaf k-d tree 12.9 against 12.6; below these bounds the sort costs more than it gives
-// (2.4*10^5 packets on a small octree 4.1 against 4.7 ms, 6*10^5 on the k-d tree 9.4 against 9.6; Cartesian densities are a few MB: a batch of 24 fit variants 53.5 against 56.2 ms).
+// (2.4*10^5 packets on a small octree 4.1 against 4.7 ms, 6*10^5 on the k-d tree 9.4 against 9.6; Cartesian
+// densities are a few MB: a batch of 24 fit variants 53.5 against 56.2 ms).
 static bool order_pays(int grid_type, size_t pool, size_t walk_bytes) {
     return grid_type != SKG_GRID_CARTESIAN && pool >= ((size_t)3 << 18) && pool < ((size_t)1 << 28) && walk_bytes >= ((size_t)8 << 20);
 }
@@ -1643,7 +1645,8 @@ cudaError_t WaveRunner::enqueue(int n) {
         W.freelist = lists_[b]; W.intlist = lists_[b] + npool_; W.freenext = lists_[b ^ 1]; W.intnext = lists_[b ^ 1] + npool_;
         W.rlist = rlist_; W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
         W.g0 = g0_;
-        W.rewalk_lattice = tree_walk_ == TW_OCTANT && grid_type_ != SKG_GRID_CARTESIAN && precision_ == SKG_PREC_FP32 && big_records_;
+        W.rewalk_lattice = tree_walk_ == TW_OCTANT && grid_type_ != SKG_GRID_CARTESIAN &&
+                           precision_ == SKG_PREC_FP32 && big_records_;
         W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
         // (a job's key lies where its optical depth will)
         W.jkey = reinterpret_cast<uint2*>(jtau_); W.speel = order_;
