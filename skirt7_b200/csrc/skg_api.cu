@@ -1204,7 +1204,7 @@ struct skg_batch {
     int* h_ells = nullptr;
     cudaEvent_t copied = nullptr;          // the previous launch's tables have been read
     cudaGraphExec_t graph = nullptr;
-    int g_type = -1, g_bk = -1, g_prec = -1, g_blocks = -1, g_gen = -1;
+    int g_type = -1, g_bk = -1, g_prec = -1, g_blocks = -1, g_gen = -1, g_slots = -1;
     size_t g_npool = 0;
     bool g_absorbs = false, g_fits = false;
     int g_waves = 0;                       // waves captured in the graph
@@ -1365,6 +1365,13 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
         REQUIRE(!opts || (opts->refill >= 0 && opts->refill <= 32), "refill lanes must be in 0..32");
         RunParams P = b->T.params((opts && opts->max_scatt > 0) ? opts->max_scatt : 100000, opts ? opts->refill : 0);
         Staging& T = b->T;
+        // the walks keep the DevGrid of every slot in shared memory, at the cost of L1: room for the slots of
+        // this launch, in a captured one up to the next power of two (it serves launches of no more slots)
+        int gslots = nslots;
+        if (flags & SKG_BATCH_GRAPH) {
+            gslots = 1;
+            while (gslots < nslots) gslots <<= 1;
+        }
         auto enqueue = [&](cudaStream_t q) {
             CK(cudaMemcpyAsync(T.hdr, b->h_hdr, sizeof(BatchHeader), cudaMemcpyHostToDevice, q));
             CK(cudaMemcpyAsync(T.items, b->h_items, T.max_items * sizeof(WorkItem), cudaMemcpyHostToDevice, q));
@@ -1373,13 +1380,12 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
             CK(cudaMemcpyAsync(T.ells, b->h_ells, T.max_ells * sizeof(int), cudaMemcpyHostToDevice, q));
             CK(cudaMemsetAsync(T.work, 0, sizeof(unsigned long long), q));
             CK(cudaMemsetAsync(T.err, 0, sizeof(unsigned), q));
-            // every slot's DevGrid is copied into shared memory: size for the batch's capacity
-            CK(b->waves.begin(P, gtype < 0 ? SKG_GRID_CARTESIAN : gtype, gbk < 0 ? TW_ROPE : gbk, precision, T.max_slots, npool,
+            CK(b->waves.begin(P, gtype < 0 ? SKG_GRID_CARTESIAN : gtype, gbk < 0 ? TW_ROPE : gbk, precision, gslots, npool,
                               total <= npool, blocks, absorbs, q));
         };
         CK(cudaEventRecord(b->ev0, s));
         if (flags & SKG_BATCH_GRAPH) {
-            bool same = b->graph && !b->g_stale && b->g_absorbs == absorbs && b->g_fits == (total <= npool) &&
+            bool same = b->graph && !b->g_stale && b->g_slots >= gslots && b->g_absorbs == absorbs && b->g_fits == (total <= npool) &&
                         b->g_gen == b->waves.generation() && b->g_type == gtype && b->g_bk == gbk && b->g_prec == precision &&
                         b->g_blocks == blocks && b->g_npool == npool;
             if (!same) {
@@ -1393,7 +1399,7 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
                 cudaGraphDestroy(gr);
                 CK(e);
                 b->g_type = gtype; b->g_bk = gbk; b->g_prec = precision; b->g_blocks = blocks; b->g_npool = npool;
-                b->g_absorbs = absorbs; b->g_fits = total <= npool; b->g_gen = b->waves.generation();
+                b->g_slots = gslots; b->g_absorbs = absorbs; b->g_fits = total <= npool; b->g_gen = b->waves.generation();
                 b->g_waves = b->waves.waves(); b->g_stale = false;
             }
             CK(cudaGraphLaunch(b->graph, s));

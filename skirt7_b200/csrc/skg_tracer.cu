@@ -39,7 +39,10 @@
 
 #include <chrono>
 #include <cstdlib>
+#include <map>
+#include <mutex>
 #include <thread>
+#include <tuple>
 
 namespace skg {
 
@@ -1429,92 +1432,102 @@ __global__ void __launch_bounds__(128, TailBlocks<Stepper>::value) tail_kernel(c
 
 namespace {
 
-int dev_sms() {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
-    return sms;
+// SMs of the current device and the blocks of a kernel that are resident on it at once, for `smem`
+// bytes of dynamic shared memory.  Above the 48 KB a kernel has by default (static and dynamic: the
+// staged jobs and the grids of 58 and more slots on an FP64 walk) it is allowed them first.  Kept per
+// device, kernel and size; a query that fails is reported and not kept.
+struct Resident { int sms = 0, blocks = 0; };
+cudaError_t resident(const void* kernel, int threads, size_t smem, Resident& out) {
+    static std::mutex lock;
+    static std::map<std::tuple<int, const void*, size_t>, Resident> known;
+    int dev = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    std::lock_guard<std::mutex> hold(lock);
+    const auto key = std::make_tuple(dev, kernel, smem);
+    const auto it = known.find(key);
+    if (it != known.end()) { out = it->second; return cudaSuccess; }
+    cudaFuncAttributes attr;
+    if ((e = cudaFuncGetAttributes(&attr, kernel)) != cudaSuccess) return e;
+    if (smem > (size_t)std::max(attr.maxDynamicSharedSizeBytes, 0) &&
+        (e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    Resident r;
+    int per = 0;
+    if ((e = cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem)) != cudaSuccess) return e;
+    if (per <= 0) return cudaErrorLaunchOutOfResources;
+    r.blocks = r.sms * per;
+    known[key] = r;
+    out = r;
+    return cudaSuccess;
 }
 
-// Resident blocks of a traversal instantiation (persistent grid = this many blocks per SM x SMs).
+// A traversal instantiation: persistent, so its blocks resident at once (or `blocks`, if given).  pdl: as a
+// programmatic dependent of the kernel before it.
 template<typename R, template<typename> class Stepper, int MODE, bool ONE>
-int resident_blocks(size_t smem) {
-    static int per = 0, sms = 0;
-    if (per == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, trav_kernel<R, Stepper, MODE, ONE>, 256, smem);
-        if (per <= 0) per = 1;
-    }
-    return sms * per;
+cudaError_t launch_trav(const WaveParams& W, size_t smem, int blocks, bool pdl, cudaStream_t s) {
+    Resident r;
+    cudaError_t e = resident((const void*)trav_kernel<R, Stepper, MODE, ONE>, 256, smem, r);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks > 0 ? blocks : r.blocks);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? SKG_PDL : 0;
+    return cudaLaunchKernelEx(&cfg, trav_kernel<R, Stepper, MODE, ONE>, W);
 }
 
+// One wave: its kernels in order, none behind one that could not be launched (the ends of paths would
+// tally optical depths that no walk wrote).
 template<typename R, template<typename> class Stepper, bool ONE>
 cudaError_t enqueue_wave(const WaveParams& W, int nslots, int trav_blocks, cudaEvent_t mid, cudaStream_t s) {
     const size_t smem = (size_t)nslots * sizeof(DevGrid);
     const int need = (W.npool + 255) / 256;
     // grid-stride passes over at most the blocks resident at once
-    static int lper = 0, dper = 0;
-    if (lper == 0) {
-        int d = 0, l = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, end_kernel, 256, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l, launch_kernel<R>, 256, 0);
-        dper = std::max(d, 1); lper = std::max(l, 1);
-    }
-    launch_kernel<R><<<std::min(need, dev_sms() * lper), 256, 0, s>>>(W);
+    cudaError_t e;
+    Resident l, d;
+    if ((e = resident((const void*)launch_kernel<R>, 256, 0, l)) != cudaSuccess) return e;
+    if ((e = resident((const void*)end_kernel, 256, 0, d)) != cudaSuccess) return e;
+    launch_kernel<R><<<std::min(need, l.blocks), 256, 0, s>>>(W);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (W.hist) {
         bin_sums_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0 + 2 * JOB_BINS);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
         bins_kernel<<<2 * JOB_BINS / BIN_BLOCK, 1024, 0, s>>>(W.hist, W.bin0, W.bin0 + 2 * JOB_BINS);
-        order_kernel<<<std::min(dev_sms() * 8, need), 256, 0, s>>>(W);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        order_kernel<<<std::min(l.sms * 8, need), 256, 0, s>>>(W);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if (mid) cudaEventRecord(mid, s);
-    auto blocks = [&](int resident) { return trav_blocks > 0 ? trav_blocks : resident; };
+    if (mid && (e = cudaEventRecord(mid, s)) != cudaSuccess) return e;
     if (W.path_tau) {
-        trav_kernel<R, Stepper, TRAV_TAU, ONE><<<blocks(resident_blocks<R, Stepper, TRAV_TAU, ONE>(smem)), 256, smem, s>>>(W);
+        if ((e = launch_trav<R, Stepper, TRAV_TAU, ONE>(W, smem, trav_blocks, false, s)) != cudaSuccess) return e;
     } else {
-        trav_kernel<R, Stepper, TRAV_PATH, ONE><<<blocks(resident_blocks<R, Stepper, TRAV_PATH, ONE>(smem)), 256, smem, s>>>(W);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(resident_blocks<R, Stepper, TRAV_TAU, ONE>(smem));
-        cfg.blockDim = dim3(256);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = SKG_PDL;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, trav_kernel<R, Stepper, TRAV_TAU, ONE>, W);
-        if (e != cudaSuccess) return e;
+        if ((e = launch_trav<R, Stepper, TRAV_PATH, ONE>(W, smem, trav_blocks, false, s)) != cudaSuccess) return e;
+        if ((e = launch_trav<R, Stepper, TRAV_TAU, ONE>(W, smem, 0, true, s)) != cudaSuccess) return e;
     }
-    end_kernel<<<std::min(need, dev_sms() * dper), 256, 0, s>>>(W);
+    end_kernel<<<std::min(need, d.blocks), 256, 0, s>>>(W);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // On large trees the few cells of the re-walks come from the lattice records, one table for all
     // directions: a wave's re-walks touch most of the eight octant tables once, and their records come
     // from DRAM (2.9 GB per launch on the 3*10^6-leaf octree).  2*10^7 packets there 190 -> 186 ms a
     // pass; 32 MB of records the same either way, a small octree 2.9 -> 3.0 ms.
-    if constexpr (std::is_same<Stepper<R>, TreeOctantStepper<float>>::value) {
-        if (W.rewalk_lattice) {
-            trav_kernel<float, TreeLatticeStepper, TRAV_REWALK, ONE>
-                <<<resident_blocks<float, TreeLatticeStepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
-        }
-    }
-    if (!W.rewalk_lattice)
-        trav_kernel<R, Stepper, TRAV_REWALK, ONE><<<resident_blocks<R, Stepper, TRAV_REWALK, ONE>(smem), 256, smem, s>>>(W);
-    return cudaGetLastError();
+    if constexpr (std::is_same<Stepper<R>, TreeOctantStepper<float>>::value)
+        if (W.rewalk_lattice) return launch_trav<float, TreeLatticeStepper, TRAV_REWALK, ONE>(W, smem, 0, false, s);
+    return launch_trav<R, Stepper, TRAV_REWALK, ONE>(W, smem, 0, false, s);
 }
 
 template<typename R, template<typename> class Stepper>
 cudaError_t enqueue_tail(WaveParams W, cudaStream_t s) {
     if (W.wave == 0) {                // the whole phase: spread the packets over the warps resident at once
-        static int per = 0;
-        if (per == 0) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tail_kernel<R, Stepper>, 128, 0);
-            per = std::max(per, 1);
-        }
-        W.tail_lanes = std::min(32, std::max(1, (W.npool + dev_sms() * per * 4 - 1) / (dev_sms() * per * 4)));
+        Resident r;
+        cudaError_t e = resident((const void*)tail_kernel<R, Stepper>, 128, 0, r);
+        if (e != cudaSuccess) return e;
+        W.tail_lanes = std::min(32, std::max(1, (W.npool + r.blocks * 4 - 1) / (r.blocks * 4)));
     }
     const int warps = (W.npool + W.tail_lanes - 1) / W.tail_lanes;
     tail_kernel<R, Stepper><<<(warps + 3) / 4, 128, 0, s>>>(W);

@@ -1,0 +1,63 @@
+"""Batches of the default capacity (64 slots): the walks of both precisions launch with any number of
+slots in use, and give each simulation the tallies that it gets alone (packets draw from streams keyed by
+their index; the sums differ by the order of the FP64 atomics)."""
+import numpy as np
+import pytest
+
+from skirt7_b200 import _abi as A
+from skirt7_b200 import models, runtime
+
+from test_walks_gpu import CLOSE, model
+
+pytestmark = pytest.mark.gpu
+
+
+def alone(ctx, n, seed, precision):
+    ctx.reset_tallies()
+    ctx.run_phase(A.PHASE_STELLAR, [0], n, seed=seed, precision=precision)
+    ctx.sync()
+    return ctx.read_instrument(0)[0].copy()
+
+
+@pytest.mark.parametrize("precision", [A.PREC_FP32, A.PREC_FP64])
+@pytest.mark.parametrize("grid", ["cartesian", "octree", "kdtree", "voronoi"])
+def test_one_simulation_in_a_batch_of_default_capacity(grid, precision):
+    ctx = runtime.Context(model(grid))
+    n = 30001                                   # above the tail pass alone on every grid
+    want = alone(ctx, n, 3, precision)
+    b = runtime.Batch()
+    for graph in (False, True):
+        ctx.reset_tallies()
+        ctx.sync()
+        b.run(A.PHASE_STELLAR, [(ctx, [0], n, 0, n, 3)], precision=precision, graph=graph)
+        b.sync()
+        assert np.allclose(ctx.read_instrument(0)[0], want, **CLOSE)
+    assert b.counters()["errors"] == 0
+    b.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("precision", [A.PREC_FP32, A.PREC_FP64])
+def test_every_slot_in_use_and_fewer_on_the_same_graph(precision):
+    ctxs = []
+    for i in range(64):
+        m = models.oligo_disk(N=(6 + i % 5, 7, 5), npix=12)
+        m.rho = np.random.default_rng(i).uniform(0.5, 2, (1, (6 + i % 5) * 35)) * 1e-24
+        ctxs.append(runtime.Context(m))
+    n = 401
+    want = [alone(c, n, 100 + i, precision) for i, c in enumerate(ctxs)]
+    assert all(w.sum() > 0 for w in want)
+    b = runtime.Batch()
+    for graph, slots in ((False, 64), (True, 64), (True, 55), (True, 57), (False, 57)):
+        for c in ctxs:
+            c.reset_tallies()
+            c.sync()
+        b.run(A.PHASE_STELLAR, [(c, [0], n, 0, n, 100 + i) for i, c in enumerate(ctxs[:slots])], precision=precision,
+              graph=graph)
+        b.sync()
+        for i, c in enumerate(ctxs):
+            got = c.read_instrument(0)[0]
+            assert np.allclose(got, want[i] if i < slots else 0, **CLOSE), (graph, slots, i)
+    b.close()
+    for c in ctxs:
+        c.close()
