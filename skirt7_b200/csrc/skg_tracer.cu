@@ -1693,11 +1693,30 @@ cudaError_t WaveRunner::record_copied() {
 cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, int precision, int nslots,
                               size_t npool, bool fits, int trav_blocks, bool absorbs, cudaStream_t s,
                               const DevGrid* one_grid) {
+    const cudaError_t e = start(P, grid_type, tree_walk, precision, nslots, npool, fits, trav_blocks, absorbs, s, one_grid);
+    return e == cudaSuccess ? e : over(e);
+}
+
+// A phase that could not be enqueued is over: nothing is added to it, what it had enqueued no longer uses
+// the pool and its simulations' tables when the call returns, and its error is not a later call's.
+cudaError_t WaveRunner::over(cudaError_t e) {
+    pending_ = timed_ = false;
+    cudaGetLastError();
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream_, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) cudaStreamSynchronize(stream_);
+    cudaGetLastError();
+    return e;
+}
+
+cudaError_t WaveRunner::start(const RunParams& P, int grid_type, int tree_walk, int precision, int nslots,
+                              size_t npool, bool fits, int trav_blocks, bool absorbs, cudaStream_t s,
+                              const DevGrid* one_grid) {
+    stream_ = s;
     if (npool == 0 || npool > cap_pool_) return cudaErrorInvalidValue;
     P_ = P; grid_type_ = grid_type; tree_walk_ = tree_walk; precision_ = precision; nslots_ = nslots;
     one_ = one_grid != nullptr && nslots == 1;
     if (one_) g0_ = *one_grid; else std::memset(&g0_, 0, sizeof(g0_));
-    trav_blocks_ = trav_blocks; stream_ = s; npool_ = (int)npool; waves_ = 0; tail_ran_ = false;
+    trav_blocks_ = trav_blocks; npool_ = (int)npool; waves_ = 0; tail_ran_ = false;
     const char* td = std::getenv("SKG_TAIL_DIV");
     tail_div_ = td ? std::atoi(td) : tail_div;
     path_tau_ = !absorbs;
@@ -1711,12 +1730,16 @@ cudaError_t WaveRunner::begin(const RunParams& P, int grid_type, int tree_walk, 
     // (the waves leave the counts of the bins at zero; cleared here, on the phase's stream, for the first and for
     // one that follows a failed phase)
     if (order_on_ && (e = cudaMemsetAsync(bins_, 0, 2 * JOB_BINS * sizeof(unsigned), s)) != cudaSuccess) return e;
-    pending_ = true;
     tail_only_ = tail_div_ > 0 && fits && npool <= (size_t)(grid_type == SKG_GRID_CARTESIAN ? SKG_TAIL_ONLY_CART : SKG_TAIL_ONLY);
-    if (!tail_only_) return enqueue(estimate);
-    if ((e = cudaMemsetAsync(pk_, 0, npool * sizeof(Packet), s)) != cudaSuccess) return e;   // (wave 0 writes every record)
-    if ((e = enqueue_tail()) != cudaSuccess) return e;
-    return record_copied();
+    if (!tail_only_) {
+        if ((e = enqueue(estimate)) != cudaSuccess) return e;
+    } else {
+        if ((e = cudaMemsetAsync(pk_, 0, npool * sizeof(Packet), s)) != cudaSuccess) return e;   // (wave 0 writes every record)
+        if ((e = enqueue_tail()) != cudaSuccess) return e;
+        if ((e = record_copied()) != cudaSuccess) return e;
+    }
+    pending_ = true;
+    return cudaSuccess;
 }
 
 cudaError_t WaveRunner::enqueue_tail() {
@@ -1769,14 +1792,14 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
             // few packets left in flight: the tail pass finishes them (and any packets still to
             // launch) in one launch; the next phase enqueues this many waves before it looks
             cudaError_t e = enqueue_tail();
+            if (e != cudaSuccess) return over(e);
             pending_ = false;
-            if (e != cudaSuccess) return e;
             estimate = waves_;
             more = true;
             break;
         }
         cudaError_t e = enqueue(estimate > 32 ? estimate / 4 : 8);
-        if (e != cudaSuccess) { pending_ = false; return e; }
+        if (e != cudaSuccess) return over(e);
         more = true;
     }
     return (end && more) ? cudaEventRecord(end, stream_) : cudaSuccess;

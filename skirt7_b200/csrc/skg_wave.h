@@ -55,6 +55,9 @@ public:
     int tail_div = 16;
 
 private:
+    cudaError_t start(const RunParams& P, int grid_type, int tree_walk, int precision, int nslots, size_t npool, bool fits,
+                      int trav_blocks, bool absorbs, cudaStream_t s, const DevGrid* one_grid);
+    cudaError_t over(cudaError_t e);
     cudaError_t enqueue(int n);
     cudaError_t enqueue_tail();
     cudaError_t record_copied();

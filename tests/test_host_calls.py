@@ -1,0 +1,39 @@
+"""What the library enqueues, where and in which order, and what it does when a call fails: its host side on
+the CPU, with a fake of the CUDA runtime (fake_cudart.cpp)."""
+import pytest
+
+import fake_cuda
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory, lib):
+    return fake_cuda.compile_fake(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_a_phase_that_could_not_be_enqueued_is_over(fake, batch):
+    """A kernel of the first wave fails to launch: the call reports it, nothing of the wave is launched behind
+    it, and the calls that follow do not go on with the failed phase."""
+    fake_cuda.run(fake, """
+        c = runtime.Context(oligo())
+        b = runtime.Batch(max_slots=2) if %r else None
+        def run():
+            if b: b.run(A.PHASE_STELLAR, [(c, [0], 30000, 0, 30000, 1)])
+            else: c.run_phase(A.PHASE_STELLAR, [0], 30000)
+        sync = b.sync if b else c.sync
+        fake.fake_busy(24, 100)                  # ends in the tail pass, after the first look at the counters
+        run(); sync()
+        assert len(log("tail_kernel")) == 1
+        fake.fake_fail(b"trav_kernel", 0)
+        try:
+            run()
+            assert False
+        except A.SkirtError as e:
+            assert e.code == A.SKG_ERR_CUDA
+        kernels = log("launch ")
+        assert len(kernels) == 1 and "launch_kernel" in kernels[0], kernels
+        sync()
+        assert not log("launch ")                # no waves and no tail pass of the failed phase
+        run(); sync()
+        assert len(log("tail_kernel")) == 1
+    """ % batch)
