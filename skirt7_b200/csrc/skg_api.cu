@@ -1391,12 +1391,20 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
             if (!same) {
                 if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
                 if (!b->g_stream) CK(cudaStreamCreateWithFlags(&b->g_stream, cudaStreamNonBlocking));
-                cudaGraph_t gr;
+                cudaGraph_t gr = nullptr;
                 CK(cudaStreamBeginCapture(b->g_stream, cudaStreamCaptureModeThreadLocal));
-                enqueue(b->g_stream);
+                try {
+                    enqueue(b->g_stream);
+                } catch (const Failure&) {                // (the capture ends with it)
+                    cudaStreamEndCapture(b->g_stream, &gr);
+                    if (gr) cudaGraphDestroy(gr);
+                    cudaGetLastError();
+                    throw;
+                }
                 CK(cudaStreamEndCapture(b->g_stream, &gr));
                 cudaError_t e = cudaGraphInstantiate(&b->graph, gr, 0);
                 cudaGraphDestroy(gr);
+                if (e != cudaSuccess) b->graph = nullptr;
                 CK(e);
                 b->g_type = gtype; b->g_bk = gbk; b->g_prec = precision; b->g_blocks = blocks; b->g_npool = npool;
                 b->g_slots = gslots; b->g_absorbs = absorbs; b->g_fits = total <= npool; b->g_gen = b->waves.generation();

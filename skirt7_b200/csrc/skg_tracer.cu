@@ -1738,7 +1738,7 @@ cudaError_t WaveRunner::start(const RunParams& P, int grid_type, int tree_walk, 
         if ((e = enqueue_tail()) != cudaSuccess) return e;
         if ((e = record_copied()) != cudaSuccess) return e;
     }
-    pending_ = true;
+    pending_ = cs == cudaStreamCaptureStatusNone;   // (a captured phase runs when it is replayed)
     return cudaSuccess;
 }
 

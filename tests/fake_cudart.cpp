@@ -34,7 +34,7 @@ std::map<const void*, std::string> kernels;
 std::map<void*, size_t> allocated;
 size_t total = (size_t)8 << 30, used = 0;
 int busy = 0, jobs = 0;             // waves of a phase with work, path jobs in each
-std::string fail_name;              // launches of kernels whose name holds this ...
+std::string fail_name;              // launches of kernels whose name holds this ("instantiate": of a graph) ...
 int fail_skip = -1;                 // ... fail after this many (-1: none)
 cudaError_t last = cudaSuccess;
 std::map<cudaStream_t, Graph*> capturing;
@@ -197,7 +197,11 @@ cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t* g) {
     log("uncapture %ld", id(s));
     return cudaSuccess;
 }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t g, unsigned long long) { *x = (cudaGraphExec_t) new Graph(*(Graph*)g); return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t g, unsigned long long) {
+    if (fail_name == "instantiate" && fail_skip-- == 0) return last = cudaErrorMemoryAllocation;
+    *x = (cudaGraphExec_t) new Graph(*(Graph*)g);
+    return cudaSuccess;
+}
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { delete (Graph*)g; return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { delete (Graph*)x; return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t s) {

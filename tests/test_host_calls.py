@@ -37,3 +37,30 @@ def test_a_phase_that_could_not_be_enqueued_is_over(fake, batch):
         run(); sync()
         assert len(log("tail_kernel")) == 1
     """ % batch)
+
+
+@pytest.mark.parametrize("what,code", [("trav_kernel", "A.SKG_ERR_CUDA"), ("instantiate", "A.SKG_ERR_OOM")])
+def test_a_capture_that_failed_is_closed(fake, what, code):
+    """A launch fails while a batch is captured, or its graph cannot be made: nothing runs, and the next
+    captured run works."""
+    fake_cuda.run(fake, """
+        c = runtime.Context(oligo())
+        b = runtime.Batch(max_slots=2)
+        def run(graph):
+            b.run(A.PHASE_STELLAR, [(c, [0], 30000, 0, 30000, 1)], graph=graph)
+        fake.fake_busy(24, 100)
+        run(False); b.sync()
+        log()
+        fake.fake_fail(b"%s", 0)
+        try:
+            run(True)
+            assert False
+        except A.SkirtError as e:
+            assert e.code == %s
+        assert len(log("uncapture")) == 1
+        b.sync()
+        assert not log("launch ")
+        run(True); b.sync()
+        lines = log()
+        assert any(l.startswith("replay") for l in lines) and any("end_kernel" in l for l in lines)
+    """ % (what, code))
