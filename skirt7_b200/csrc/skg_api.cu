@@ -1208,6 +1208,7 @@ struct skg_batch {
     size_t g_npool = 0;
     bool g_absorbs = false, g_fits = false;
     int g_waves = 0;                       // waves captured in the graph
+    WaveRunner::Phase g_phase;             // and what they were launched with
     bool g_stale = false;                  // a replay needed more waves than captured
     cudaStream_t g_stream = nullptr;
     WaveRunner waves;
@@ -1387,7 +1388,8 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
         if (flags & SKG_BATCH_GRAPH) {
             bool same = b->graph && !b->g_stale && b->g_slots >= gslots && b->g_absorbs == absorbs && b->g_fits == (total <= npool) &&
                         b->g_gen == b->waves.generation() && b->g_type == gtype && b->g_bk == gbk && b->g_prec == precision &&
-                        b->g_blocks == blocks && b->g_npool == npool;
+                        b->g_blocks == blocks && b->g_npool == npool && b->g_phase.P.max_scatt == P.max_scatt &&
+                        b->g_phase.P.refill == P.refill;
             if (!same) {
                 if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
                 if (!b->g_stream) CK(cudaStreamCreateWithFlags(&b->g_stream, cudaStreamNonBlocking));
@@ -1408,10 +1410,10 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
                 CK(e);
                 b->g_type = gtype; b->g_bk = gbk; b->g_prec = precision; b->g_blocks = blocks; b->g_npool = npool;
                 b->g_slots = gslots; b->g_absorbs = absorbs; b->g_fits = total <= npool; b->g_gen = b->waves.generation();
-                b->g_waves = b->waves.waves(); b->g_stale = false;
+                b->g_waves = b->waves.waves(); b->g_phase = b->waves.phase(); b->g_stale = false;
             }
             CK(cudaGraphLaunch(b->graph, s));
-            b->waves.replayed(s, b->g_waves);       // the replay runs the captured waves on s
+            b->waves.replayed(s, b->g_waves, b->g_phase);
         } else {
             enqueue(s);
         }

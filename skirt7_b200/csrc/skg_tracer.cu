@@ -1646,24 +1646,24 @@ cudaError_t WaveRunner::reserve(size_t pool, int ngroups, int grid_type, size_t 
 }
 
 cudaError_t WaveRunner::enqueue(int n) {
-    WaveFn fn = pick(grid_type_, tree_walk_, precision_, one_).wave;
+    WaveFn fn = pick(ph_.grid_type, ph_.tree_walk, ph_.precision, ph_.one).wave;
     cudaError_t e;
     for (int i = 0; i < n; i++) {
         const int w = waves_ + i, b = w & 1;
         WaveParams W;
-        W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = w;
+        W.R = ph_.P; W.pk = pk_; W.npool = ph_.npool; W.wave = w;
         W.jobs = jobs_; W.jtau = jtau_; W.jL = jL_;
         W.jcount = ctr_ + J_N * b; W.jnext = ctr_ + J_N * (b ^ 1);
         W.last_busy = ctr_ + 2 * J_N;
-        W.freelist = lists_[b]; W.intlist = lists_[b] + npool_; W.freenext = lists_[b ^ 1]; W.intnext = lists_[b ^ 1] + npool_;
-        W.rlist = rlist_; W.path_tau = path_tau_; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
-        W.g0 = g0_;
-        W.rewalk_lattice = tree_walk_ == TW_OCTANT && grid_type_ != SKG_GRID_CARTESIAN &&
-                           precision_ == SKG_PREC_FP32 && big_records_;
-        W.hist = order_on_ ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
+        W.freelist = lists_[b]; W.intlist = lists_[b] + ph_.npool; W.freenext = lists_[b ^ 1]; W.intnext = lists_[b ^ 1] + ph_.npool;
+        W.rlist = rlist_; W.path_tau = ph_.path_tau; W.ckpt = ph_.ckpt_on ? ckpt_ : nullptr;
+        W.g0 = ph_.g0;
+        W.rewalk_lattice = ph_.tree_walk == TW_OCTANT && ph_.grid_type != SKG_GRID_CARTESIAN &&
+                           ph_.precision == SKG_PREC_FP32 && ph_.big_records;
+        W.hist = ph_.order_on ? bins_ : nullptr; W.bin0 = bins_ + 2 * JOB_BINS;
         // (a job's key lies where its optical depth will)
         W.jkey = reinterpret_cast<uint2*>(jtau_); W.speel = order_;
-        W.spath = reinterpret_cast<int*>(order_ + (cap_order_ - npool_));
+        W.spath = reinterpret_cast<int*>(order_ + (cap_order_ - ph_.npool));
         if ((e = cudaMemsetAsync(ctr_ + J_N * (b ^ 1), 0, J_N * sizeof(unsigned), stream_)) != cudaSuccess) return e;
         if (timed_) {
             while (ev_.size() < 3 * (size_t)(w + 1)) {
@@ -1673,7 +1673,7 @@ cudaError_t WaveRunner::enqueue(int n) {
             }
             if ((e = cudaEventRecord(ev_[3 * w], stream_)) != cudaSuccess) return e;
         }
-        if ((e = fn(W, nslots_, trav_blocks_, timed_ ? ev_[3 * w + 1] : nullptr, stream_)) != cudaSuccess) return e;
+        if ((e = fn(W, ph_.nslots, ph_.trav_blocks, timed_ ? ev_[3 * w + 1] : nullptr, stream_)) != cudaSuccess) return e;
         if (timed_ && (e = cudaEventRecord(ev_[3 * w + 2], stream_)) != cudaSuccess) return e;
     }
     waves_ += n;
@@ -1713,15 +1713,16 @@ cudaError_t WaveRunner::start(const RunParams& P, int grid_type, int tree_walk, 
                               const DevGrid* one_grid) {
     stream_ = s;
     if (npool == 0 || npool > cap_pool_) return cudaErrorInvalidValue;
-    P_ = P; grid_type_ = grid_type; tree_walk_ = tree_walk; precision_ = precision; nslots_ = nslots;
-    one_ = one_grid != nullptr && nslots == 1;
-    if (one_) g0_ = *one_grid; else std::memset(&g0_, 0, sizeof(g0_));
-    trav_blocks_ = trav_blocks; npool_ = (int)npool; waves_ = 0; tail_ran_ = false;
+    ph_.P = P; ph_.grid_type = grid_type; ph_.tree_walk = tree_walk; ph_.precision = precision; ph_.nslots = nslots;
+    ph_.one = one_grid != nullptr && nslots == 1;
+    if (ph_.one) ph_.g0 = *one_grid; else std::memset(&ph_.g0, 0, sizeof(ph_.g0));
+    ph_.trav_blocks = trav_blocks; ph_.npool = (int)npool; waves_ = 0; tail_ran_ = false;
     const char* td = std::getenv("SKG_TAIL_DIV");
-    tail_div_ = td ? std::atoi(td) : tail_div;
-    path_tau_ = !absorbs;
+    ph_.tail_div = td ? std::atoi(td) : tail_div;
+    ph_.path_tau = !absorbs;
+    ph_.order_on = order_on_; ph_.big_records = big_records_;
     const char* ck = std::getenv("SKG_CKPT");
-    ckpt_on_ = !(ck && std::atoi(ck) == 0) && ckpt_ && cap_ckpt_ >= (size_t)npool;
+    ph_.ckpt_on = !(ck && std::atoi(ck) == 0) && ckpt_ && cap_ckpt_ >= (size_t)npool;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(s, &cs);
     timed_ = timing && cs == cudaStreamCaptureStatusNone;
@@ -1730,7 +1731,7 @@ cudaError_t WaveRunner::start(const RunParams& P, int grid_type, int tree_walk, 
     // (the waves leave the counts of the bins at zero; cleared here, on the phase's stream, for the first and for
     // one that follows a failed phase)
     if (order_on_ && (e = cudaMemsetAsync(bins_, 0, 2 * JOB_BINS * sizeof(unsigned), s)) != cudaSuccess) return e;
-    tail_only_ = tail_div_ > 0 && fits && npool <= (size_t)(grid_type == SKG_GRID_CARTESIAN ? SKG_TAIL_ONLY_CART : SKG_TAIL_ONLY);
+    tail_only_ = ph_.tail_div > 0 && fits && npool <= (size_t)(grid_type == SKG_GRID_CARTESIAN ? SKG_TAIL_ONLY_CART : SKG_TAIL_ONLY);
     if (!tail_only_) {
         if ((e = enqueue(estimate)) != cudaSuccess) return e;
     } else {
@@ -1744,11 +1745,11 @@ cudaError_t WaveRunner::start(const RunParams& P, int grid_type, int tree_walk, 
 
 cudaError_t WaveRunner::enqueue_tail() {
     WaveParams W;
-    W.R = P_; W.pk = pk_; W.npool = npool_; W.wave = waves_;
+    W.R = ph_.P; W.pk = pk_; W.npool = ph_.npool; W.wave = waves_;
     W.jobs = nullptr; W.jtau = nullptr; W.jL = nullptr; W.jcount = nullptr; W.jnext = nullptr;
     W.last_busy = ctr_ + 2 * J_N;
     W.tail_lanes = 32;
-    W.freelist = nullptr; W.intlist = nullptr; W.freenext = nullptr; W.intnext = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ckpt_on_ ? ckpt_ : nullptr;
+    W.freelist = nullptr; W.intlist = nullptr; W.freenext = nullptr; W.intnext = nullptr; W.rlist = nullptr; W.path_tau = 0; W.ckpt = ph_.ckpt_on ? ckpt_ : nullptr;
     W.rewalk_lattice = 0;
     W.hist = nullptr; W.bin0 = nullptr; W.jkey = nullptr; W.spath = nullptr; W.speel = nullptr;
     cudaError_t e;
@@ -1757,8 +1758,8 @@ cudaError_t WaveRunner::enqueue_tail() {
             if (!tail_ev_[i] && (e = cudaEventCreate(&tail_ev_[i])) != cudaSuccess) return e;
         if ((e = cudaEventRecord(tail_ev_[0], stream_)) != cudaSuccess) return e;
     }
-    W.g0 = g0_;
-    if ((e = pick(grid_type_, tree_walk_, precision_, one_).tail(W, stream_)) != cudaSuccess) return e;
+    W.g0 = ph_.g0;
+    if ((e = pick(ph_.grid_type, ph_.tree_walk, ph_.precision, ph_.one).tail(W, stream_)) != cudaSuccess) return e;
     tail_ran_ = true;
     return timed_ ? cudaEventRecord(tail_ev_[1], stream_) : cudaSuccess;
 }
@@ -1788,7 +1789,7 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
             estimate = (int)h_ctr_[2 * J_N] + 2;        // the last busy wave, the empty one, one spare
             break;
         }
-        if (tail_div_ > 0 && (size_t)busy * (size_t)tail_div_ <= (size_t)npool_) {
+        if (ph_.tail_div > 0 && (size_t)busy * (size_t)ph_.tail_div <= (size_t)ph_.npool) {
             // few packets left in flight: the tail pass finishes them (and any packets still to
             // launch) in one launch; the next phase enqueues this many waves before it looks
             cudaError_t e = enqueue_tail();

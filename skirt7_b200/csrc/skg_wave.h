@@ -37,8 +37,24 @@ public:
     // Waits for the enqueued waves and enqueues more until no packet is left; then records
     // `end` (if given) on the phase's stream.  timeout_ms < 0 waits without limit.
     cudaError_t finish(int timeout_ms, cudaEvent_t end, bool* timed_out);
-    // A captured begin() (pool reset and n waves) was launched as a graph on stream s.
-    void replayed(cudaStream_t s, int n) { pending_ = true; stream_ = s; waves_ = n; tail_only_ = n == 0; }
+    // What the waves of a phase are launched with.
+    struct Phase {
+        RunParams P{};
+        int grid_type = 0, tree_walk = TW_ROPE, precision = 0, nslots = 1, trav_blocks = 0, npool = 0;
+        bool one = false;              // a single-slot launch with its grid in g0
+        DevGrid g0{};
+        bool path_tau = false;
+        int tail_div = 16;
+        bool ckpt_on = true;           // path-walk checkpoints (environment variable SKG_CKPT=0: off)
+        bool order_on = false;         // its jobs are walked in spatial order
+        bool big_records = false;      // the walks' records of one direction exceed half the L2
+    };
+    const Phase& phase() const { return ph_; }
+    // A captured begin() (pool reset and n waves) of the phase `was` was launched as a graph on stream s: the
+    // waves that finish() adds are launched as the captured ones, whatever ran in between.
+    void replayed(cudaStream_t s, int n, const Phase& was) {
+        ph_ = was; pending_ = true; timed_ = tail_ran_ = false; stream_ = s; waves_ = n; tail_only_ = n == 0;
+    }
     bool pending() const { return pending_; }
     int waves() const { return waves_; }
     size_t pool_capacity() const { return cap_pool_; }
@@ -77,9 +93,7 @@ private:
     unsigned* bins_ = nullptr;        // [2][JOB_BINS] counts, [2][JOB_BINS] first places (walk order)
     uint2* order_ = nullptr;          // peel-off jobs in walk order; at its end, the path jobs' packets
     size_t cap_order_ = 0;
-    bool order_on_ = false;           // the running phase walks its jobs in spatial order
-    bool big_records_ = false;        // the walks' records of one direction exceed half the L2
-    bool path_tau_ = false;
+    bool order_on_ = false, big_records_ = false;   // of the phase that reserve() was called for
     static constexpr int NCTR = 2 * J_N + 1;
     unsigned* ctr_ = nullptr;         // [J_N (w & 1) + JobCount]: counters of wave w; [2 J_N]: last busy wave
     unsigned* h_ctr_ = nullptr;       // pinned copy read by finish()
@@ -87,17 +101,10 @@ private:
 
     bool pending_ = false;
     cudaStream_t stream_ = nullptr;
-    RunParams P_{};
-    int grid_type_ = 0, precision_ = 0, nslots_ = 1, trav_blocks_ = 0;
-    bool one_ = false;                 // a single-slot launch with its grid in g0_
-    DevGrid g0_{};
-    int tree_walk_ = TW_ROPE;
-    int npool_ = 0;
+    Phase ph_;
     int waves_ = 0;
     std::vector<cudaEvent_t> ev_;      // 3 per wave: before the launch pass, before the walks, after the ends and re-walks
     bool timed_ = false;               // the running phase records ev_
-    int tail_div_ = 16;
-    bool ckpt_on_ = true;              // path-walk checkpoints (environment variable SKG_CKPT=0: off)
     bool tail_only_ = false;           // the phase is the tail pass alone
     bool tail_ran_ = false;            // the phase ended with the tail pass
     cudaEvent_t tail_ev_[2] = {nullptr, nullptr};

@@ -7,6 +7,7 @@ import pytest
 from skirt7_b200 import _abi as A
 from skirt7_b200 import models, runtime
 
+from helpers import cell_center_density
 from test_walks_gpu import CLOSE, model
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,31 @@ def test_every_slot_in_use_and_fewer_on_the_same_graph(precision):
     b.close()
     for c in ctxs:
         c.close()
+
+
+def test_a_replay_goes_on_as_it_was_captured():
+    """A captured phase with absorption on a pool of 2^16; a smaller direct phase without, on another walk; the
+    graph again, for a simulation that takes more waves than were captured (thick dust)."""
+    def ctx(tau, absorb):
+        m = models.oligo_disk(N=(12, 11, 9), tauV=tau, npix=12, write_absorption=absorb)
+        m.rho = cell_center_density(m)
+        return runtime.Context(m)
+    thin, thick, plain = ctx(0.01, True), ctx(200.0, True), ctx(1.0, False)
+    n = 60000
+    want = alone(thick, n, 5, A.PREC_FP32)
+    absorbed = thick.read_absorption()[0]
+    b = runtime.Batch(max_slots=2)
+    b.run(A.PHASE_STELLAR, [(thin, [0], n, 0, n, 5)], graph=True)
+    b.sync()
+    captured = b.counters()["waves"]
+    for _ in range(2):
+        b.run(A.PHASE_STELLAR, [(plain, [0], 23000, 0, 23000, 5)], precision=A.PREC_FP64, pool=21000)
+        b.sync()
+        thick.reset_tallies()
+        thick.sync()
+        b.run(A.PHASE_STELLAR, [(thick, [0], n, 0, n, 5)], graph=True)
+        b.sync()
+        assert np.allclose(thick.read_instrument(0)[0], want, **CLOSE)
+        assert np.allclose(thick.read_absorption()[0], absorbed, **CLOSE)
+    assert captured > 1 and b.counters()["errors"] == 0
+    b.close()

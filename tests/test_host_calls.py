@@ -64,3 +64,43 @@ def test_a_capture_that_failed_is_closed(fake, what, code):
         lines = log()
         assert any(l.startswith("replay") for l in lines) and any("end_kernel" in l for l in lines)
     """ % (what, code))
+
+
+def test_waves_added_to_a_replay_are_launched_as_captured(fake):
+    """Between two replays of a captured batch a smaller phase of another kind runs directly: the waves and the
+    tail pass added to the second replay have the captured pool and kind of walk.  Budgets frozen in the
+    captured launches make another graph."""
+    fake_cuda.run(fake, """
+        keeps, plain = runtime.Context(oligo(write_absorption=True)), runtime.Context(oligo(write_absorption=False))
+        b = runtime.Batch(max_slots=2)
+        def run(ctx, n, graph, **kw):
+            log()
+            b.run(A.PHASE_STELLAR, [(ctx, [0], n, 0, n, 1)], graph=graph, **kw)
+            b.sync()
+            return log()
+        waves = lambda lines: [l for l in lines if "launch " in l and "WaveParams" in l]
+        fake.fake_busy(1, 60000)
+        run(keeps, 60000, True)
+        run(plain, 22000, False, precision=A.PREC_FP64, pool=21000, max_scatt=9, refill=3)
+        # more waves than were captured, and the tail pass, behind the replay
+        fake.fake_busy(30, 60000)
+        lines = run(keeps, 60000, True)
+        assert not any(l.startswith("capture") for l in lines)
+        added = waves(lines[lines.index("end of replay"):])
+        assert len(added) == 40                           # eight waves of five kernels
+        replayed = waves(lines[:lines.index("end of replay")])
+        what = lambda l: (l.split(" (")[0].split("launch ")[1].split("(")[0], l.split("npool")[1])
+        for l in added:
+            assert what(l)[1] in {what(r)[1] for r in replayed}, l
+            assert what(l)[0] in {what(r)[0] for r in replayed}, l
+        run(plain, 22000, False, precision=A.PREC_FP64, pool=21000, max_scatt=9, refill=3)
+        fake.fake_busy(24, 100)
+        lines = run(keeps, 60000, True)
+        tail = [l for l in lines if "tail_kernel" in l]
+        assert len(tail) == 1 and "<float" in tail[0] and "npool 65536" in tail[0] and "refill 0" in tail[0], tail
+        for kw in (dict(max_scatt=7), dict(refill=5)):
+            lines = run(keeps, 60000, True, **kw)
+            (k, v), = kw.items()
+            assert any(l.startswith("capture") for l in lines)
+            assert all("%s %d " % (k, v) in l for l in waves(lines))
+    """)
