@@ -1781,10 +1781,11 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
             wait_a_little(t0, 50);
         }
         if (tail_only_) { pending_ = false; break; }
-        // packets with jobs in the last wave (without dust a packet has peel-offs alone)
+        // packets with jobs in the last wave (without dust a packet has peel-offs alone, or, off every
+        // frame, no job at all: its record then waits on the next wave's free list)
         const unsigned* c = h_ctr_ + J_N * ((waves_ - 1) & 1);
         const unsigned busy = c[J_PATH] ? c[J_PATH] : c[J_PEEL];
-        if (busy == 0) {
+        if (busy == 0 && h_ctr_[J_N * (waves_ & 1) + J_FREE] == 0) {
             pending_ = false;
             estimate = (int)h_ctr_[2 * J_N] + 2;        // the last busy wave, the empty one, one spare
             break;
