@@ -375,6 +375,10 @@ struct skg_ctx {
     unsigned* herr = nullptr;
     cudaEvent_t hev = nullptr;
     bool hev_pending = false;
+    // The end of the resets on the context's stream, which launches on other streams (a batch's, a caller's)
+    // wait for; nothing to wait for once skg_sync has seen that stream idle.
+    cudaEvent_t done = nullptr;
+    bool behind = false;
     Staging own;                              // tables of this context's own launches
     WaveRunner waves;                         // packet pool and job lists of this context's phases
     uint64_t wave_count = 0;                  // waves since the last tally reset
@@ -398,6 +402,15 @@ static bool carries_luminosity(const DevScene& S, int phase) {
 // entries of 32 bytes per Voronoi cell.
 static size_t walk_bytes(const DevGrid& g) {
     return (size_t)g.ncells * (g.type == SKG_GRID_CARTESIAN ? 4 : g.type == SKG_GRID_VORONOI ? 512 : 32);
+}
+
+// Work has been enqueued on the context's stream; stream s goes on behind it.
+static void mark(skg_ctx* ctx) {
+    CK(cudaEventRecord(ctx->done, ctx->stream));
+    ctx->behind = true;
+}
+static void follow(skg_ctx* ctx, cudaStream_t s) {
+    if (ctx->behind && s != ctx->stream) CK(cudaStreamWaitEvent(s, ctx->done, 0));
 }
 
 static int fail(skg_ctx* ctx, const Failure& f) {
@@ -696,6 +709,7 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
         if (!ctx->herr) throw Failure{SKG_ERR_OOM, "device allocation failed"};
         CK(cudaMemsetAsync(ctx->herr, 0, sizeof(unsigned), s));
         CK(cudaEventCreateWithFlags(&ctx->hev, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&ctx->done, cudaEventDisableTiming));
         ctx->ds = upload(A, &H, 1, s);
         CK(cudaStreamSynchronize(s));
         *out = ctx;
@@ -708,6 +722,7 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
         if (ctx->ev0) cudaEventDestroy(ctx->ev0);
         if (ctx->ev1) cudaEventDestroy(ctx->ev1);
         if (ctx->hev) cudaEventDestroy(ctx->hev);
+        if (ctx->done) cudaEventDestroy(ctx->done);
         if (ctx->stream) cudaStreamDestroy(ctx->stream);
         delete ctx;
         return rc;
@@ -721,6 +736,7 @@ int skg_ctx_destroy(skg_ctx* ctx) {
     if (ctx->hev_pending) cudaEventSynchronize(ctx->hev);
     ctx->A.release();
     cudaEventDestroy(ctx->ev0); cudaEventDestroy(ctx->ev1); cudaEventDestroy(ctx->hev);
+    cudaEventDestroy(ctx->done);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return SKG_OK;
@@ -751,7 +767,7 @@ int skg_sync(skg_ctx* ctx, int timeout_ms) {
             wait_a_little(t0, 200);
         }
     }
-    ctx->hev_pending = false;
+    ctx->hev_pending = ctx->behind = false;
     unsigned err = 0, herr = 0;
     cudaMemcpy(&err, ctx->err, sizeof(unsigned), cudaMemcpyDeviceToHost);
     cudaMemcpy(&herr, ctx->herr, sizeof(unsigned), cudaMemcpyDeviceToHost);
@@ -872,6 +888,7 @@ int skg_run_phase(skg_ctx* ctx, int phase, const int32_t* ells, int nell, uint64
         const size_t pool_max = (opts && opts->pool > 0) ? (size_t)opts->pool : ((size_t)1 << (big ? 23 : 21));
         const size_t npool = (size_t)std::min<uint64_t>(total, pool_max);
         CK(ctx->waves.reserve(npool, ctx->hs.ngroups, ctx->grid.type, walk_bytes(ctx->grid)));
+        follow(ctx, s);
         // one slot, one work item (pageable host sources: the copies are staged before return)
         BatchHeader H = {phase, 1, 1, 0, total};
         WorkItem W;
@@ -939,6 +956,7 @@ int skg_reset_tallies(skg_ctx* ctx) {
         if (ctx->hs.labs_stel) CK(cudaMemsetAsync(ctx->hs.labs_stel, 0, nlab * sizeof(double), s));
         if (ctx->hs.labs_dust) CK(cudaMemsetAsync(ctx->hs.labs_dust, 0, nlab * sizeof(double), s));
         CK(cudaMemsetAsync(ctx->counters, 0, 10 * sizeof(unsigned long long), s));
+        mark(ctx);
         return SKG_OK;
     } catch (const Failure& f) { return fail(ctx, f); }
 }
@@ -969,6 +987,9 @@ int skg_read_instrument_device(skg_ctx* ctx, int instr, double* d_cube, double* 
     try {
         CK(cudaSetDevice(ctx->device));
         cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(s, &cs));
+        if (cs == cudaStreamCaptureStatusNone) follow(ctx, s);    // (a capture cannot wait for work outside it)
         if (d_cube && ctx->cube_len[instr])
             CK(cudaMemcpyAsync(d_cube, ctx->hs.instr[instr].cube, ctx->cube_len[instr] * sizeof(double),
                                cudaMemcpyDeviceToDevice, s));
@@ -1069,6 +1090,7 @@ int skg_reset_dust_absorption(skg_ctx* ctx) {
         CK(cudaSetDevice(ctx->device));
         if (ctx->hs.labs_dust)
             CK(cudaMemsetAsync(ctx->hs.labs_dust, 0, (size_t)ctx->ncells * ctx->nlambda * sizeof(double), ctx->stream));
+        mark(ctx);
         return SKG_OK;
     } catch (const Failure& f) { return fail(ctx, f); }
 }
@@ -1384,6 +1406,7 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
             CK(b->waves.begin(P, gtype < 0 ? SKG_GRID_CARTESIAN : gtype, gbk < 0 ? TW_ROPE : gbk, precision, gslots, npool,
                               total <= npool, blocks, absorbs, q));
         };
+        for (skg_ctx* c : slots) follow(c, s);
         CK(cudaEventRecord(b->ev0, s));
         if (flags & SKG_BATCH_GRAPH) {
             bool same = b->graph && !b->g_stale && b->g_slots >= gslots && b->g_absorbs == absorbs && b->g_fits == (total <= npool) &&

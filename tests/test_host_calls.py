@@ -104,3 +104,42 @@ def test_waves_added_to_a_replay_are_launched_as_captured(fake):
             assert any(l.startswith("capture") for l in lines)
             assert all("%s %d " % (k, v) in l for l in waves(lines))
     """)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_batch_waits_for_its_simulations_resets(fake, graph):
+    """Resets are enqueued on the contexts' streams; a batch's launches, on another stream, wait for them, and
+    for nothing where the contexts have been synchronised since."""
+    fake_cuda.run(fake, """
+        ctxs = [runtime.Context(oligo()) for _ in range(3)]
+        b = runtime.Batch(max_slots=4)
+        run = lambda: b.run(A.PHASE_STELLAR, [(c, [0], 9000, 0, 9000, 1) for c in ctxs], graph=%r)
+        run(); b.sync()
+        ctxs[2].sync()
+        for c in ctxs: c.reset_tallies()
+        ctxs[1].sync()
+        lines = log()
+        # the event behind each context's last memset
+        ends = [l.split()[1:] for a, l in zip(lines, lines[1:]) if l.startswith("record") and a.startswith("memset")]
+        assert len(ends) == 3 and len({s for _, s in ends}) == 3, ends
+        run(); b.sync()
+        lines = log()
+        first = next(i for i, l in enumerate(lines) if l.startswith(("launch", "replay")))
+        waits = [l.split()[1:] for l in lines[:first] if l.startswith("wait")]
+        stream = lines[first].split()[1]
+        assert waits == [[stream, ends[0][0]], [stream, ends[2][0]]], (waits, ends)
+    """ % graph)
+
+
+@pytest.mark.parametrize("call", ["c.run_phase(A.PHASE_STELLAR, [0], 30000, stream=77)",
+                                  "c.read_instrument_device(0, cube.ctypes.data, stream=77)"])
+def test_a_callers_stream_waits_for_the_reset(fake, call):
+    fake_cuda.run(fake, """
+        import numpy as np
+        c = runtime.Context(oligo())
+        cube = np.zeros(64)
+        c.reset_tallies()
+        end = [l for l in log() if l.startswith("record")][-1].split()[1]
+        %s
+        assert "wait 77 " + end in log()
+    """ % call)
