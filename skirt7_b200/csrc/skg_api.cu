@@ -375,8 +375,8 @@ struct skg_ctx {
     unsigned* herr = nullptr;
     cudaEvent_t hev = nullptr;
     bool hev_pending = false;
-    // The end of the resets on the context's stream, which launches on other streams (a batch's, a caller's)
-    // wait for; nothing to wait for once skg_sync has seen that stream idle.
+    // The end of the resets and finished phases on the context's stream, which launches on other streams (a
+    // batch's, a caller's) wait for; nothing to wait for once skg_sync has seen that stream idle.
     cudaEvent_t done = nullptr;
     bool behind = false;
     Staging own;                              // tables of this context's own launches
@@ -420,7 +420,9 @@ static int fail(skg_ctx* ctx, const Failure& f) {
 }
 
 // Completes the context's running phase: waits for its enqueued waves and adds waves until no
-// packet is left (the reads, resets and the next phase need the finished tallies).
+// packet is left (the reads, resets and the next phase need the finished tallies).  Its last launch, the tail
+// pass, may still run: the context's stream goes on behind it where the phase has a caller's, and other
+// streams behind that.
 static int settle(skg_ctx* ctx, int timeout_ms) {
     if (!ctx->waves.pending()) return SKG_OK;
     cudaSetDevice(ctx->device);
@@ -429,6 +431,10 @@ static int settle(skg_ctx* ctx, int timeout_ms) {
     if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, Failure{SKG_ERR_CUDA, cudaGetErrorString(e)}); }
     if (timed_out) return fail(ctx, Failure{SKG_ERR_TIMEOUT, "timed out waiting for the device"});
     ctx->wave_count += ctx->waves.waves();
+    try {
+        if (ctx->waves.stream() != ctx->stream) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev1, 0));
+        mark(ctx);
+    } catch (const Failure& f) { return fail(ctx, f); }
     return SKG_OK;
 }
 
@@ -733,6 +739,7 @@ int skg_ctx_destroy(skg_ctx* ctx) {
     if (!ctx) return SKG_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    cudaEventSynchronize(ctx->ev1);                  // (a phase on a caller's stream)
     if (ctx->hev_pending) cudaEventSynchronize(ctx->hev);
     ctx->A.release();
     cudaEventDestroy(ctx->ev0); cudaEventDestroy(ctx->ev1); cudaEventDestroy(ctx->hev);
@@ -934,7 +941,8 @@ int skg_phase_times(skg_ctx* ctx, float* event_ms, float* traversal_ms, int32_t*
     int rc = settle(ctx, -1);
     if (rc) return rc;
     cudaSetDevice(ctx->device);
-    cudaError_t e = ctx->waves.times(event_ms, traversal_ms);
+    cudaError_t e = cudaEventSynchronize(ctx->ev1);
+    if (e == cudaSuccess) e = ctx->waves.times(event_ms, traversal_ms);
     if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, Failure{SKG_ERR_CUDA, cudaGetErrorString(e)}); }
     if (waves) *waves = ctx->waves.waves();
     return SKG_OK;
@@ -1296,6 +1304,7 @@ int skg_batch_destroy(skg_batch* b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->g_stream) cudaStreamSynchronize(b->g_stream);
+    if (b->ev1) cudaEventSynchronize(b->ev1);        // (a phase on a caller's stream)
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->g_stream) cudaStreamDestroy(b->g_stream);
     b->A.release();
@@ -1407,6 +1416,7 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
                               total <= npool, blocks, absorbs, q));
         };
         for (skg_ctx* c : slots) follow(c, s);
+        CK(cudaStreamWaitEvent(s, b->ev1, 0));       // (the last phase's tail pass, on whichever stream it runs)
         CK(cudaEventRecord(b->ev0, s));
         if (flags & SKG_BATCH_GRAPH) {
             bool same = b->graph && !b->g_stale && b->g_slots >= gslots && b->g_absorbs == absorbs && b->g_fits == (total <= npool) &&

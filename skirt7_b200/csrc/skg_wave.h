@@ -57,6 +57,7 @@ public:
     }
     bool pending() const { return pending_; }
     int waves() const { return waves_; }
+    cudaStream_t stream() const { return stream_; }
     size_t pool_capacity() const { return cap_pool_; }
     // changes when reserve() has moved a buffer (a captured launch then holds freed memory)
     int generation() const { return generation_; }

@@ -125,8 +125,9 @@ def test_a_batch_waits_for_its_simulations_resets(fake, graph):
         run(); b.sync()
         lines = log()
         first = next(i for i, l in enumerate(lines) if l.startswith(("launch", "replay")))
-        waits = [l.split()[1:] for l in lines[:first] if l.startswith("wait")]
         stream = lines[first].split()[1]
+        waits = [l.split()[1:] for l in lines[:first] if l.startswith("wait")]
+        waits = [w for w in waits if w[1] in {e for e, _ in ends}]
         assert waits == [[stream, ends[0][0]], [stream, ends[2][0]]], (waits, ends)
     """ % graph)
 
@@ -143,3 +144,47 @@ def test_a_callers_stream_waits_for_the_reset(fake, call):
         %s
         assert "wait 77 " + end in log()
     """ % call)
+
+
+def test_what_follows_a_phase_on_a_callers_stream_waits_for_its_tail_pass(fake):
+    """The tail pass is enqueued when the phase is completed: the context's stream goes on behind it (reads,
+    resets, the dust emission), and so does the next phase on yet another stream, which shares its pool."""
+    fake_cuda.run(fake, """
+        c = runtime.Context(oligo())
+        own = [l for l in log("memset")][-1].split()[1]
+        fake.fake_busy(24, 100)
+        for call in (c.sync, c.reset_tallies, lambda: c.run_phase(A.PHASE_STELLAR, [0], 30000, stream=88)):
+            c.run_phase(A.PHASE_STELLAR, [0], 30000, stream=77)
+            log()
+            call()
+            lines = log()
+            tail = next(i for i, l in enumerate(lines) if "tail_kernel" in l)
+            assert lines[tail].startswith("launch 77 ")
+            end = [l for l in lines[tail:] if l.startswith("record") and l.endswith(" 77")][-1].split()[1]
+            wait = lines.index("wait %s %s" % (own, end))
+            assert not any(l.startswith(("memset", "launch")) for l in lines[tail + 1:wait])
+            done = lines[wait + 1].split()
+            assert done[0] == "record" and done[2] == own
+            if lines[-1].endswith(" 88"):
+                first = next(i for i, l in enumerate(lines) if l.startswith(("launch 88", "memset 88")))
+                assert "wait 88 " + done[1] in lines[:first]
+            c.sync()
+    """)
+
+
+def test_the_next_launch_of_a_batch_waits_for_its_tail_pass(fake):
+    fake_cuda.run(fake, """
+        c = runtime.Context(oligo())
+        b = runtime.Batch(max_slots=2)
+        fake.fake_busy(24, 100)
+        run = lambda s: b.run(A.PHASE_STELLAR, [(c, [0], 30000, 0, 30000, 1)], stream=s)
+        run(77)
+        log()
+        run(88)
+        lines = log()
+        tail = next(i for i, l in enumerate(lines) if "tail_kernel" in l)
+        end = next(l for l in lines[tail:] if l.startswith("record") and l.endswith(" 77")).split()[1]
+        first = next(i for i, l in enumerate(lines) if l.startswith(("launch 88", "memset 88")))
+        assert "wait 88 " + end in lines[tail:first]
+        b.sync()
+    """)
