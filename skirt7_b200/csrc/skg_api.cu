@@ -360,6 +360,7 @@ struct skg_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0;
     Allocs A;
+    Allocs extra;                             // the tables of walk_tables()
     DevGrid grid;
     DevScene hs;
     DevScene* ds = nullptr;
@@ -411,6 +412,73 @@ static void mark(skg_ctx* ctx) {
 }
 static void follow(skg_ctx* ctx, cudaStream_t s) {
     if (ctx->behind && s != ctx->stream) CK(cudaStreamWaitEvent(s, ctx->done, 0));
+}
+
+// May a table that the context can do without take this much device memory?  While a quarter of the device
+// stays free beside it (what the pool of freed memory holds back counts as free), for the packet pools (2 to 3 GB at
+// most) and for other contexts.
+static bool spare(int device, size_t bytes) {
+    size_t unused = 0, total = 0;
+    cudaMemPool_t pool;
+    uint64_t held = 0, used = 0;
+    if (cudaMemGetInfo(&unused, &total) != cudaSuccess || cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return bytes <= total && unused + (size_t)(held - std::min(used, held)) >= bytes + total / 4;
+}
+
+// The tables that the FP32 walks are faster with, and do without where there is no room for them.  Made after
+// everything that the scene needs.
+static void walk_tables(skg_ctx* ctx, const skg_scene* sc) {
+    cudaStream_t s = ctx->stream;
+    DevGrid& g = ctx->grid;
+    const DevScene& H = ctx->hs;
+    const int64_t nc = ctx->ncells;
+    Allocs& A = ctx->extra;
+    A.stream = s;
+
+    // octant records of trees (256 bytes per cell; without them the walk takes the lattice records)
+    const char* kind = std::getenv("SKG_TREE_RECORDS");
+    if (g.lattice && g.search != SKG_SEARCH_BOOKKEEPING && nc <= (1 << 27) && !(kind && std::strcmp(kind, "lattice") == 0) &&
+        spare(ctx->device, 256 * (size_t)nc)) {
+        uint4* rec = A.alloc<uint4>(16 * (size_t)nc);
+        if (rec) { CK(launch_octant_records(g, rec, s)); g.orec = rec; }
+    }
+
+    // Voronoi: the planes ahead of each peel-off direction (about half of every list; 270 bytes per cell and
+    // group, so for scenes of few groups, whose entries together an int counts)
+    if (g.type == SKG_GRID_VORONOI && sc->ncomp > 0 && H.ngroups >= 1 && H.ngroups <= 4 &&
+        (int64_t)H.ngroups * nc < (1ll << 26) &&
+        (int64_t)H.ngroups * (sc->grid.vnbr_offsets[nc] + nc) < (1ll << 31)) {
+        const size_t n = (size_t)H.ngroups * nc;
+        Allocs T;
+        T.stream = s;
+        int* cnt = T.alloc<int>(n + 1);
+        int* first = T.alloc<int>(n + 1);
+        const size_t sb = offset_scan_scratch_bytes((int)(n + 1));
+        char* scratch = T.alloc<char>(sb);
+        int total = 0;
+        if (cnt && first && scratch) {
+            CK(launch_group_counts(g, H.gkx, H.gky, H.gkz, H.ngroups, cnt, s));
+            CK(launch_offset_scan(cnt, first, (int)(n + 1), scratch, sb, s));
+            CK(cudaMemcpyAsync(&total, first + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+        }
+        if (total > 0 && spare(ctx->device, 32 * (size_t)total + sizeof(int2) * n)) {
+            int2* po = A.alloc<int2>(n);
+            float4* gp = po ? A.alloc<float4>((size_t)total) : nullptr;
+            int4* gn = gp ? A.alloc<int4>((size_t)total) : nullptr;
+            if (gn) {
+                CK(launch_group_planes(g, H.gkx, H.gky, H.gkz, H.ngroups, first, gp, gn, po, s));
+                g.gplane = gp; g.gnext = gn; g.gpoff = po;
+            } else {
+                A.release();
+            }
+        }
+    }
 }
 
 static int fail(skg_ctx* ctx, const Failure& f) {
@@ -553,14 +621,6 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
             if (sc->ncomp == 1 && (ctx->grid.lrec || ctx->grid.prec || ctx->grid.vnext)) CK(launch_embed_density(ctx->grid, rf, s));
         }
 
-        // octant records of the FP32 walk (256 bytes per cell; without them it takes the lattice records)
-        const char* kind = std::getenv("SKG_TREE_RECORDS");
-        if (ctx->grid.lattice && ctx->grid.search != SKG_SEARCH_BOOKKEEPING && nc <= (1 << 27) &&
-            !(kind && std::strcmp(kind, "lattice") == 0)) {
-            uint4* rec = A.alloc<uint4>(16 * (size_t)nc);
-            if (rec) { CK(launch_octant_records(ctx->grid, rec, s)); ctx->grid.orec = rec; }
-        }
-
         // stellar system (StellarSystem.cpp:35-52)
         H.nstellar = sc->nstellar;
         std::vector<double> starL(sc->nstellar * nl), Lv(nl, 0.0), Xvv((size_t)nl * (sc->nstellar + 1), 0.0);
@@ -641,33 +701,6 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
             H.ngroups = ng;
         }
 
-        // Voronoi: the planes ahead of each peel-off direction (about half of every list; 270 bytes per
-        // cell and group, so for scenes of few groups)
-        if (ctx->grid.type == SKG_GRID_VORONOI && sc->ncomp > 0 && H.ngroups >= 1 && H.ngroups <= 4 &&
-            (int64_t)H.ngroups * nc < (1ll << 26)) {
-            const size_t n = (size_t)H.ngroups * nc;
-            Allocs T;
-            T.stream = s;
-            int* cnt = T.alloc<int>(n + 1);
-            int* first = T.alloc<int>(n + 1);
-            const size_t sb = offset_scan_scratch_bytes((int)(n + 1));
-            char* scratch = T.alloc<char>(sb);
-            int2* po = A.alloc<int2>(n);
-            int total = 0;
-            if (cnt && first && scratch && po) {
-                CK(launch_group_counts(ctx->grid, H.gkx, H.gky, H.gkz, H.ngroups, cnt, s));
-                CK(launch_offset_scan(cnt, first, (int)(n + 1), scratch, sb, s));
-                CK(cudaMemcpyAsync(&total, first + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-                CK(cudaStreamSynchronize(s));
-                float4* gp = total > 0 ? A.alloc<float4>((size_t)total) : nullptr;
-                int4* gn = gp ? A.alloc<int4>((size_t)total) : nullptr;
-                if (gn) {
-                    CK(launch_group_planes(ctx->grid, H.gkx, H.gky, H.gkz, H.ngroups, first, gp, gn, po, s));
-                    ctx->grid.gplane = gp; ctx->grid.gnext = gn; ctx->grid.gpoff = po;
-                }
-            }
-        }
-
         H.min_weight_reduction = sc->min_weight_reduction > 0 ? sc->min_weight_reduction : 1e4;
         H.min_scatt_events = sc->min_scatt_events;
         H.xi = sc->scatt_bias;
@@ -717,6 +750,7 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
         CK(cudaEventCreateWithFlags(&ctx->hev, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&ctx->done, cudaEventDisableTiming));
         ctx->ds = upload(A, &H, 1, s);
+        walk_tables(ctx, sc);
         CK(cudaStreamSynchronize(s));
         *out = ctx;
         return SKG_OK;
@@ -724,7 +758,7 @@ int skg_ctx_create(const skg_scene* sc, int device, skg_ctx** out) {
         int rc = fail(ctx, f);
         set_error(f.msg);
         if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-        ctx->A.release();
+        ctx->A.release(); ctx->extra.release();
         if (ctx->ev0) cudaEventDestroy(ctx->ev0);
         if (ctx->ev1) cudaEventDestroy(ctx->ev1);
         if (ctx->hev) cudaEventDestroy(ctx->hev);
@@ -741,7 +775,7 @@ int skg_ctx_destroy(skg_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaEventSynchronize(ctx->ev1);                  // (a phase on a caller's stream)
     if (ctx->hev_pending) cudaEventSynchronize(ctx->hev);
-    ctx->A.release();
+    ctx->A.release(); ctx->extra.release();
     cudaEventDestroy(ctx->ev0); cudaEventDestroy(ctx->ev1); cudaEventDestroy(ctx->hev);
     cudaEventDestroy(ctx->done);
     cudaStreamDestroy(ctx->stream);
@@ -752,7 +786,7 @@ int skg_ctx_destroy(skg_ctx* ctx) {
 int skg_ctx_info(const skg_ctx* ctx, int64_t* ncells, int64_t* device_bytes) {
     if (!ctx) return SKG_ERR_INVALID;
     if (ncells) *ncells = ctx->ncells;
-    if (device_bytes) *device_bytes = (int64_t)ctx->A.bytes;
+    if (device_bytes) *device_bytes = (int64_t)(ctx->A.bytes + ctx->extra.bytes);
     return SKG_OK;
 }
 

@@ -188,3 +188,38 @@ def test_the_next_launch_of_a_batch_waits_for_its_tail_pass(fake):
         assert "wait 88 " + end in lines[tail:first]
         b.sync()
     """)
+
+
+def test_tables_that_can_be_missed_leave_room_for_those_that_cannot(fake):
+    """On a device with room for a tree scene's own tables but not for its octant records too, the scene is set
+    up and walks on the lattice records; the records are made while a quarter of the device stays free."""
+    fake_cuda.run(fake, """
+        import numpy as np
+        splits = np.zeros(585, dtype=np.uint8)             # every node of levels 0 to 2: 512 leaves
+        splits[:73] = 1
+        def scene():
+            m = models.pan_disk(nlambda=50, npix=8, dust_emission=True, write_absorption=True)
+            m.dustGrid = runtime.tree_from_splits(A.GRID_OCTREE, (-1., -1., -1., 1., 1., 1.), splits)
+            m.rho = np.full((1, 512), 1e-24)
+            return m
+        def context(memory):
+            fake.fake_memory(memory)
+            c = runtime.Context(scene())
+            fake.fake_memory(8 << 30)
+            log()
+            c.run_phase(A.PHASE_STELLAR, [0], 9000); c.sync()
+            walks = {l.split("Tree")[1].split("Stepper")[0] for l in log("trav_kernel")}
+            need = c.device_bytes
+            c.close()
+            assert fake.fake_used() == 0
+            return need, walks
+        os.environ["SKG_TREE_RECORDS"] = "lattice"
+        need, walks = context(8 << 30)
+        assert walks == {"Lattice"}
+        del os.environ["SKG_TREE_RECORDS"]
+        full, walks = context(8 << 30)
+        assert walks == {"Octant"} and full == need + 256 * 512
+        for room in (0, 1000, 256 * 512, need // 4):
+            assert context(need + room) == (need, {"Lattice"}), room
+        assert context((full + 4096) * 4 // 3) == (full, {"Octant"})
+    """)
