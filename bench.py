@@ -87,6 +87,20 @@ def parse():
 WORKLOAD_PACKETS = {"octree_pan": 1e7, "cartesian_oligo": 1e7, "voronoi_clumpy": 1e8, "kdtree_dust": 1e7}
 
 
+def phase_launches(waves, grid, cells, packets, pool, absorbs):
+    """Kernels of a phase: per wave the scatter-and-launch pass, the optical depths, the ends and the re-walks, the
+    paths of a phase that tallies absorption in a kernel of their own, and the three kernels of the walk order
+    (tree and Voronoi grids of 8 MB of records, from 786432 packets in flight); a phase without waves is
+    the tail pass.  (The tail pass behind the waves is not counted.)"""
+    if waves == 0:
+        return 1
+    if not pool:
+        pool = 1 << (23 if packets >= 1 << 26 and grid != "VoronoiDustGrid" else 21)
+    records = cells * {"CartesianDustGrid": 0, "VoronoiDustGrid": 512}.get(grid, 32)
+    ordered = records >= 8 << 20 and 3 << 18 <= min(packets, pool) < 1 << 28
+    return waves * (4 + (1 if absorbs else 0) + (3 if ordered else 0))
+
+
 def peaks():
     try:
         with open(MEASURED) as f:
@@ -561,8 +575,13 @@ def main():
             "setup": {"grid_build_s": wl.grid_s, "grid": "device", "autotune_s": tune_s,
                       "launch": {k: launch[k] for k in ("pool", "refill", "blocks")} if launch else "library defaults",
                       "autotune_trials": launch["trials"] if launch else None},
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
+            # achieved and frac: the algorithmic bytes over the measured HBM rate.  The caches serve most of them, so
+            # frac is no share of HBM's rate (dram_frac is); what bounds the walks is the L1, one gathered record per
+            # cycle and SM, or on Cartesian grids the instruction issue
+            "roofline": {"bound": "issue" if wl.gtype == "CartesianDustGrid" else "l1", "achieved": achieved,
+                         "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
+                         "peak_kind": peak_kind, "dram_frac": traffic * waves / (trav_ms / 1e3) / 1e9 / peak
+                         if traffic and trav_ms > 0 else None,
                          "traffic_basis": ("scaled, not measured in this run: ncu DRAM bytes per cell step of "
                                            "this workload's traversal pass (%.2f B, one capture of a stellar "
                                            "phase) x this launch's cell steps" % bps) if bps else None,
@@ -573,9 +592,9 @@ def main():
                          "phase_ms": kms, "event_pass_ms": ev_ms, "traversal_pass_ms": trav_ms},
             "e2e": {"value": e2e, "unit": "packets/s", "h2d_bytes_per_step": len(phases) * (4 * nl + 64),
                     "d2h_bytes_per_step": cubes_bytes, "steps": e2e_steps},
-            # per wave: the scatter-and-launch pass, the optical depths, the ends, the re-walks, and on
-            # the tree and Voronoi workloads the three kernels of the walk order
-            "gpu_launches": (4 if wl.gtype == "CartesianDustGrid" else 7) * waves * len(phases) * args.steps,
+            # (the waves of the stellar phase stand for those of the other phases)
+            "gpu_launches": phase_launches(waves, wl.gtype, ctx.ncells, npp_rank * nl, launch["pool"] if launch else 0,
+                                           c["absorb_adds"] > 0) * len(phases) * args.steps,
             "clocks": clk,
             "counters_stellar_phase": c,
         }
