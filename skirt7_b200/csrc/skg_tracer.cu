@@ -1733,7 +1733,8 @@ cudaError_t WaveRunner::start(const RunParams& P, int grid_type, int tree_walk, 
     if (order_on_ && (e = cudaMemsetAsync(bins_, 0, 2 * JOB_BINS * sizeof(unsigned), s)) != cudaSuccess) return e;
     tail_only_ = ph_.tail_div > 0 && fits && npool <= (size_t)(grid_type == SKG_GRID_CARTESIAN ? SKG_TAIL_ONLY_CART : SKG_TAIL_ONLY);
     if (!tail_only_) {
-        if ((e = enqueue(estimate)) != cudaSuccess) return e;
+        // (a divisor of 1 hands the phase over whatever the first look finds: it looks after one wave)
+        if ((e = enqueue(ph_.tail_div == 1 ? 1 : estimate)) != cudaSuccess) return e;
     } else {
         if ((e = cudaMemsetAsync(pk_, 0, npool * sizeof(Packet), s)) != cudaSuccess) return e;   // (wave 0 writes every record)
         if ((e = enqueue_tail()) != cudaSuccess) return e;
@@ -1796,7 +1797,7 @@ cudaError_t WaveRunner::finish(int timeout_ms, cudaEvent_t end, bool* timed_out)
             cudaError_t e = enqueue_tail();
             if (e != cudaSuccess) return over(e);
             pending_ = false;
-            estimate = waves_;
+            if (ph_.tail_div != 1) estimate = waves_;
             more = true;
             break;
         }

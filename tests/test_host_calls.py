@@ -223,3 +223,23 @@ def test_tables_that_can_be_missed_leave_room_for_those_that_cannot(fake):
             assert context(need + room) == (need, {"Lattice"}), room
         assert context((full + 4096) * 4 // 3) == (full, {"Octant"})
     """)
+
+
+def test_a_divisor_of_one_hands_over_after_the_first_wave(fake):
+    """SKG_TAIL_DIV=1 (the plain path: one thread runs a packet's whole life) leaves one wave before the tail
+    pass, and later phases as many waves up front as before."""
+    fake_cuda.run(fake, """
+        c = runtime.Context(oligo())
+        def waves():
+            log()
+            c.run_phase(A.PHASE_STELLAR, [0], 30000)
+            c.sync()
+            lines = log("launch ")
+            return sum("launch_kernel" in l for l in lines), sum("tail_kernel" in l for l in lines)
+        fake.fake_busy(40, 30000)
+        before = waves(), waves()
+        os.environ["SKG_TAIL_DIV"] = "1"
+        assert waves() == (1, 1)
+        del os.environ["SKG_TAIL_DIV"]
+        assert waves() == before[1]
+    """)
