@@ -163,7 +163,9 @@ cudaError_t launch_dust_emission(const DevGrid& g, const DevScene* dS, const dou
 // P_{i+1} = sum_{j<=i} p_j / sum p): sums of tiles of cells, their offsets per wavelength, then the
 // tiles again with their offset and the normalisation -- three launches for all wavelengths, the
 // luminosities read twice and the result written once (a library scan per wavelength and a pass to
-// normalise before: 80 launches for 40 wavelengths).
+// normalise before: 80 launches for 40 wavelengths).  The last entry is 1.  The others are sums in more than one
+// order (lanes, warps, tiles), so where cells without luminosity follow, an entry may lie a rounding below the one
+// before it; deviates are multiples of 2^-33, some 10^6 times as far apart.
 constexpr int CDF_TILE = 2048;                     // 8 warps of 8 rows of 32 cells
 SKG_D double warp_incl(double v, int lane) {
     for (int d = 1; d < 32; d <<= 1) { const double t = __shfl_up_sync(0xffffffffu, v, d); if (lane >= d) v += t; }
@@ -226,11 +228,10 @@ __global__ void __launch_bounds__(256) cdf_kernel(int nc, const double* __restri
     double before = offsets[(size_t)ell * gridDim.x + blockIdx.x];
     for (int w = 0; w < warp; w++) before += ws[w];
     const double tot = Ltot[ell];
-    const double inv = tot > 0 ? 1.0 / tot : 0.0;
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         const int64_t m = m0 + 32 * r;
-        if (m < nc) out[m + 1] = (before + v[r]) * inv;
+        if (m < nc) out[m + 1] = !(tot > 0) ? 0.0 : m == nc - 1 ? 1.0 : fmin((before + v[r]) / tot, 1.0);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = 0.0;
 }
