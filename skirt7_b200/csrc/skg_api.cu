@@ -1059,7 +1059,15 @@ int skg_read_absorption(skg_ctx* ctx, double* labs_stellar, double* labs_dust) {
             if (!dev) { std::memset(out, 0, n * sizeof(double)); return; }
             if (nl == 1) { CK(cudaMemcpyAsync(out, dev, n * sizeof(double), cudaMemcpyDeviceToHost, s)); return; }
             if (!buf) buf = T.alloc<double>(piece * nl);
-            if (!buf) throw Failure{SKG_ERR_OOM, "device allocation failed"};
+            if (!buf) {                    // (no room on the device: wavelength by wavelength on the host)
+                std::vector<double> row(nc);
+                for (size_t e = 0; e < nl; e++) {
+                    CK(cudaMemcpyAsync(row.data(), dev + e * nc, nc * sizeof(double), cudaMemcpyDeviceToHost, s));
+                    CK(cudaStreamSynchronize(s));
+                    for (size_t m = 0; m < nc; m++) out[m * nl + e] = row[m];
+                }
+                return;
+            }
             for (size_t m0 = 0; m0 < nc; m0 += piece) {
                 const size_t k = std::min(piece, nc - m0);
                 CK(launch_cell_major(dev, (int64_t)nc, (int)nl, (int64_t)m0, (int64_t)k, buf, s));

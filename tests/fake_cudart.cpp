@@ -111,6 +111,11 @@ void fake_busy(int waves, int n) { busy = waves; jobs = n; }
 void fake_fail(const char* kernel, int after) { fail_name = kernel; fail_skip = after; }
 void fake_memory(size_t bytes) { total = bytes; }
 size_t fake_used() { return used; }
+void fake_fill(size_t bytes) {       // 0, 1, 2, ... in every allocation of this size
+    for (auto& a : allocated)
+        if (a.second == bytes)
+            for (size_t i = 0; i < bytes / sizeof(double); i++) ((double*)a.first)[i] = (double)i;
+}
 
 // ---- registration and launches
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }

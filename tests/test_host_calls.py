@@ -243,3 +243,22 @@ def test_a_divisor_of_one_hands_over_after_the_first_wave(fake):
         del os.environ["SKG_TAIL_DIV"]
         assert waves() == before[1]
     """)
+
+
+def test_absorbed_luminosities_are_read_on_a_full_device(fake):
+    """The transpose takes its scratch on the device; without room for it the tables are read all the same."""
+    fake_cuda.run(fake, """
+        import numpy as np
+        c = runtime.Context(oligo(wavelengths=[(0.4 + 0.1 * i) * 1e-6 for i in range(3)], write_absorption=True))
+        nc, nl = 6 * 5 * 4, 3
+        fake.fake_fill.argtypes = [C.c_size_t]
+        fake.fake_fill(8 * nc * nl)                        # the tables, [wavelength][cell]
+        fake.fake_memory(fake.fake_used())
+        c.dust_tallied = True
+        for labs in c.read_absorption():
+            assert np.array_equal(labs, np.arange(nc * nl).reshape(nl, nc).T)
+        assert not log("cell_major")
+        fake.fake_memory(8 << 30)
+        c.read_absorption()
+        assert len(log("cell_major")) == 2
+    """)
