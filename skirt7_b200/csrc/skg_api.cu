@@ -1440,7 +1440,8 @@ int skg_batch_run(skg_batch* b, int phase, const skg_work* work, int nwork, cons
         RunParams P = b->T.params((opts && opts->max_scatt > 0) ? opts->max_scatt : 100000, opts ? opts->refill : 0);
         Staging& T = b->T;
         // the walks keep the DevGrid of every slot in shared memory, at the cost of L1: room for the slots of
-        // this launch, in a captured one up to the next power of two (it serves launches of no more slots)
+        // this launch, in a captured one up to the next power of two (it serves launches of no more slots).  In a
+        // batch of 64 slots 24 fit variants took 27.8 ms with room for all 64, 25.7 so; one simulation 17.5, 15.9
         int gslots = nslots;
         if (flags & SKG_BATCH_GRAPH) {
             gslots = 1;

@@ -118,9 +118,9 @@ struct RunParams {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Wavefront state.  The packets in flight live in a pool of 128-byte records; each wave an event
-// pass (one thread per record) advances every packet to its next traversals and writes them as
-// jobs, and a traversal pass walks all jobs of the wave.
+// Wavefront state.  The packets in flight live in a pool of 128-byte records; each wave a launch pass (one
+// thread per packet at its interaction point and per free record) brings packets to their next traversals and
+// writes these as jobs, and a traversal pass walks all jobs of the wave and ends their paths.
 enum PacketState : int { PK_EMPTY = 0, PK_WAIT, PK_INTERACT, PK_TERM, PK_DONE };
 #ifndef SKG_BIN_XY
 #define SKG_BIN_XY 6
@@ -176,7 +176,7 @@ struct WaveParams {
     Packet* pk;
     int npool;
     int wave;                         // index of this wave within the phase
-    // this wave's jobs (written by the event pass, walked by the traversal pass): path jobs at
+    // this wave's jobs (written by the launch pass, walked by the traversal pass): path jobs at
     // [0, npool) and peel-off jobs from npool on, so that the longest jobs are taken first
     int2* jobs;                       // (packet, type)
     double* jtau;                     // peel-off optical depth

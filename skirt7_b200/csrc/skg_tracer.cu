@@ -27,9 +27,9 @@
 //                   test and the sampling of the interaction optical depth (simulatepropagation, :513-531),
 //                   with the next wave's lists of interacting packets and free records; per peel-off the
 //                   instruments' tallies.
-// The traversal kernels hold nothing but the walk, so they keep few registers, no local memory and
-// a small instruction footprint; the divergent event code runs once per packet per wave in kernels
-// of its own.  Instruments seen from the same direction share one peel-off traversal
+// The traversal kernels hold nothing but the walk: 64 or 80 registers, with at most 84 bytes of spills (FP64
+// paths on trees; a single simulation's FP32 optical depths on octant records 56, on Voronoi and rope records none).  What happens
+// to a packet between its walks runs once per packet per wave in kernels of its own.  Instruments seen from the same direction share one peel-off traversal
 // (identical optical depth; the reference recomputes it per instrument).
 #include "skg_scene.cuh"
 #include "skg_internal.h"
@@ -53,8 +53,8 @@ namespace skg {
 // own state alone, and the path's long end (end_kernel) holds none of them.  Octree disk, 2*10^7
 // packets: traversal pass 179.6 ms against 209.8 with the end of the path and the re-walk inside the
 // path-job kernel (220 bytes of spills at 64 registers); fit-variant batch 46.2 against 53.5 ms.
-// blocks per SM of the path and re-walk kernels: 3 (80 registers, no spills) against 4 (64, spilling
-// 64-112 bytes): traversal pass of the k-d tree disk with absorption 21.3 against 22.8 ms, Cartesian
+// blocks per SM of the path and re-walk kernels: 3 (80 registers; FP32 spills at most 56 bytes) against 4 (64,
+// spilling 64-112 bytes): traversal pass of the k-d tree disk with absorption 21.3 against 22.8 ms, Cartesian
 // disk with absorption 6.75 against 7.35, re-walks of the octree disk 1.4 ms of 157 less
 #ifndef SKG_PATH_MIN_BLOCKS
 #define SKG_PATH_MIN_BLOCKS 3
@@ -166,18 +166,16 @@ SKG_D double step_dtau(const DevScene& S, const St& st, float kext1, int m, int 
 
 // Instrument::detect for the members of one direction group after the shared traversal
 // (SEDInstrument.cpp:32-42, FrameInstrument.cpp:33-47, SimpleInstrument.cpp:35-49,
-// FullInstrument.cpp:109-177).  SED bins go to the block's private copy `psed` when it is given
-// (every packet of a wavelength adds to the same SED bin: global atomics would serialise on it).
-// Returns the number of tally updates.
-// detect_group inlined into the event kernel: its call kept a 240-byte stack frame there (972
-// bytes of spill loads per thread at 64 registers against 52 inlined); event pass of a
-// 10^7-packet phase 14.3 against 16.1 ms (octree disk)
+// FullInstrument.cpp:109-177), every tally an atomic.  Returns the number of tally updates.  (detect_peels has the
+// same rules for a launch of one simulation, with its SED bins summed per block: a change of one is a change of both.)
+// Inlined: as a call it kept a 240-byte stack frame (972 bytes of spill loads per thread at 64 registers against
+// 52), and the detections of a 10^7-packet octree phase took 16.1 against 14.3 ms.
 #ifndef SKG_DETECT_INLINE
 #define SKG_DETECT_INLINE 1
 #endif
 // frame pixel tallies: lanes of a warp that add to the same pixel sum their values over the warp
 // first and one of them adds (1), or every lane adds its own value (0).  Octree disk, 5*10^8
-// packets: phase 7870 ms with the aggregation against 7850-7930 ms without, event pass 652 against
+// packets: phase 7870 ms with the aggregation against 7850-7930 ms without, detections 652 against
 // 632-640 ms -- lanes of a warp rarely hit one pixel (their packets sit anywhere in the galaxy),
 // so the match costs more than the atomics it saves; off by default.
 #ifndef SKG_WARP_AGG
@@ -398,7 +396,7 @@ SKG_D int find_item(const WorkItem* items, int n, uint64_t p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// event pass
+// launch pass and detections
 
 // Bins of the walk order: the octant of a path job's direction or the group (mod 8) of a peel-off
 // job, then the Morton cell of its start on a division of the grid's box.
@@ -657,8 +655,8 @@ SKG_D void sed_add(double* sed, int key, double v) {
 // Detection: one thread per peel-off job of the wave, right after its walks (Instrument::detect of every
 // member of its direction group; detect_group has the rules).  A launch of one simulation tallies its
 // SED bins per block and adds them once at the end.  (A pass over all records of the pool in the next wave
-// before, which also made the record lists: event and launch passes of the octree disk, 2*10^7 packets,
-// 35.4 ms a phase against 26.5; Cartesian disk, 10^6, 2.40 against 1.25; a batch of 24 fit variants 35.1
+// before, which also made the record lists: with the launch pass 35.4 ms a phase of the octree disk, 2*10^7 packets,
+// against 26.5; Cartesian disk, 10^6, 2.40 against 1.25; a batch of 24 fit variants 35.1
 // against 30.6 ms in all.)
 SKG_D void detect_peels(const WaveParams& W, double* s_sed) {
     const RunParams& P = W.R;
@@ -1243,11 +1241,9 @@ __global__ void __launch_bounds__(256) end_kernel(const WaveParams W) {
 //
 // When few packets are left in flight, each wave costs about as long as its longest walk while
 // most of the device idles, and a packet still needs a wave per event.  The tail pass gives every
-// remaining packet a thread that runs the rest of its life at once -- the previous wave's pending
-// peel-off detections, then interaction, scattering peel-offs, scattering, path and re-walk until
-// it terminates, then further packets while the work counter has any -- with the same random
-// streams, samplers and tallies as the waves (device functions shared with the event and traversal
-// passes), so a phase gives the same results with or without it, up to the summation order of the
+// remaining packet a thread that runs the rest of its life at once -- interaction, scattering peel-offs,
+// scattering, path and re-walk until it terminates, then further packets while the work counter has any -- with
+// the same random streams, samplers and tallies as the waves (device functions shared with their kernels), so a phase gives the same results with or without it, up to the summation order of the
 // FP64 tally atomics.
 
 // Optical depth from (x, y, z) toward (kx, ky, kz) to the edge of the grid (DustSystem::opticaldepth,

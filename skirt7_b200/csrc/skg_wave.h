@@ -3,10 +3,11 @@
 // A phase runs as a sequence of waves on one stream.  Wave w: a launch pass (scatter the packets that
 // the previous wave brought to their interaction point, launch new packets into the records that it freed, and write the
 // next traversals as jobs), the walks of every job, their ends (escape, termination, detection) and the re-walks.
-// The number of waves is not known in advance: begin() enqueues an estimate, finish() reads how many
-// packets still had work in the last enqueued wave and enqueues more until none has -- or, once few
-// have, the tail pass, which finishes every remaining packet in one launch.  Phases of few packets
-// are the tail pass alone.
+// The number of waves is not known in advance: begin() enqueues an estimate (as many as the last phase took),
+// finish() reads, behind the last of them, how many packets still had work and enqueues more until none has and
+// no record waits for a new packet -- or, if few have by then, the tail pass, which finishes every remaining
+// packet in one launch.  (A phase that ends within the estimate never sees the tail pass.)  Phases of few packets are
+// the tail pass alone.
 #pragma once
 #include "skg_scene.cuh"
 
@@ -61,14 +62,14 @@ public:
     size_t pool_capacity() const { return cap_pool_; }
     // changes when reserve() has moved a buffer (a captured launch then holds freed memory)
     int generation() const { return generation_; }
-    // With timing on, each wave's two kernels are bracketed by events (not inside graph capture).
+    // With timing on, each wave's launch and traversal passes are bracketed by events (not inside graph capture).
     bool timing = false;
-    // Device time of the finished phase's event passes and traversal passes (ms).
+    // Device time of the finished phase's launch passes and traversal passes (ms).
     cudaError_t times(float* event_ms, float* trav_ms) const;
 
     int estimate = 24;                // waves the next phase enqueues up front
-    // the tail pass takes over when at most npool / tail_div packets had work in the last wave
-    // (0: waves to the end; the environment variable SKG_TAIL_DIV overrides it per phase)
+    // the tail pass takes over when finish() finds at most npool / tail_div packets with work in the last
+    // enqueued wave (0: waves to the end; the environment variable SKG_TAIL_DIV overrides it per phase)
     int tail_div = 16;
 
 private:
