@@ -28,9 +28,10 @@
 //                   with the next wave's lists of interacting packets and free records; per peel-off the
 //                   instruments' tallies.
 // The traversal kernels hold nothing but the walk: 64 or 80 registers, with at most 84 bytes of spills (FP64
-// paths on trees; a single simulation's FP32 optical depths on octant records 56, on Voronoi and rope records none).  What happens
-// to a packet between its walks runs once per packet per wave in kernels of its own.  Instruments seen from the same direction share one peel-off traversal
-// (identical optical depth; the reference recomputes it per instrument).
+// paths on trees; a single simulation's FP32 optical depths on octant records 56, on Voronoi and rope records
+// none).  What happens to a packet between its walks runs once per packet per wave in kernels of its own.
+// Instruments seen from the same direction share one peel-off traversal (identical optical depth; the
+// reference recomputes it per instrument).
 #include "skg_scene.cuh"
 #include "skg_internal.h"
 #include "skg_wave.h"
