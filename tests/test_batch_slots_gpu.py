@@ -22,12 +22,12 @@ def alone(ctx, n, seed, precision):
 
 @pytest.mark.parametrize("precision", [A.PREC_FP32, A.PREC_FP64])
 @pytest.mark.parametrize("grid", ["cartesian", "octree", "kdtree", "voronoi"])
-def test_one_simulation_in_a_batch_of_default_capacity(grid, precision):
+@pytest.mark.parametrize("n", [30001, 701])     # waves on every grid; the tail pass alone
+def test_one_simulation_in_a_batch_of_default_capacity(grid, precision, n):
     ctx = runtime.Context(model(grid))
-    n = 30001                                   # above the tail pass alone on every grid
     want = alone(ctx, n, 3, precision)
     b = runtime.Batch()
-    for graph in (False, True):
+    for graph in (False, True, True):
         ctx.reset_tallies()
         ctx.sync()
         b.run(A.PHASE_STELLAR, [(ctx, [0], n, 0, n, 3)], precision=precision, graph=graph)
@@ -89,4 +89,31 @@ def test_a_replay_goes_on_as_it_was_captured():
         assert np.allclose(thick.read_instrument(0)[0], want, **CLOSE)
         assert np.allclose(thick.read_absorption()[0], absorbed, **CLOSE)
     assert captured > 1 and b.counters()["errors"] == 0
+    b.close()
+
+
+@pytest.mark.parametrize("tail", ["0", "16"])
+def test_replays_that_take_more_waves_than_the_last(tail, monkeypatch):
+    """A captured phase that ends within its waves, replayed as it is and then for thick dust: the host sees the
+    replay's own counters, not those that the last one left, and adds waves."""
+    monkeypatch.setenv("SKG_TAIL_DIV", tail)
+    def ctx(tau):
+        m = models.oligo_disk(N=(12, 11, 9), tauV=tau, npix=12, write_absorption=False)
+        m.rho = cell_center_density(m)
+        return runtime.Context(m)
+    thin, thick = ctx(1e-4), ctx(10.0)
+    n, pool = 60000, 6000
+    want = alone(thick, n, 5, A.PREC_FP32), alone(thin, n, 5, A.PREC_FP32)
+    b = runtime.Batch(max_slots=2)
+    for i, c in enumerate((thin, thin, thick, thin, thin, thick)):
+        c.reset_tallies()
+        b.run(A.PHASE_STELLAR, [(c, [0], n, 0, n, 5)], graph=True, pool=pool)
+        b.sync()
+        assert np.allclose(c.read_instrument(0)[0], want[c is thin], **CLOSE), i
+        waves = b.counters()["waves"]
+        if i < 2:
+            captured = waves
+        elif i == 2:
+            assert waves > captured or tail != "0"
+    assert b.counters()["errors"] == 0 and b.counters()["packets"] == 6 * n
     b.close()
